@@ -864,32 +864,29 @@ __device__ __forceinline__ void guard_claim(const WorkDev &w, uint4 &rec, uint64
 // Writes the results of the warp's records (lane k owns record `mine`, whose results
 // start at out_base, checked by guard_claim; the valid lanes are a prefix): the
 // lanes stage their records and offsets, then the warp writes U records at a time,
-// each by the whole warp, lane l taking slots 2l and 2l + 1 of the 64-slot block.
+// each by the whole warp.
 struct EmitStage {
 	uint4 rec[32];
 	unsigned long long ob[32];
 };
 
-template <typename T, bool HAS_ID, bool POINTS, int U>
-__device__ __forceinline__ void emit_blocks(const TreeDev<T> &t, const uint4 &mine, uint64_t out_base, bool valid,
-                                            EmitStage &st, void *__restrict__ out)
+// Ids: lane l takes slots 2l and 2l + 1 of the 64-slot block (one 8-byte load).  Slots
+// l and l + 32, whose stores cover consecutive words, took 1468 against 1318 us for
+// the 948 M ids of a 4096-query batch at 2^28 points: a second load a record costs
+// more than the denser stores give, the kernel being bound by its instructions.
+template <int U>
+__device__ __forceinline__ void emit_ids(const uint32_t *__restrict__ id, int nrec, const EmitStage &st,
+                                         uint32_t *__restrict__ out)
 {
-	using Pt = Point<T, HAS_ID>;  // U: records in flight per warp
-	static_assert(32 % U == 0, "a batch of records ends inside the 32 staged ones");
 	const uint32_t lane = lane_id();
 	const uint32_t psh = (2 * lane) & 31;
 	// the record's slots before this lane's pair, as masks of its two 32-slot words
 	const uint32_t below_z = lane < 16 ? (1u << psh) - 1u : FULL;
 	const uint32_t below_w = lane < 16 ? 0u : (1u << psh) - 1u;
-	st.rec[lane] = mine;
-	st.ob[lane] = out_base;
-	__syncwarp();
-	const int nrec = __popc(__ballot_sync(FULL, valid));
 	for (int k0 = 0; k0 < nrec; k0 += U) {
-		uint32_t b2[U], hb[U];
+		uint32_t b2[U];
 		uint64_t o[U];
 		uint2 idv[U];
-		T d1[POINTS ? U : 1][2], d2[POINTS ? U : 1][2];
 #pragma unroll
 		for (int u = 0; u < U; u++) {
 			// every lane staged a record, and those past nrec are empty (zero masks), so
@@ -900,30 +897,8 @@ __device__ __forceinline__ void emit_blocks(const TreeDev<T> &t, const uint4 &mi
 			b2[u] = ((lane < 16 ? rc.z : rc.w) >> psh) & 3u;
 			const uint32_t before = __popc(rc.z & below_z) + __popc(rc.w & below_w);
 			o[u] = st.ob[k] + before;
-			hb[u] = (rc.x & ~63u) + 2 * lane;  // (without RECORD_WHOLE)
-			if constexpr (!POINTS || HAS_ID)
-				idv[u] = b2[u] ? *reinterpret_cast<const uint2 *>(t.id + hb[u]) : make_uint2(0, 0);
-			if constexpr (POINTS) {
-				// the slot pair's dim1 and dim2 with one 8-byte (16 for doubles) load each
-				d1[u][0] = d1[u][1] = d2[u][0] = d2[u][1] = T(0);
-				if (b2[u]) {
-					if constexpr (sizeof(T) == 4) {
-						const uint2 a = *reinterpret_cast<const uint2 *>(t.dim1 + hb[u]);
-						const uint2 c = *reinterpret_cast<const uint2 *>(t.dim2 + hb[u]);
-						memcpy(&d1[u][0], &a.x, 4);
-						memcpy(&d1[u][1], &a.y, 4);
-						memcpy(&d2[u][0], &c.x, 4);
-						memcpy(&d2[u][1], &c.y, 4);
-					} else {
-						const double2 a = *reinterpret_cast<const double2 *>(t.dim1 + hb[u]);
-						const double2 c = *reinterpret_cast<const double2 *>(t.dim2 + hb[u]);
-						d1[u][0] = a.x;
-						d1[u][1] = a.y;
-						d2[u][0] = c.x;
-						d2[u][1] = c.y;
-					}
-				}
-			}
+			const uint32_t hb = (rc.x & ~63u) + 2 * lane;  // (without RECORD_WHOLE)
+			idv[u] = b2[u] ? *reinterpret_cast<const uint2 *>(id + hb) : make_uint2(0, 0);
 		}
 #pragma unroll
 		for (int u = 0; u < U; u++) {
@@ -931,22 +906,100 @@ __device__ __forceinline__ void emit_blocks(const TreeDev<T> &t, const uint4 &mi
 			for (int j = 0; j < 2; j++) {
 				if ((b2[u] >> j) & 1u) {
 					const uint64_t oo = o[u] + (j & b2[u]);  // the second slot follows a reported first
-					if constexpr (POINTS) {
-						Pt rec;
-						rec.dim1 = d1[u][j];
-						rec.dim2 = d2[u][j];
-						if constexpr (HAS_ID)
-							rec.id = j ? idv[u].y : idv[u].x;
-						static_cast<Pt *>(out)[oo] = rec;
-					} else {
-						// evict-first: the output streams through L2 once and should not push
-						// out tree rows that other queries' records read again
-						__stcs(static_cast<uint32_t *>(out) + oo, j ? idv[u].y : idv[u].x);
-					}
+					// evict-first: the output streams through L2 once and should not push
+					// out tree rows that other queries' records read again
+					__stcs(out + oo, j ? idv[u].y : idv[u].x);
 				}
 			}
 		}
 	}
+}
+
+// A packed point's id, with the padding of a 24-byte point (it leaves with the words).
+template <typename T>
+__device__ __forceinline__ void pack_id(Point<T, true> &p, uint32_t id)
+{
+	if constexpr (sizeof(T) == 8)
+		*reinterpret_cast<unsigned long long *>(&p.id) = id;
+	else
+		p.id = id;
+}
+
+// Points: lane l takes slots l and l + 32 (a load reads one whole row of a field), and
+// the points of a record are packed into shared memory in the order of the output and
+// leave it as consecutive words.  A store a lane of a field of an 8- to 24-byte point
+// touched every sector of the record's range once per field: 127 us for the 6.2 M
+// 24-byte points of a 601-query batch at 12.3 M points, 69 us packed.
+template <typename T, bool HAS_ID, int U>
+__device__ __forceinline__ void emit_points(const TreeDev<T> &t, int nrec, const EmitStage &st,
+                                            Point<T, HAS_ID> *pack, Point<T, HAS_ID> *__restrict__ out)
+{
+	using Pt = Point<T, HAS_ID>;
+	using W = typename std::conditional<sizeof(T) == 8, unsigned long long, uint32_t>::type;
+	const uint32_t lane = lane_id(), below = lanemask_lt();
+	for (int k0 = 0; k0 < nrec; k0 += U) {
+		uint32_t m[U][2], idv[U][2];
+		T d1[U][2], d2[U][2];
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const uint4 rc = st.rec[k0 + u];  // (empty past nrec, as in emit_ids)
+			m[u][0] = rc.z;
+			m[u][1] = rc.w;
+#pragma unroll
+			for (int j = 0; j < 2; j++) {
+				const uint32_t h = (rc.x & ~63u) + 32 * j + lane;
+				const bool on = (m[u][j] >> lane) & 1u;
+				d1[u][j] = on ? t.dim1[h] : T(0);
+				d2[u][j] = on ? t.dim2[h] : T(0);
+				if constexpr (HAS_ID)
+					idv[u][j] = on ? t.id[h] : 0u;
+			}
+		}
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const uint32_t nz = __popc(m[u][0]);
+#pragma unroll
+			for (int j = 0; j < 2; j++) {
+				if ((m[u][j] >> lane) & 1u) {
+					Pt &p = pack[(j ? nz : 0u) + __popc(m[u][j] & below)];
+					p.dim1 = d1[u][j];
+					p.dim2 = d2[u][j];
+					if constexpr (HAS_ID)
+						pack_id(p, idv[u][j]);
+				}
+			}
+			__syncwarp();
+			const uint32_t words = (nz + __popc(m[u][1])) * (uint32_t) (sizeof(Pt) / sizeof(W));
+			const W *src = reinterpret_cast<const W *>(pack);
+			W *dst = reinterpret_cast<W *>(out + st.ob[k0 + u]);
+			for (uint32_t i = lane; i < words; i += 32)
+				__stcs(dst + i, src[i]);  // evict-first, as the ids
+			__syncwarp();  // the pack is refilled by the next record
+		}
+	}
+}
+
+// Shared memory of one emitting warp.
+template <typename Pt, bool POINTS>
+struct EmitWarp {
+	EmitStage st;
+	Pt pack[POINTS ? 64 : 1];
+};
+
+template <typename T, bool HAS_ID, bool POINTS, int U>
+__device__ __forceinline__ void emit_blocks(const TreeDev<T> &t, const uint4 &mine, uint64_t out_base, bool valid,
+                                            EmitWarp<Point<T, HAS_ID>, POINTS> &sm, void *__restrict__ out)
+{
+	static_assert(32 % U == 0, "a batch of records ends inside the 32 staged ones");
+	const uint32_t lane = lane_id();
+	sm.st.rec[lane] = mine;
+	sm.st.ob[lane] = out_base;
+	__syncwarp();
+	const int nrec = __popc(__ballot_sync(FULL, valid));
+	if constexpr (POINTS)
+		emit_points<T, HAS_ID, U>(t, nrec, sm.st, sm.pack, static_cast<Point<T, HAS_ID> *>(out));
+	else
+		emit_ids<U>(t.id, nrec, sm.st, static_cast<uint32_t *>(out));
 	__syncwarp();  // the stage is reused by the warp's next batch
 }
 
@@ -958,7 +1011,7 @@ __global__ void __launch_bounds__(THREADS) k_emit(TreeDev<T> t, WorkDev w, void 
 	// a programmatic dependent of the scan (a no-op after any other predecessor)
 	asm volatile("griddepcontrol.wait;" ::: "memory");
 	__shared__ uint64_t s_total;
-	__shared__ EmitStage s_stage[THREADS / 32];
+	__shared__ EmitWarp<Point<T, HAS_ID>, POINTS> s_warp[THREADS / 32];
 	if (threadIdx.x == 0) {
 		uint64_t b = 0;
 		for (uint32_t e = 0; e < t.levels; e++)
@@ -991,7 +1044,7 @@ __global__ void __launch_bounds__(THREADS) k_emit(TreeDev<T> t, WorkDev w, void 
 		uint4 m1 = v1 ? w.rec[nb + lane] : make_uint4(0, 0, 0, 0);
 		const uint64_t ob1 = nb < total ? claim_output(w, m1.y, __popc(m1.z) + __popc(m1.w), v1) : 0;
 		guard_claim(w, m1, ob1, capacity);
-		emit_blocks<T, HAS_ID, POINTS, U>(t, m0, ob0, v0, s_stage[threadIdx.x >> 5], out);
+		emit_blocks<T, HAS_ID, POINTS, U>(t, m0, ob0, v0, s_warp[threadIdx.x >> 5], out);
 		wb = nb;
 		v0 = v1;
 		m0 = m1;
@@ -1002,7 +1055,7 @@ __global__ void __launch_bounds__(THREADS) k_emit(TreeDev<T> t, WorkDev w, void 
 		uint4 mine = valid ? w.ro[wb + lane] : make_uint4(0, 0, 0, 0);
 		const uint64_t ob = claim_output(w, mine.y, __popc(mine.z) + __popc(mine.w), valid);
 		guard_claim(w, mine, ob, capacity);
-		emit_blocks<T, HAS_ID, POINTS, U>(t, mine, ob, valid, s_stage[threadIdx.x >> 5], out);
+		emit_blocks<T, HAS_ID, POINTS, U>(t, mine, ob, valid, s_warp[threadIdx.x >> 5], out);
 	}
 }
 
