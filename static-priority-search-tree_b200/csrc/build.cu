@@ -926,8 +926,7 @@ T *as(void *p)
 	return static_cast<T *>(p);
 }
 
-// All construction scratch lives in one device allocation (one cudaMalloc maps it
-// far faster than a dozen stream-ordered allocations that regrow a trimmed pool).
+// All construction scratch lives in one device allocation.
 struct ScratchLayout {
 	size_t k1, kalt, c2, valt, k2, v32a, v32b, P, rs_status, rs_misc, hist1, flags, Ba, Bb, best, top, taken, tmax;
 	size_t total;
@@ -972,20 +971,16 @@ ScratchLayout scratch_layout(pst_dtype dt, pst_idtype it, uint64_t n)
 }
 
 struct Scratch {
-	char *base = nullptr;
-	explicit Scratch(size_t bytes)
+	cudaStream_t s;
+	char *base;
+	Scratch(size_t bytes, cudaStream_t stream)
+	    : s(stream), base(static_cast<char *>(pool_alloc(bytes, "construction scratch")))
 	{
-		cudaError_t e = cudaMalloc(&base, std::max<size_t>(bytes, 256));
-		if (e == cudaErrorMemoryAllocation) {
-			cudaGetLastError();
-			fail(PST_ERR_NOMEM, "construction scratch allocation of " + std::to_string(bytes) + " B failed");
-		}
-		check_cuda(e, "cudaMalloc(construction scratch)");
 	}
 	~Scratch()
 	{
-		if (base)
-			cudaFree(base);  // waits for the construction's work
+		cudaStreamSynchronize(s);  // the construction's work
+		pool_release(base, device_info().device);
 	}
 	Scratch(const Scratch &) = delete;
 	Scratch &operator=(const Scratch &) = delete;
@@ -1012,14 +1007,7 @@ uint64_t build_scratch_bytes(pst_dtype dt, pst_idtype it, uint64_t n) { return s
 void alloc_tree(TreeStorage &t, cudaStream_t s)
 {
 	const TreeLayout L = tree_layout(t.dtype, t.idtype, t.n);
-	cudaError_t e = cudaMalloc(&t.mem, L.total);
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		t.mem = nullptr;
-		fail(PST_ERR_NOMEM, "tree allocation of " + std::to_string(L.total) + " B failed");
-	}
-	check_cuda(e, "cudaMalloc(tree)");
-	attach_tree_memory(t, t.mem);
+	attach_tree_memory(t, pool_alloc(L.total, "tree"));
 	PST_CUDA(cudaMemsetAsync(t.occ, 0, L.total - L.off_occ, s));
 }
 
@@ -1034,7 +1022,7 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 
 	// ---- scratch
 	const ScratchLayout SL = scratch_layout(t.dtype, t.idtype, n);
-	Scratch scr(SL.total);
+	Scratch scr(SL.total, s);
 	void *k1 = scr.at<void>(SL.k1), *kalt = scr.at<void>(SL.kalt);
 	uint64_t *c2 = scr.at<uint64_t>(SL.c2);
 	void *valt = scr.at<void>(SL.valt);
@@ -1204,7 +1192,7 @@ static uint64_t aux_bytes(pst_dtype dt, uint64_t n)
 	const uint32_t D = tree_levels(n);
 	if (D < 8)
 		return 0;
-	const uint64_t last_par = ((1ull << (D - 2)) / 64 + 31) / 32 * 4;
+	const uint64_t last_par = align_up(((1ull << (D - 2)) / 64 + 31) / 32 * 4);
 	return last_par + (1ull << (D - 1)) / 64 * value_size(dt);
 }
 
@@ -1353,24 +1341,16 @@ void finish_tree_aux(TreeStorage &t, cudaStream_t s)
 	const uint32_t L = t.levels - 2;
 	const uint64_t nb = (1ull << L) / 64;
 	const uint64_t words = (nb + 31) / 32;
-	cudaError_t e = cudaMalloc(&t.last_par, words * 4);
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		fail(PST_ERR_NOMEM, "search index allocation failed");
-	}
-	check_cuda(e, "cudaMalloc(search index)");
+	const size_t vs = value_size(t.dtype);
+	const size_t par_bytes = align_up(words * 4);
+	t.aux = pool_alloc(par_bytes + ((1ull << (t.levels - 1)) / 64) * vs, "search index");
+	t.last_par = static_cast<uint32_t *>(t.aux);
+	t.sub_min = static_cast<char *>(t.aux) + par_bytes;
 	const unsigned g = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((nb + 255) / 256, 65535));
 	k_last_par<<<g, 256, 0, s>>>(t.occ, L, t.last_par);
 	PST_CUDA(cudaGetLastError());
 	// sub_min: one value per 64-slot block of positions [64, 2^(D-1)), levels
 	// 6..D-2, built from the bottom up
-	const size_t vs = value_size(t.dtype);
-	e = cudaMalloc(&t.sub_min, ((1ull << (t.levels - 1)) / 64) * vs);
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		fail(PST_ERR_NOMEM, "search index allocation failed");
-	}
-	check_cuda(e, "cudaMalloc(search index)");
 	for (uint32_t lv = t.levels - 2; lv >= 6; lv--) {
 		const uint64_t warps = (1ull << lv) / 64;
 		const unsigned gb = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((warps * 32 + 255) / 256, 1u << 20));
@@ -1394,14 +1374,12 @@ void finish_tree_aux(TreeStorage &t, cudaStream_t s)
 
 void free_tree(TreeStorage &t)
 {
-	if (t.mem)
-		cudaFree(t.mem);
+	t.passes->wait_all();  // asynchronous passes may still read the tree
+	pool_release(t.mem, t.device);
 	t.mem = nullptr;
-	if (t.last_par)
-		cudaFree(t.last_par);
+	pool_release(t.aux, t.device);
+	t.aux = nullptr;
 	t.last_par = nullptr;
-	if (t.sub_min)
-		cudaFree(t.sub_min);
 	t.sub_min = nullptr;
 }
 

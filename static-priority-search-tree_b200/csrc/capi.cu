@@ -513,6 +513,7 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 				           "copy offsets");
 			if (total)
 				check_cuda(cudaMemcpyAsync(total, &b.ctl->total, 8, cudaMemcpyDeviceToHost, s), "copy total");
+			b.mark_async(s);
 		}
 	});
 	if (st != PST_OK)

@@ -374,18 +374,16 @@ uint64_t mc_run(const float *vol, const uint32_t P[3], const uint32_t mc[3], con
 	const McGrid g = make_grid(P, mc);
 	uint64_t *counts = nullptr, *offsets = nullptr, *scan = nullptr, *total_d = nullptr;
 	const size_t tmp = scan_tmp_elems(n) * 8;
-	char *buf = nullptr;
 	const size_t bytes = n * 8 + (n + 1) * 8 + tmp + 64;
-	cudaError_t e = cudaMallocAsync((void **) &buf, bytes, s);
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		fail(PST_ERR_NOMEM, "marching-cubes scratch of " + std::to_string(bytes) + " B failed");
-	}
-	check_cuda(e, "cudaMallocAsync(marching cubes)");
+	char *buf = static_cast<char *>(pool_alloc(bytes, "marching-cubes scratch"));
 	struct Free {
 		char *p;
 		cudaStream_t s;
-		~Free() { cudaFreeAsync(p, s); }
+		~Free()
+		{
+			cudaStreamSynchronize(s);
+			pool_release(p, device_info().device);
+		}
 	} fr{buf, s};
 	offsets = reinterpret_cast<uint64_t *>(buf);
 	scan = reinterpret_cast<uint64_t *>(buf + (n + 1) * 8);

@@ -1,0 +1,41 @@
+// Device memory of the library's own objects (trees, engines, scratch): freed blocks are
+// kept, up to a bound, for the next object of about their size.
+#pragma once
+
+#include <map>
+#include <mutex>
+
+#include "common.cuh"
+
+namespace pst {
+
+// Memory on the current device, ready for any stream; fails with PST_ERR_NOMEM, naming
+// `what`.
+void *pool_alloc(size_t bytes, const char *what);
+// Frees p of `device`, which no work queued anywhere may still use.  p may be null.
+void pool_release(void *p, int device) noexcept;
+// Gives the blocks kept on the current device back.
+void pool_trim() noexcept;
+
+// Unique id of the calling thread's current context on device `dev`, made current when
+// the thread has none.
+unsigned long long current_context_id(int dev);
+
+// The asynchronous passes over one tree that may still be running, one event per
+// engine.  The tree and its engines share it, so either may be destroyed first: an
+// engine waits for its own pass, a tree for all of them, before its memory is freed.
+class InFlight {
+  public:
+	// Marks the end of the work queued on `s` for `owner` (after its earlier mark, which
+	// may lie on another stream).
+	void mark(const void *owner, cudaStream_t s);
+	void wait(const void *owner) noexcept;  // and forget it
+	void wait_all() noexcept;
+	~InFlight();
+
+  private:
+	std::mutex mu;
+	std::map<const void *, cudaEvent_t> ev;
+};
+
+}  // namespace pst

@@ -30,8 +30,6 @@
 #include <type_traits>
 #include <vector>
 
-#include <cuda.h>
-
 #include "scan_sort.cuh"
 #include "search.cuh"
 
@@ -1231,11 +1229,11 @@ void Batch::release()
 {
 	full_graph.drop();
 	top_graph.drop();
-	for (void *p : {(void *) q_raw, (void *) kind, min1, max1, min2, (void *) path0, (void *) path1, (void *) seed0,
-	                (void *) seed1, (void *) ro, (void *) counts, (void *) cursor, (void *) offsets, (void *) scan_tmp,
-	                (void *) ctl, (void *) rec})
-		if (p)
-			cudaFree(p);
+	if (passes)
+		passes->wait(this);  // an asynchronous pass may still use the buffers
+	pool_release(work, device);
+	pool_release(rec, device);
+	work = nullptr;
 	if (ctl_host)
 		cudaFreeHost(ctl_host);
 	if (q_stage)
@@ -1247,19 +1245,11 @@ void Batch::release()
 	rec = nullptr;
 }
 
-static void dmalloc(void **p, size_t bytes)
-{
-	cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		fail(PST_ERR_NOMEM, "batch workspace allocation of " + std::to_string(bytes) + " B failed");
-	}
-	check_cuda(e, "cudaMalloc(batch)");
-}
-
 void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 {
 	tree = t;
+	passes = t->passes;
+	device = device_info().device;
 	max_q = std::max<uint32_t>(o.max_queries, 1);
 	use_graph = o.use_graph != 0;
 	threads = o.block_threads ? o.block_threads : BFS_THREADS;
@@ -1285,45 +1275,55 @@ void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 	const size_t vs = value_size(t->dtype);
 	path_cap = 2 * max_q;
 	ro_cap = 2 * max_q * 32;
-	dmalloc((void **) &q_raw, (size_t) max_q * sizeof(pst_query));
-	dmalloc((void **) &kind, (size_t) max_q * 4);
-	dmalloc(&min1, (size_t) max_q * vs);
-	dmalloc(&max1, (size_t) max_q * vs);
-	dmalloc(&min2, (size_t) max_q * vs);
-	dmalloc((void **) &path0, (size_t) path_cap * sizeof(uint4));
-	dmalloc((void **) &path1, (size_t) path_cap * sizeof(uint4));
-	dmalloc((void **) &seed0, (size_t) path_cap * sizeof(uint4));
-	dmalloc((void **) &seed1, (size_t) path_cap * sizeof(uint4));
-	dmalloc((void **) &ro, (size_t) ro_cap * sizeof(uint4));
-	dmalloc((void **) &counts, (size_t) max_q * 8);
-	dmalloc((void **) &cursor, (size_t) max_q * 8);
-	dmalloc((void **) &offsets, ((size_t) max_q + 1) * 8);
-	dmalloc((void **) &scan_tmp, scan_tmp_elems(max_q) * 8);
-	dmalloc((void **) &ctl, sizeof(BatchCtl));
+	{
+		// laid out twice: once for the size, once for the addresses
+		size_t off = 0;
+		auto take = [&](auto **p, size_t bytes) {
+			if (work)
+				*p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(static_cast<char *>(work) + off);
+			off += (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
+		};
+		auto layout = [&] {
+			off = 0;
+			take(&q_raw, (size_t) max_q * sizeof(pst_query));
+			take(&kind, (size_t) max_q * 4);
+			take(&min1, (size_t) max_q * vs);
+			take(&max1, (size_t) max_q * vs);
+			take(&min2, (size_t) max_q * vs);
+			take(&path0, (size_t) path_cap * sizeof(uint4));
+			take(&path1, (size_t) path_cap * sizeof(uint4));
+			take(&seed0, (size_t) path_cap * sizeof(uint4));
+			take(&seed1, (size_t) path_cap * sizeof(uint4));
+			take(&ro, (size_t) ro_cap * sizeof(uint4));
+			take(&counts, (size_t) max_q * 8);
+			take(&cursor, (size_t) max_q * 8);
+			take(&offsets, ((size_t) max_q + 1) * 8);
+			take(&scan_tmp, scan_tmp_elems(max_q) * 8);
+			take(&ctl, sizeof(BatchCtl));
+		};
+		layout();
+		work = pool_alloc(off, "batch workspace");
+		layout();
+	}
 	PST_CUDA(cudaMallocHost((void **) &ctl_host, sizeof(BatchCtl)));
 	PST_CUDA(cudaMallocHost((void **) &q_stage, (size_t) max_q * sizeof(pst_query)));
 	memset(ctl_host, 0, sizeof(BatchCtl));
 	PST_CUDA(cudaHostGetDevicePointer((void **) &ctl_host_d, ctl_host, 0));
 	const uint64_t want = o.task_capacity ? o.task_capacity : std::max<uint64_t>(1ull << 16, (uint64_t) max_q * 64);
-	grow_tasks(want, 0);
-	PST_CUDA(cudaStreamSynchronize(0));
+	rec = static_cast<uint4 *>(pool_alloc(want * sizeof(uint4), "frontier"));
+	task_cap = want;
 }
 
 void Batch::grow_tasks(uint64_t cap, cudaStream_t s)
 {
-	// Stream-ordered on `s` (the stream of every pass that used the old frontier), so
-	// a growth does not wait for work on the device's other streams.
-	if (rec)
-		PST_CUDA(cudaFreeAsync(rec, s));
+	// Only the passes that used the old frontier are waited for (those on `s`, and an
+	// asynchronous one), not work on the device's other streams.
+	PST_CUDA(cudaStreamSynchronize(s));
+	passes->wait(this);
+	pool_release(rec, device);
 	rec = nullptr;
-	const size_t bytes = std::max<size_t>(cap * sizeof(uint4), 16);
-	cudaError_t e = cudaMallocAsync((void **) &rec, bytes, s);
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		task_cap = 0;
-		fail(PST_ERR_NOMEM, "frontier allocation of " + std::to_string(bytes) + " B failed");
-	}
-	check_cuda(e, "cudaMallocAsync(frontier)");
+	task_cap = 0;
+	rec = static_cast<uint4 *>(pool_alloc(cap * sizeof(uint4), "frontier"));
 	task_cap = cap;
 	// the captured passes hold the old frontier's address
 	full_graph.drop();
@@ -1632,44 +1632,6 @@ struct NoallocSlot {
 	unsigned char *ptr = nullptr;
 };
 NoallocSlot g_noalloc_slot[64];
-
-using CtxGetCurrentFn = CUresult (*)(CUcontext *);
-using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long *);
-
-// Unique id of the calling thread's current context, made current first for device
-// `dev` when the thread has none yet (the library does not link the driver library
-// itself: the two driver calls come from the runtime's entry points).
-unsigned long long current_context_id(int dev)
-{
-	static CtxGetCurrentFn get_cur = nullptr;
-	static CtxGetIdFn get_id = nullptr;
-	static std::once_flag once;
-	std::call_once(once, [] {
-		void *p = nullptr;
-		cudaDriverEntryPointQueryResult q{};
-		if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
-		    q == cudaDriverEntryPointSuccess)
-			get_cur = reinterpret_cast<CtxGetCurrentFn>(p);
-		p = nullptr;
-		if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
-		    q == cudaDriverEntryPointSuccess)
-			get_id = reinterpret_cast<CtxGetIdFn>(p);
-		cudaGetLastError();
-	});
-	if (!get_cur || !get_id)
-		fail(PST_ERR_CUDA, "driver entry points cuCtxGetCurrent / cuCtxGetId are unavailable");
-	CUcontext c = nullptr;
-	if (get_cur(&c) == CUDA_SUCCESS && !c) {
-		// a thread that has made no other CUDA call: cudaSetDevice makes the device's
-		// primary context current on it
-		check_cuda(cudaSetDevice(dev), "cudaSetDevice");
-		get_cur(&c);
-	}
-	unsigned long long id = 0;
-	if (!c || get_id(c, &id) != CUDA_SUCCESS)
-		fail(PST_ERR_CUDA, "no current CUDA context");
-	return id;
-}
 
 // Device address of the scratch array for device `dev`, which must be current
 // (the host-side name of a __device__ array is only a stand-in for it): looked up

@@ -39,6 +39,9 @@ struct BatchCtl {
 
 struct Batch {
 	TreeStorage *tree = nullptr;
+	std::shared_ptr<InFlight> passes;  // the tree's, kept for an engine that outlives it
+	int device = 0;
+	void *work = nullptr;              // one allocation of every buffer below but the frontier
 	uint32_t max_q = 0;
 	bool use_graph = true;
 	uint32_t threads = BFS_THREADS;  // CTA size of the level and emit kernels
@@ -80,6 +83,8 @@ struct Batch {
 	void stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s);
 	// Whole count pass (every level kernel and the scan), asynchronous.
 	void launch_count(cudaStream_t s);
+	// Notes that work queued on `s` may still run when the call returns.
+	void mark_async(cudaStream_t s) { passes->mark(this, s); }
 	// Top pass of a small batch (nq <= top_q), asynchronous: when it stops
 	// above the bottom (ctl->cta_levels < tree levels), launch_count_rest finishes it.
 	void launch_count_top(cudaStream_t s);

@@ -70,14 +70,7 @@ void allocate(TreeStorage &t, uint64_t bytes)
 {
 	if (!bytes)
 		return;
-	void *mem = nullptr;
-	cudaError_t e = cudaMalloc(&mem, bytes);
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		fail(PST_ERR_NOMEM, "tree allocation of " + std::to_string(bytes) + " B failed");
-	}
-	check_cuda(e, "cudaMalloc(tree)");
-	attach_tree_memory(t, mem);
+	attach_tree_memory(t, pool_alloc(bytes, "tree"));
 }
 
 struct PinnedPair {

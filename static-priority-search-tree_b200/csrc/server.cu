@@ -220,6 +220,13 @@ struct Server {
 			cudaGetLastError();
 			return false;
 		}
+		if (bytes + opts.hbm_headroom_bytes <= fr)
+			return true;
+		pool_trim();  // memory the library keeps for reuse counts as free
+		if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+			cudaGetLastError();
+			return false;
+		}
 		return bytes + opts.hbm_headroom_bytes <= fr;
 	}
 

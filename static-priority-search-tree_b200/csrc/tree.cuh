@@ -1,9 +1,11 @@
 // Tree storage and the entry points of construction and search (host side).
 #pragma once
 
+#include <memory>
 #include <mutex>
 
 #include "common.cuh"
+#include "pool.cuh"
 
 namespace pst {
 
@@ -15,18 +17,20 @@ struct TreeStorage {
 	pst_idtype idtype = PST_ID_NONE;
 	uint64_t n = 0;
 	uint32_t levels = 0;
-	void *mem = nullptr;  // single cudaMalloc holding every field
+	void *mem = nullptr;  // one allocation holding every field
 	size_t bytes = 0;
 	void *dim1 = nullptr;
 	void *dim2 = nullptr;
 	void *med = nullptr;
 	uint32_t *id = nullptr;
 	uint32_t *occ = nullptr;
-	uint32_t *last_par = nullptr;  // separate allocation, see TreeDev::last_par
-	void *sub_min = nullptr;       // separate allocation, see TreeDev::sub_min
+	void *aux = nullptr;           // the search indexes' own allocation:
+	uint32_t *last_par = nullptr;  // see TreeDev::last_par
+	void *sub_min = nullptr;       // see TreeDev::sub_min
 	int device = 0;
 	std::mutex mu;        // serialises the single-query engine
 	Batch *single = nullptr;
+	std::shared_ptr<InFlight> passes = std::make_shared<InFlight>();
 
 	template <typename T>
 	TreeDev<T> view() const
