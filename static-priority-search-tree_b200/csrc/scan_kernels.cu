@@ -1,6 +1,7 @@
 // Streaming kernels: the interval parallel search comparator and metacell formation.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "scan_kernels.cuh"
@@ -162,6 +163,21 @@ __device__ __forceinline__ void plane_minmax(const T *__restrict__ vol, uint64_t
 	}
 }
 
+// Minimum and maximum of the vertices [x0, x1] x [y0, y1] x [z0, z1], plane by plane, as
+// k_metacells folds them.
+template <typename T>
+__device__ __noinline__ void metacell_fold(const T *__restrict__ vol, uint64_t px, uint64_t py, uint32_t x0,
+                                           uint32_t x1, uint32_t y0, uint32_t y1, uint32_t z0, uint32_t z1, T &lo, T &hi)
+{
+	plane_minmax(vol, px, py, z0, x0, x1, y0, y1, lo, hi);
+	for (uint32_t z = z0 + 1; z <= z1; z++) {
+		T pl, ph;
+		plane_minmax(vol, px, py, z, x0, x1, y0, y1, pl, ph);
+		lo = pl < lo ? pl : lo;
+		hi = ph > hi ? ph : hi;
+	}
+}
+
 // Metacell layers [mz_begin, mz_end); `vol` holds the vertex planes from z_base on
 // (the whole volume: z_base = 0; one z-slab of it: its first plane).
 template <typename T, bool HAS_ID>
@@ -204,10 +220,206 @@ __global__ void k_metacells(const T *__restrict__ vol, uint32_t px, uint32_t py,
 	}
 }
 
+// Metacells wider than one vertex, over rows of any length and alignment: a thread owns a
+// vertex column (consecutive threads read consecutive vertices), folds it over the rows
+// and planes of GROUP metacell rows, and only then are the columns of a metacell folded
+// with one another, through shared memory.  Every vertex is loaded once per CTA, and
+// what two CTAs share comes from L2; the rows of a plane are independent loads (sides of
+// 1 to 8 rows are compiled in).  With a thread per metacell a row's lanes are mcx
+// vertices apart and load them one by one: 509 x 381 x 263 f32 vertices took 130 us in
+// 4^3 metacells, 130 in 2^3 and 465 in 8^3; by columns 66, 105 and 58 us (3.3, 2.7 and
+// 3.5 TB/s).  A copy that loads the next plane's rows before it folds a plane was slower
+// (97 us for 4^3: the second set of registers spills).
+//
+// Folding columns first takes a metacell's values in another order than vertex after
+// vertex, which matters where two values compare equal and differ (-0.0 and +0.0) or
+// do not compare (NaN).  Where a result could show that, the metacell is folded again in
+// that order (metacell_fold).
+template <typename T, int MCY>  // MCY 0: any number of rows, eight at a time
+struct ColumnShape {
+	// metacell rows of a CTA, and the vertex rows it loads together
+	static constexpr int GROUP = MCY == 0 ? 1 : MCY == 1 ? 4 : (sizeof(T) == 4 ? 8 : 4) / MCY > 1 ? (sizeof(T) == 4 ? 8 : 4) / MCY : 1;
+	static constexpr int ROWS = MCY ? GROUP * MCY + 1 : 8;
+};
+
+// Threads of a CTA: a row of 512 vertices and the one past its last metacell fit.
+constexpr int MC_COL_THREADS = 544;
+
+// The folds of a column.  For floats in one instruction each: NaN if any value is one, and
+// -0.0 below +0.0.
+__device__ __forceinline__ float fold_min(float a, float b)
+{
+	float r;
+	asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+__device__ __forceinline__ float fold_max(float a, float b)
+{
+	float r;
+	asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+__device__ __forceinline__ int32_t fold_min(int32_t a, int32_t b) { return min(a, b); }
+__device__ __forceinline__ int32_t fold_max(int32_t a, int32_t b) { return max(a, b); }
+__device__ __forceinline__ double fold_min(double a, double b) { return b < a ? b : a; }
+__device__ __forceinline__ double fold_max(double a, double b) { return b > a ? b : a; }
+
+// Whether the order of a fold over these values could show in its result.  Doubles are
+// asked one by one; a float's folds tell by themselves: a minimum of +0.0 means that no
+// -0.0 was there, and a maximum of -0.0 that no +0.0 was.
+__device__ __forceinline__ bool order_shows(double v)
+{
+	return v != v || (unsigned long long) __double_as_longlong(v) == 0x8000000000000000ull;
+}
+template <typename T>
+__device__ __forceinline__ bool order_shows(T) { return false; }
+template <typename T>
+__device__ __forceinline__ bool order_shows(T, T) { return false; }
+__device__ __forceinline__ bool order_shows(float lo, float hi)
+{
+	return lo != lo || hi != hi || __float_as_uint(lo) == 0x80000000u || (__float_as_uint(hi) == 0u && lo < 0.0f);
+}
+
+template <typename T, bool HAS_ID, int MCY>
+__global__ void __launch_bounds__(MC_COL_THREADS, 2) k_metacells_cols(
+    const T *__restrict__ vol, uint32_t px, uint32_t py, uint32_t pz, uint32_t mcx, uint32_t mcy, uint32_t mcz,
+    uint32_t span, uint32_t Mx, uint32_t My, uint32_t mz_begin, uint32_t mz_end, uint32_t z_base,
+    uint32_t mz_per_cta, Point<T, HAS_ID> *__restrict__ out)
+{
+	constexpr int GROUP = ColumnShape<T, MCY>::GROUP, ROWS = ColumnShape<T, MCY>::ROWS;
+	__shared__ T s_lo[GROUP][MC_COL_THREADS], s_hi[GROUP][MC_COL_THREADS];
+	__shared__ bool s_mark[sizeof(T) == 8 ? MC_COL_THREADS : 1];
+	__shared__ Point<T, HAS_ID> s_out[MC_COL_THREADS];
+	const uint32_t chunks = (span + 31) / 32;
+	const uint32_t mx0 = blockIdx.x * span, my0 = blockIdx.y * GROUP;  // span: metacells of the CTA along x
+	const uint32_t y0 = my0 * mcy;
+	const uint32_t mz0 = mz_begin + blockIdx.z * mz_per_cta, mz1 = min(mz0 + mz_per_cta, mz_end);
+	// the column's vertices, as offsets from the plane's row y0 (rows and columns past the
+	// volume repeat its last one, as the last vertices of a cut metacell do)
+	const uint32_t dx = min(mx0 * mcx + threadIdx.x, px - 1);
+	const uint32_t row_last = min(GROUP * mcy, py - 1 - y0);
+	uint32_t off[ROWS];
+#pragma unroll
+	for (int r = 0; r < ROWS; r++)
+		off[r] = min((uint32_t) r, row_last) * px + dx;
+	T lo[GROUP], hi[GROUP], plo[GROUP], phi[GROUP];
+	bool mark = false, pmark = false;
+	// plane z's folds into plo, phi, pmark
+	auto plane = [&](uint32_t z) {
+		const T *p = vol + ((uint64_t) (z - z_base) * py + y0) * px;
+		T v[ROWS];
+#pragma unroll
+		for (int r = 0; r < ROWS; r++)
+			v[r] = p[off[r]];
+		pmark = false;
+#pragma unroll
+		for (int r = 0; r < ROWS; r++)
+			pmark |= order_shows(v[r]);
+#pragma unroll
+		for (int g = 0; g < GROUP; g++) {
+			plo[g] = phi[g] = v[g * MCY];
+#pragma unroll
+			for (int k = 1; k < (MCY ? MCY + 1 : ROWS); k++) {
+				plo[g] = fold_min(plo[g], v[g * MCY + k]);
+				phi[g] = fold_max(phi[g], v[g * MCY + k]);
+			}
+		}
+		if constexpr (MCY == 0) {
+			for (uint32_t r0 = ROWS; r0 <= row_last; r0 += ROWS) {
+#pragma unroll
+				for (int r = 0; r < ROWS; r++)
+					v[r] = p[min(r0 + r, row_last) * px + dx];
+#pragma unroll
+				for (int r = 0; r < ROWS; r++) {
+					pmark |= order_shows(v[r]);
+					plo[0] = fold_min(plo[0], v[r]);
+					phi[0] = fold_max(phi[0], v[r]);
+				}
+			}
+		}
+	};
+	plane(mz0 * mcz);
+	for (uint32_t mz = mz0; mz < mz1; mz++) {
+		const uint32_t z0 = mz * mcz, z1 = min(z0 + mcz, pz - 1);
+		mark = pmark;
+#pragma unroll
+		for (int g = 0; g < GROUP; g++) {
+			lo[g] = plo[g];  // the plane shared with the layer below
+			hi[g] = phi[g];
+		}
+#pragma unroll(sizeof(T) == 4 ? 2 : 1)
+		for (uint32_t z = z0 + 1; z <= z1; z++) {
+			plane(z);
+			mark |= pmark;
+#pragma unroll
+			for (int g = 0; g < GROUP; g++) {
+				lo[g] = fold_min(lo[g], plo[g]);
+				hi[g] = fold_max(hi[g], phi[g]);
+			}
+		}
+#pragma unroll
+		for (int g = 0; g < GROUP; g++) {
+			s_lo[g][threadIdx.x] = lo[g];
+			s_hi[g][threadIdx.x] = hi[g];
+		}
+		if constexpr (sizeof(T) == 8)
+			s_mark[threadIdx.x] = mark;
+		__syncthreads();
+		// a warp takes 32 consecutive metacells of a row, whose records leave as consecutive
+		// words
+		for (uint32_t t = threadIdx.x >> 5; t < GROUP * chunks; t += blockDim.x >> 5) {
+			const uint32_t g = t / chunks, m0 = (t - g * chunks) * 32, c = (m0 + lane_id()) * mcx;
+			const uint32_t mx = mx0 + m0 + lane_id(), my = my0 + g;
+			if (my >= My || mx0 + m0 >= Mx)
+				continue;
+			const uint32_t count = min(min(span - m0, Mx - (mx0 + m0)), 32u);
+			const uint64_t id0 = (uint64_t) (mx0 + m0) + ((uint64_t) my + (uint64_t) mz * My) * Mx;
+			if (lane_id() < count) {
+				T l = s_lo[g][c], h = s_hi[g][c];
+				bool m = sizeof(T) == 8 && s_mark[c];
+				auto next = [&](uint32_t k) {
+					l = fold_min(l, s_lo[g][c + k]);
+					h = fold_max(h, s_hi[g][c + k]);
+					if constexpr (sizeof(T) == 8)
+						m |= s_mark[c + k];
+				};
+				if (MCY && mcx == (uint32_t) MCY) {
+#pragma unroll
+					for (uint32_t k = 1; k <= (uint32_t) MCY; k++)
+						next(k);
+				} else {
+					for (uint32_t k = 1; k <= mcx; k++)
+						next(k);
+				}
+				if (m || order_shows(l, h))
+					metacell_fold(vol, px, py, mx * mcx, min(mx * mcx + mcx, px - 1), my * mcy,
+					              min(my * mcy + mcy, py - 1), z0 - z_base, z1 - z_base, l, h);
+				Point<T, HAS_ID> &p = s_out[threadIdx.x];
+				p.dim1 = l;
+				p.dim2 = h;
+				if constexpr (HAS_ID && sizeof(T) == 8)
+					*reinterpret_cast<unsigned long long *>(&p.id) = (uint32_t) id0 + lane_id();  // with its padding
+				else if constexpr (HAS_ID)
+					p.id = (uint32_t) id0 + lane_id();
+			}
+			__syncwarp();
+			using W = typename std::conditional<sizeof(T) == 8, unsigned long long, uint32_t>::type;
+			const W *src = reinterpret_cast<const W *>(s_out + (threadIdx.x & ~31u));
+			W *dst = reinterpret_cast<W *>(out + id0);
+			for (uint32_t i = lane_id(); i < count * (uint32_t) (sizeof(Point<T, HAS_ID>) / sizeof(W)); i += 32)
+				dst[i] = src[i];
+			__syncwarp();  // the warp's records are rewritten by its next 32
+		}
+		__syncthreads();  // the columns are rewritten by the next layer
+	}
+}
+
 // The common layout: metacells 4 vertices wide over 4-byte values, rows a multiple of
 // 4 vertices long, the volume 16-byte aligned.  A metacell's 4 low vertices of a row
 // are one aligned 16-byte load; its fifth (the next metacell's first) comes from the
-// next lane, or from memory for a warp's last metacell.  Same walk as k_metacells.
+// next lane, or from memory for a warp's last metacell.  Same walk as k_metacells.  A
+// load brings a whole metacell row, which columns (k_metacells_cols) take four for: 123
+// against 137 us for 512^3 f32 vertices in 4^3 metacells.
 template <typename T>
 struct Quad;
 template <>
@@ -330,30 +542,75 @@ void ips_dispatch(pst_idtype it, pst_ret ret, const void *pts, uint64_t n, T v, 
 	}
 }
 
+// Launch shape of k_metacells_cols: rows of up to 512 vertices a CTA, and in z as many
+// layers a CTA (of at least 16 vertices in all) as leave the device two CTAs an SM.
+template <typename T, bool HAS_ID, int MCY>
+void metacell_cols_launch(const T *vol, const uint32_t P[3], const uint32_t mc[3], const uint32_t M[3],
+                          uint32_t mz_begin, uint32_t mz_end, Point<T, HAS_ID> *out, cudaStream_t s)
+{
+	constexpr uint32_t GROUP = ColumnShape<T, MCY>::GROUP;
+	// as few CTAs along x as hold the row, each with an equal share of it
+	const uint32_t layers = mz_end - mz_begin, most = (MC_COL_THREADS - 1) / mc[0];
+	const uint32_t gx = (M[0] + most - 1) / most, span = (M[0] + gx - 1) / gx;
+	const uint32_t threads = (span * mc[0] + 1 + 31) / 32 * 32;
+	const uint32_t gy = (M[1] + GROUP - 1) / GROUP;
+	uint32_t mzp = std::max(1u, 16 / mc[2]);
+	while (mzp > 1 && (uint64_t) gx * gy * ((layers + mzp - 1) / mzp) < (uint64_t) device_info().sms * 2)
+		mzp /= 2;
+	mzp = std::max(mzp, (layers + 65534) / 65535);
+	const dim3 grid(gx, gy, (layers + mzp - 1) / mzp);
+	k_metacells_cols<T, HAS_ID, MCY><<<grid, threads, 0, s>>>(vol, P[0], P[1], P[2], mc[0], mc[1], mc[2], span,
+	                                                         M[0], M[1], mz_begin, mz_end, mz_begin * mc[2], mzp, out);
+}
+
 template <typename T, bool HAS_ID>
 void metacell_launch(const void *vol, const uint32_t P[3], const uint32_t mc[3], const uint32_t M[3],
                      uint32_t mz_begin, uint32_t mz_end, void *out, cudaStream_t s)
 {
 	if (mz_end <= mz_begin)
 		return;
-	const uint32_t threads = M[0] >= 256 ? 256 : ((M[0] + 31) / 32) * 32;
-	const uint32_t mzp = 8;
-	dim3 grid((M[0] + threads - 1) / threads, M[1], (mz_end - mz_begin + mzp - 1) / mzp);
-	if (grid.y > 65535 || grid.z > 65535)
+	const uint32_t layers = mz_end - mz_begin;
+	if (M[1] > 65535 || (layers + 7) / 8 > 65535)
 		fail(PST_ERR_INVALID, "metacell grid too large");
-	bool quad = false;
-	if constexpr (sizeof(T) == 4)
-		quad = mc[0] == 4 && P[0] % 4 == 0 && (reinterpret_cast<uintptr_t>(vol) & 15u) == 0;
-	if constexpr (sizeof(T) == 4) {
-		if (quad)
-			k_metacells4<T, HAS_ID><<<grid, threads, 0, s>>>(static_cast<const T *>(vol), P[0], P[1], P[2], mc[1], mc[2],
-			                                                 M[0], M[1], mz_begin, mz_end, mz_begin * mc[2], mzp,
-			                                                 static_cast<Point<T, HAS_ID> *>(out));
+	const T *v = static_cast<const T *>(vol);
+	Point<T, HAS_ID> *o = static_cast<Point<T, HAS_ID> *>(out);
+	const uint32_t threads = M[0] >= 256 ? 256 : ((M[0] + 31) / 32) * 32;
+	if (mc[0] == 4 && sizeof(T) == 4 && P[0] % 4 == 0 && (reinterpret_cast<uintptr_t>(vol) & 15u) == 0) {
+		if constexpr (sizeof(T) == 4) {
+			// fewer layers a CTA while the device has room for more threads: a layer's planes
+			// are one chain of loads (128^3 vertices: 65 us with 8 layers a CTA, 16 with one;
+			// 512^3: 129 us with 8, 123 with 2 or 4)
+			const uint32_t gx = (M[0] + threads - 1) / threads;
+			uint32_t mzp = 4;
+			while (mzp > 1 && (uint64_t) gx * threads * M[1] * ((layers + mzp - 1) / mzp) <
+			                      (uint64_t) device_info().sms * 2048)
+				mzp /= 2;
+			mzp = std::max(mzp, (layers + 65534) / 65535);
+			const dim3 grid(gx, M[1], (layers + mzp - 1) / mzp);
+			k_metacells4<T, HAS_ID><<<grid, threads, 0, s>>>(v, P[0], P[1], P[2], mc[1], mc[2], M[0], M[1], mz_begin,
+			                                                 mz_end, mz_begin * mc[2], mzp, o);
+		}
+	} else if (mc[0] == 1 || mc[0] >= (uint32_t) MC_COL_THREADS ||
+	           (uint64_t) P[0] * std::min(P[1], 2 * mc[1]) >= (1ull << 30)) {
+		// one vertex wide (consecutive threads are consecutive vertices already: 970 us for
+		// 512^3 f32 voxels, 1090 by columns), wider than a CTA of columns, or rows too long
+		// for its 32-bit offsets: a thread per metacell
+		const dim3 grid((M[0] + threads - 1) / threads, M[1], (layers + 7) / 8);
+		k_metacells<T, HAS_ID><<<grid, threads, 0, s>>>(v, P[0], P[1], P[2], mc[0], mc[1], mc[2], M[0], M[1], mz_begin,
+		                                                mz_end, mz_begin * mc[2], 8, o);
+	} else {
+		switch (mc[1]) {
+		case 1: metacell_cols_launch<T, HAS_ID, 1>(v, P, mc, M, mz_begin, mz_end, o, s); break;
+		case 2: metacell_cols_launch<T, HAS_ID, 2>(v, P, mc, M, mz_begin, mz_end, o, s); break;
+		case 3: metacell_cols_launch<T, HAS_ID, 3>(v, P, mc, M, mz_begin, mz_end, o, s); break;
+		case 4: metacell_cols_launch<T, HAS_ID, 4>(v, P, mc, M, mz_begin, mz_end, o, s); break;
+		case 5: metacell_cols_launch<T, HAS_ID, 5>(v, P, mc, M, mz_begin, mz_end, o, s); break;
+		case 6: metacell_cols_launch<T, HAS_ID, 6>(v, P, mc, M, mz_begin, mz_end, o, s); break;
+		case 7: metacell_cols_launch<T, HAS_ID, 7>(v, P, mc, M, mz_begin, mz_end, o, s); break;
+		case 8: metacell_cols_launch<T, HAS_ID, 8>(v, P, mc, M, mz_begin, mz_end, o, s); break;
+		default: metacell_cols_launch<T, HAS_ID, 0>(v, P, mc, M, mz_begin, mz_end, o, s);
+		}
 	}
-	if (!quad)
-		k_metacells<T, HAS_ID><<<grid, threads, 0, s>>>(static_cast<const T *>(vol), P[0], P[1], P[2], mc[0], mc[1],
-		                                                mc[2], M[0], M[1], mz_begin, mz_end, mz_begin * mc[2], mzp,
-		                                                static_cast<Point<T, HAS_ID> *>(out));
 	PST_CUDA(cudaGetLastError());
 }
 
