@@ -21,6 +21,10 @@ namespace {
 // blocks stayed in it, but grows by about 8 ms a GB (cudaMalloc: 0.2 ms), which made the
 // build of a 2^28-point tree 117 ms slower.
 constexpr size_t KEEP_SHARE = 32;
+// Pinned host memory kept per device, for the control block and the staged queries of
+// engines: cudaMallocHost and cudaFreeHost took 3.1 and 0.6 ms a call in a process that
+// holds little pinned memory, more than the rest of a 384^3 isosurface pass.
+constexpr size_t KEEP_PINNED = size_t(8) << 20;
 // Requests are rounded up to an eighth of their power of two, so that objects of about
 // one size share blocks, and from BIG on to whole pages only: a tree that just fits the
 // device has to go on fitting it.
@@ -44,11 +48,21 @@ struct Block {
 // One device's blocks, with the context they belong to: cudaDeviceReset ends that
 // context, and its blocks are forgotten at the next call.
 struct Pool {
+	const bool pinned;
 	std::mutex mu;
 	unsigned long long ctx = 0;
 	size_t keep = 0, kept = 0;
 	std::vector<Block> idle;                    // oldest first
 	std::unordered_map<void *, size_t> live;
+
+	explicit Pool(bool host) : pinned(host) {}
+	cudaError_t get(void **ptr, size_t bytes) const { return pinned ? cudaMallocHost(ptr, bytes) : cudaMalloc(ptr, bytes); }
+	void give_back(const std::vector<Block> &blocks) const noexcept
+	{
+		for (const Block &b : blocks)
+			if ((pinned ? cudaFreeHost(b.ptr) : cudaFree(b.ptr)) != cudaSuccess)
+				cudaGetLastError();
+	}
 
 	// (with mu held)
 	void enter(unsigned long long now)
@@ -60,7 +74,7 @@ struct Pool {
 		kept = 0;
 		size_t fr = 0, total = 0;
 		check_cuda(cudaMemGetInfo(&fr, &total), "cudaMemGetInfo");
-		keep = total / KEEP_SHARE;
+		keep = pinned ? KEEP_PINNED : total / KEEP_SHARE;
 		ctx = now;
 	}
 
@@ -93,9 +107,14 @@ struct Pool {
 		return out;
 	}
 };
-Pool g_pools[64];
 
-Pool &pool_of(int dev)
+// The pools of every device.
+struct Pools {
+	Pool mem{false}, pinned{true};
+};
+Pools g_pools[64];
+
+Pools &pools_of(int dev)
 {
 	if (dev < 0 || dev >= 64)
 		fail(PST_ERR_CUDA, "device index out of range");
@@ -107,13 +126,6 @@ int current_device()
 	int dev = 0;
 	check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
 	return dev;
-}
-
-void give_back(const std::vector<Block> &blocks)
-{
-	for (const Block &b : blocks)
-		if (cudaFree(b.ptr) != cudaSuccess)
-			cudaGetLastError();
 }
 
 }  // namespace
@@ -155,11 +167,11 @@ unsigned long long current_context_id(int dev)
 	return id;
 }
 
-void *pool_alloc(size_t bytes, const char *what)
+namespace {
+
+void *alloc_in(Pool &p, int dev, size_t bytes, const char *what)
 {
-	const int dev = current_device();
 	const unsigned long long ctx = current_context_id(dev);
-	Pool &p = pool_of(dev);
 	const size_t want = block_bytes(bytes);
 	{
 		std::lock_guard<std::mutex> lk(p.mu);
@@ -168,11 +180,11 @@ void *pool_alloc(size_t bytes, const char *what)
 			return ptr;
 	}
 	void *ptr = nullptr;
-	cudaError_t e = cudaMalloc(&ptr, want);
+	cudaError_t e = p.get(&ptr, want);
 	if (e == cudaErrorMemoryAllocation) {
 		cudaGetLastError();
 		pool_trim();
-		e = cudaMalloc(&ptr, want);
+		e = p.get(&ptr, want);
 	}
 	if (e == cudaErrorMemoryAllocation) {
 		cudaGetLastError();
@@ -184,7 +196,42 @@ void *pool_alloc(size_t bytes, const char *what)
 	return ptr;
 }
 
-void pool_release(void *ptr, int device) noexcept
+void release_in(Pool &p, int dev, void *ptr)
+{
+	std::vector<Block> out;
+	{
+		const unsigned long long ctx = current_context_id(dev);
+		std::lock_guard<std::mutex> lk(p.mu);
+		p.enter(ctx);
+		const auto it = p.live.find(ptr);
+		if (it == p.live.end())
+			return;  // a block of a context that is gone went with it
+		const Block b{ptr, it->second};
+		p.live.erase(it);
+		if (b.bytes > p.keep) {
+			out.push_back(b);
+		} else {
+			p.idle.push_back(b);
+			p.kept += b.bytes;
+			out = p.shrink(p.keep);
+		}
+	}
+	p.give_back(out);
+}
+
+void trim(Pool &p, int dev)
+{
+	std::vector<Block> out;
+	{
+		const unsigned long long ctx = current_context_id(dev);
+		std::lock_guard<std::mutex> lk(p.mu);
+		p.enter(ctx);
+		out = p.shrink(0);
+	}
+	p.give_back(out);
+}
+
+void release_on(bool pinned, void *ptr, int device) noexcept
 {
 	if (!ptr)
 		return;
@@ -192,26 +239,7 @@ void pool_release(void *ptr, int device) noexcept
 		const int cur = current_device();
 		if (cur != device)
 			check_cuda(cudaSetDevice(device), "cudaSetDevice");
-		Pool &p = pool_of(device);
-		std::vector<Block> out;
-		{
-			const unsigned long long ctx = current_context_id(device);
-			std::lock_guard<std::mutex> lk(p.mu);
-			p.enter(ctx);
-			const auto it = p.live.find(ptr);
-			if (it != p.live.end()) {  // (a block of a context that is gone went with it)
-				const Block b{ptr, it->second};
-				p.live.erase(it);
-				if (b.bytes > p.keep) {
-					out.push_back(b);
-				} else {
-					p.idle.push_back(b);
-					p.kept += b.bytes;
-					out = p.shrink(p.keep);
-				}
-			}
-		}
-		give_back(out);
+		release_in(pinned ? pools_of(device).pinned : pools_of(device).mem, device, ptr);
 		if (cur != device)
 			cudaSetDevice(cur);
 	} catch (...) {
@@ -219,19 +247,29 @@ void pool_release(void *ptr, int device) noexcept
 	}
 }
 
+}  // namespace
+
+void *pool_alloc(size_t bytes, const char *what)
+{
+	const int dev = current_device();
+	return alloc_in(pools_of(dev).mem, dev, bytes, what);
+}
+
+void *pinned_alloc(size_t bytes, const char *what)
+{
+	const int dev = current_device();
+	return alloc_in(pools_of(dev).pinned, dev, bytes, what);
+}
+
+void pool_release(void *ptr, int device) noexcept { release_on(false, ptr, device); }
+void pinned_release(void *ptr, int device) noexcept { release_on(true, ptr, device); }
+
 void pool_trim() noexcept
 {
 	try {
 		const int dev = current_device();
-		const unsigned long long ctx = current_context_id(dev);
-		Pool &p = pool_of(dev);
-		std::vector<Block> out;
-		{
-			std::lock_guard<std::mutex> lk(p.mu);
-			p.enter(ctx);
-			out = p.shrink(0);
-		}
-		give_back(out);
+		trim(pools_of(dev).mem, dev);
+		trim(pools_of(dev).pinned, dev);
 	} catch (...) {
 		cudaGetLastError();
 	}

@@ -14,6 +14,9 @@ namespace pst {
 void *pool_alloc(size_t bytes, const char *what);
 // Frees p of `device`, which no work queued anywhere may still use.  p may be null.
 void pool_release(void *p, int device) noexcept;
+// The same for pinned host memory (mapped, as cudaMallocHost gives it).
+void *pinned_alloc(size_t bytes, const char *what);
+void pinned_release(void *p, int device) noexcept;
 // Gives the blocks kept on the current device back.
 void pool_trim() noexcept;
 

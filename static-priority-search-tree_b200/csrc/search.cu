@@ -1234,10 +1234,7 @@ void Batch::release()
 	pool_release(work, device);
 	pool_release(rec, device);
 	work = nullptr;
-	if (ctl_host)
-		cudaFreeHost(ctl_host);
-	if (q_stage)
-		cudaFreeHost(q_stage);
+	pinned_release(ctl_host, device);  // the staged queries lie behind the control block
 	q_raw = nullptr;
 	ctl_host = nullptr;
 	ctl_host_d = nullptr;
@@ -1305,8 +1302,8 @@ void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 		work = pool_alloc(off, "batch workspace");
 		layout();
 	}
-	PST_CUDA(cudaMallocHost((void **) &ctl_host, sizeof(BatchCtl)));
-	PST_CUDA(cudaMallocHost((void **) &q_stage, (size_t) max_q * sizeof(pst_query)));
+	ctl_host = static_cast<BatchCtl *>(pinned_alloc(sizeof(BatchCtl) + (size_t) max_q * sizeof(pst_query), "query staging"));
+	q_stage = reinterpret_cast<pst_query *>(ctl_host + 1);
 	memset(ctl_host, 0, sizeof(BatchCtl));
 	PST_CUDA(cudaHostGetDevicePointer((void **) &ctl_host_d, ctl_host, 0));
 	const uint64_t want = o.task_capacity ? o.task_capacity : std::max<uint64_t>(1ull << 16, (uint64_t) max_q * 64);
@@ -1427,12 +1424,19 @@ void Batch::enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t
 
 void Batch::launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStream_t s)
 {
-	if (!use_graph) {
+	// an engine's first passes on a stream are launched as they are: capturing one and
+	// destroying it again takes 310 us, many engines live for a query or two, and a replay
+	// saves 4 us (a top pass) to 60 us of host time (a whole pass)
+	if (!use_graph || g.stream != s || g.direct < DIRECT_PASSES) {
+		if (g.stream != s)
+			g.direct = 0;
+		g.drop();
+		g.direct++;
+		g.stream = s;
 		(this->*enqueue)(s);
 		return;
 	}
-	if (!g.exec || g.stream != s) {
-		g.drop();
+	if (!g.exec) {
 		cudaStream_t cs;
 		PST_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
 		cudaGraph_t gr;
@@ -1448,7 +1452,6 @@ void Batch::launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStr
 		PST_CUDA(cudaGraphInstantiate(&g.exec, gr, 0));
 		cudaGraphDestroy(gr);
 		cudaStreamDestroy(cs);
-		g.stream = s;
 	}
 	PST_CUDA(cudaGraphLaunch(g.exec, s));
 }

@@ -11,6 +11,8 @@ constexpr int BFS_THREADS = 256;
 // walks the upper levels without a kernel boundary between them.
 constexpr uint32_t SMALL_BATCH_Q = 32;
 constexpr uint32_t MAX_TOP_PASS_Q = 1024;
+// Passes of an engine on a stream that are launched kernel by kernel before one is captured.
+constexpr uint32_t DIRECT_PASSES = 4;
 
 enum : uint32_t {
 	BATCH_FLAG_TASK_OVERFLOW = 1u,  // frontier buffer too small (results incomplete)
@@ -72,6 +74,7 @@ struct Batch {
 	struct Graph {
 		cudaGraphExec_t exec = nullptr;
 		cudaStream_t stream = nullptr;
+		uint32_t direct = 0;  // passes launched on `stream` without it
 		void drop();
 	};
 	Graph full_graph, top_graph;
