@@ -17,12 +17,11 @@
 //      4-byte values, (dim2 rank << 32 | tb + 1) for doubles (one extra sort finds
 //      the ranks).  One radix sort by dim1 key carries these keys along, so position
 //      i of the sorted arrays is the i-th point in dim1 order;
-//   2. for the wide top levels, a segmented arg-max over the sorted dim2 keys picks
-//      every node's point of the level at once.  It reads a maximum per 512-position
-//      tile and scans only the tiles cut by a node boundary; points taken by
-//      ancestors are marked in a bitmap, and only the tiles that lost a point are
-//      re-reduced.  A per-node kernel then finds the taken point's position (binary
-//      search on (dim1 key, tb)) and places the median;
+//   2. for the wide top levels, one kernel a level: a warp (or, while nodes are few, a
+//      CTA) per node finds the largest dim2 key of its positions from a maximum per
+//      512-position tile and per 32 tiles and the positions of the tiles that its bounds
+//      cut, takes it out (its key becomes 0), brings the maxima up to date and places
+//      the median;
 //   3. once every node of a level holds at most ST_CAP points, one CTA per node
 //      builds the whole remaining subtree in shared memory.
 #include <algorithm>
@@ -88,12 +87,9 @@ TreeLayout tree_layout(pst_dtype dt, pst_idtype it, uint64_t n)
 #endif
 constexpr uint32_t ST_CAP = PST_SUBTREE_CAP;
 constexpr int ST_THREADS = 256;
-// Arg-max tiles: every segment of a level before the subtree level spans at least
-// ST_CAP >= TM_TILE positions, so a tile is cut by at most one segment boundary.
-constexpr uint32_t TM_TILE = ST_CAP < 512 ? ST_CAP : 512;
-constexpr int AM_THREADS = 256;
-static_assert(ST_CAP >= TM_TILE, "tile/segment invariant");
-static_assert(TM_TILE % 32 == 0, "tiles are whole bitmap words");
+// Arg-max tiles, and the tiles a second maximum covers.
+constexpr uint32_t TM_TILE = 512, TM_SUPER = 32;
+constexpr int LV_THREADS = 256;
 
 // First level whose largest node holds at most ST_CAP points.  Counts within a
 // level take at most two consecutive values (m, m+1).
@@ -109,17 +105,17 @@ uint32_t subtree_level(uint64_t n)
 }
 
 // Sorted arrays, position i = i-th point in dim1 order:
-//   k1s[i]  dim1 key, c2s[i] 64-bit dim2 key (never 0; low 32 bits = tb + 1),
-//   taken   one bit per position, set once the point is stored in a node.
+//   k1s[i]  dim1 key, c2s[i] 64-bit dim2 key (low 32 bits = tb + 1, so never 0) until
+//   the point is stored in a node, then 0.
 template <typename T, bool HAS_ID>
 struct BuildCtx {
 	using K = typename KeyOf<T>::K;
 	const Point<T, HAS_ID> *pts;
 	const uint32_t *P;  // tiebreak rank -> input index (null: identity)
 	const K *k1s;
-	const uint64_t *c2s;
-	uint32_t *taken;
-	uint64_t *tmax;     // per TM_TILE tile: max c2s over positions not taken (0 if none)
+	uint64_t *c2s;
+	uint64_t *tmax;     // per TM_TILE tile: max c2s
+	uint64_t *smax;     // per TM_SUPER tiles: max c2s
 	T *dim1;
 	T *dim2;
 	T *med;
@@ -147,16 +143,15 @@ struct BuildCtx {
 			p.id = tb_of(c2);
 		return p;
 	}
-	__device__ __forceinline__ Point<T, HAS_ID> point_at(uint32_t pos) const
+	// The point at position pos, whose dim2 key is (or was) c2.
+	__device__ __forceinline__ Point<T, HAS_ID> point_of(uint32_t pos, uint64_t c2) const
 	{
 		if constexpr (sizeof(K) == 4) {
 			if (recon)
-				return point_from_keys(k1s[pos], c2s[pos]);
+				return point_from_keys(k1s[pos], c2);
 		}
-		return point_of_tb(tb_of(c2s[pos]));
+		return point_of_tb(tb_of(c2));
 	}
-	__device__ __forceinline__ bool is_taken(uint64_t pos) const { return (taken[pos >> 5] >> (pos & 31)) & 1u; }
-
 	__device__ __forceinline__ void write_node(uint32_t h, const Point<T, HAS_ID> &p) const
 	{
 		dim1[h] = p.dim1;
@@ -165,16 +160,6 @@ struct BuildCtx {
 			id[h] = p.id;
 	}
 };
-
-__device__ __forceinline__ uint64_t warp_max_u64(uint64_t v)
-{
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) {
-		const uint64_t t = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-		v = t > v ? t : v;
-	}
-	return v;
-}
 
 template <typename K>
 __device__ __forceinline__ void atomic_min_key(K *p, K v)
@@ -330,223 +315,238 @@ __global__ void k_rank_keys(const uint32_t *S2, uint64_t n, uint64_t *c2)
 	}
 }
 
+// The node count of node_count in 32 bits (trees hold fewer than 2^31 points).
+__device__ __forceinline__ uint32_t node_count32(uint32_t n, uint32_t d, uint32_t j)
+{
+	uint32_t c = n;
+	for (int b = (int) d - 1; b >= 0 && c != 0; b--)
+		c = ((j >> b) & 1u) ? c - 1u - (c >> 1) : c >> 1;
+	return c;
+}
+
 // ---------------------------------------------------------------------------
 // Wide levels.
 
-// Maximum of c2s over the positions of tile t that are not taken; one warp per tile.
-__device__ __forceinline__ uint64_t tile_max(const uint64_t *__restrict__ c2s, const uint32_t *__restrict__ taken,
-                                             uint64_t n, uint64_t t)
+// The largest of the lanes' 64-bit keys.
+__device__ __forceinline__ uint64_t warp_max_key(uint64_t k)
 {
-	const uint32_t lane = lane_id();
-	const uint64_t t0 = t * TM_TILE;
-	uint64_t m = 0;
-#pragma unroll 4
-	for (uint32_t k = 0; k < TM_TILE / 32; k++) {
-		const uint64_t i = t0 + k * 32 + lane;
-		if (i < n) {
-			const uint32_t w = taken[i >> 5];  // one word per k, the same for the whole warp
-			if (!((w >> lane) & 1u))
-				m = max(m, c2s[i]);
-		}
-	}
-	return warp_max_u64(m);
+	const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, (uint32_t) (k >> 32));
+	const uint32_t lo = __reduce_max_sync(0xFFFFFFFFu, (uint32_t) (k >> 32) == hi ? (uint32_t) k : 0u);
+	return (uint64_t) hi << 32 | lo;
 }
 
-__global__ void __launch_bounds__(AM_THREADS) k_tile_max_all(const uint64_t *__restrict__ c2s,
-                                                             const uint32_t *__restrict__ taken, uint64_t n,
-                                                             uint64_t *tmax)
+// Keys of tile t, lane + 32 k at v[k] (0 past n), all in flight together.
+__device__ __forceinline__ void load_tile(const uint64_t *c2s, uint64_t n, uint64_t t, uint64_t (&v)[TM_TILE / 32])
 {
+	const uint64_t i = t * TM_TILE + lane_id();
+#pragma unroll
+	for (uint32_t k = 0; k < TM_TILE / 32; k++)
+		v[k] = i + 32 * k < n ? c2s[i + 32 * k] : 0ull;
+}
+
+// First maxima: a CTA per TM_SUPER tiles.
+__global__ void __launch_bounds__(LV_THREADS) k_tile_max(const uint64_t *__restrict__ c2s, uint64_t n, uint64_t *tmax,
+                                                         uint64_t *smax)
+{
+	__shared__ uint64_t s_m[LV_THREADS / 32];
 	const uint64_t ntiles = (n + TM_TILE - 1) / TM_TILE;
-	const uint64_t gw = ((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	const uint64_t nw = ((uint64_t) gridDim.x * blockDim.x) >> 5;
-	for (uint64_t t = gw; t < ntiles; t += nw) {
-		const uint64_t m = tile_max(c2s, taken, n, t);
+	const uint32_t warp = threadIdx.x >> 5;
+	uint64_t best = 0;
+	for (uint32_t k = warp; k < TM_SUPER; k += LV_THREADS / 32) {
+		const uint64_t t = (uint64_t) blockIdx.x * TM_SUPER + k;
+		if (t >= ntiles)
+			break;
+		uint64_t v[TM_TILE / 32], m = 0;
+		load_tile(c2s, n, t, v);
+#pragma unroll
+		for (uint32_t i = 0; i < TM_TILE / 32; i++)
+			m = max(m, v[i]);
+		m = warp_max_key(m);
+		best = max(best, m);
 		if (lane_id() == 0)
 			tmax[t] = m;
 	}
-}
-
-// Re-reduces the tiles that lost a point at level d (one warp per node).
-__global__ void __launch_bounds__(AM_THREADS) k_tile_refresh(const uint64_t *__restrict__ c2s,
-                                                             const uint32_t *__restrict__ taken, uint64_t n,
-                                                             const uint32_t *__restrict__ top_pos, uint32_t d,
-                                                             uint64_t *tmax, const uint32_t *err)
-{
-	const uint32_t nseg = 1u << d;
-	const uint64_t gw = ((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	if (gw >= nseg || *err)  // after an error top_pos may hold unwritten entries
-		return;
-	const uint64_t t = top_pos[nseg + gw] / TM_TILE;
-	if (t >= (n + TM_TILE - 1) / TM_TILE)
-		return;
-	const uint64_t m = tile_max(c2s, taken, n, t);
 	if (lane_id() == 0)
-		tmax[t] = m;  // tiles shared by two nodes get the same value twice
-}
-
-// best[s] = max c2s over the positions of [B[s], B[s+1]) not taken.  A thread owns a
-// tile: tiles inside one segment contribute their tmax (one atomic per run of equal
-// segments in a warp); a tile cut by a boundary is scanned by the whole warp.
-__global__ void __launch_bounds__(AM_THREADS) k_level_argmax(const uint64_t *__restrict__ c2s,
-                                                             const uint32_t *__restrict__ taken,
-                                                             const uint64_t *__restrict__ tmax, uint64_t n,
-                                                             const uint32_t *__restrict__ B, uint32_t nseg,
-                                                             unsigned long long *best, const uint32_t *err,
-                                                             float seg_per_pos)
-{
-	if (*err)  // after an error the bounds may hold unwritten entries
-		return;
-	const uint64_t ntiles = (n + TM_TILE - 1) / TM_TILE;
-	const uint32_t lane = lane_id();
-	const uint64_t gw = ((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	const uint64_t nw = ((uint64_t) gridDim.x * blockDim.x) >> 5;
-	for (uint64_t wb = gw * 32; wb < ntiles; wb += nw * 32) {
-		const uint64_t t = wb + lane;
-		const bool valid = t < ntiles;
-		const uint64_t t0 = t * TM_TILE;
-		const uint64_t t1 = valid ? min(t0 + TM_TILE, n) : 0;
-		uint32_t seg = 0xFFFFFFFFu;
-		uint64_t seg_end = 0;
-		if (valid) {
-			// the largest s with B[s] <= t0: the level's segments are all within a few
-			// positions of n / nseg long, so s lies next to t0 * nseg / n and a short
-			// walk from there finds it (B increases, B[0] = 0)
-			uint32_t g = min((uint32_t) ((float) t0 * seg_per_pos), nseg - 1);
-			while (g > 0 && B[g] > t0)
-				g--;
-			while (g + 1 < nseg && B[g + 1] <= t0)
-				g++;
-			seg = g;
-			seg_end = B[g + 1];
-		}
-		const bool whole = valid && t1 <= seg_end;
-		uint64_t v = whole ? tmax[t] : 0;
-		// max over runs of equal segments (segments do not decrease along the lanes)
-		const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, seg, 1);
-		const uint32_t heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || prev != seg);
-		const uint32_t start = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint64_t u = __shfl_up_sync(0xFFFFFFFFu, v, o);
-			if (lane >= start + o)
-				v = u > v ? u : v;
-		}
-		const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, seg, 1);
-		if (valid && (lane == 31 || next != seg) && v)
-			atomicMax(&best[seg], (unsigned long long) v);
-		// tiles cut by a boundary: positions below seg_end belong to seg, the rest to seg + 1
-		uint32_t cut = __ballot_sync(0xFFFFFFFFu, valid && !whole);
-		while (cut) {
-			const int src = __ffs(cut) - 1;
-			cut &= cut - 1;
-			const uint64_t c0 = __shfl_sync(0xFFFFFFFFu, t0, src);
-			const uint64_t c1 = __shfl_sync(0xFFFFFFFFu, t1, src);
-			const uint64_t ce = __shfl_sync(0xFFFFFFFFu, seg_end, src);
-			const uint32_t cs = __shfl_sync(0xFFFFFFFFu, seg, src);
-			uint64_t ma = 0, mb = 0;
-#pragma unroll 4
-			for (uint32_t k = 0; k < TM_TILE / 32; k++) {
-				const uint64_t i = c0 + k * 32 + lane;
-				if (i < c1) {
-					const uint32_t w = taken[i >> 5];
-					if (!((w >> lane) & 1u)) {
-						const uint64_t x = c2s[i];
-						if (i < ce)
-							ma = max(ma, x);
-						else
-							mb = max(mb, x);
-					}
-				}
-			}
-			ma = warp_max_u64(ma);
-			mb = warp_max_u64(mb);
-			if (lane == 0) {
-				if (ma)
-					atomicMax(&best[cs], (unsigned long long) ma);
-				if (mb)
-					atomicMax(&best[cs + 1], (unsigned long long) mb);
-			}
-		}
+		s_m[warp] = best;
+	__syncthreads();
+	if (warp == 0) {
+		best = warp_max_key(lane_id() < LV_THREADS / 32 ? s_m[lane_id()] : 0ull);
+		if (lane_id() == 0)
+			smax[blockIdx.x] = best;
 	}
 }
 
-// One thread per node of level d: locate the arg-max point, place the median, write
-// the node and the next level's segment bounds.  Bounds are dim1-sorted positions
-// that still include points taken by ancestors; those (at most d of them inside a
-// segment, each the point of one ancestor) are skipped when counting to the median.
-template <typename T, bool HAS_ID>
-__global__ void k_level_nodes(BuildCtx<T, HAS_ID> c, uint32_t d, const uint32_t *__restrict__ B,
-                              uint32_t *__restrict__ Bn, const unsigned long long *__restrict__ best)
+// Where a node's largest key was seen: a position, a tile, or TM_SUPER tiles.
+constexpr uint32_t AT_TILE = 0x80000000u, AT_SUPER = 0xC0000000u, AT_INDEX = 0x3FFFFFFFu;
+
+// Level d of the wide levels: GROUP threads (32 or LV_THREADS) per node.  Bounds are
+// dim1-sorted positions that still include points taken by ancestors; those (each the
+// point of one ancestor) are skipped when counting to the median.
+//
+// A tile (or 32) is only asked for its maximum while it lies inside one node, so it is
+// only that node's warp that changes it, and a tile that a bound cuts is never asked
+// again: no maximum is brought up to date for it.  A level waits on a chain of some six
+// loads, not on bandwidth, until its nodes get down to a few tiles; then it reads the
+// keys of the tiles that bounds cut, about 6 kB a node.  In place of three kernels a level
+// (arg-max by tiles, a binary search for the winner's position by a thread per node, a
+// second reduction of the tiles that lost a point): 450 -> 69 us for the 12 levels of
+// 2^21 points with the first maxima, 1.15 -> 0.38 ms for the 17 of 2^26.
+template <typename T, bool HAS_ID, int GROUP>
+__global__ void __launch_bounds__(LV_THREADS) k_level(BuildCtx<T, HAS_ID> c, uint32_t d, const uint32_t *B, uint32_t *Bn)
 {
-	using K = typename KeyOf<T>::K;
+	// a programmatic dependent of the level before it
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	__shared__ uint64_t s_key[LV_THREADS / 32];
+	__shared__ uint32_t s_at[LV_THREADS / 32];
 	const uint32_t nseg = 1u << d;
-	const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+	const uint32_t j = blockIdx.x * (LV_THREADS / GROUP) + threadIdx.x / GROUP;
 	if (j >= nseg)
 		return;
-	if (*c.err)
-		return;
+	const uint32_t lane = lane_id(), t = threadIdx.x % GROUP;
 	const uint32_t h = nseg + j;
-	const uint64_t cnt = node_count(c.n, d, j);
 	const uint32_t lo = B[j], hi = B[j + 1];
-	const uint64_t bj = best[j];
-	if (bj == 0 || cnt < 2 || lo >= hi || hi > c.n) {
-		atomicOr(c.err, 1u);
+	const bool err = __any_sync(0xFFFFFFFFu, *c.err != 0);
+	// the ancestors' positions, wanted for the median
+	const uint32_t anc = lane < d ? c.top_pos[h >> (lane + 1)] : 0u;
+	const uint32_t cnt = node_count32((uint32_t) c.n, d, j);
+	if (err)  // after an error the bounds may hold unwritten entries
+		return;
+	if (cnt < 2 || lo >= hi || hi > c.n) {
+		if (t == 0)
+			atomicOr(c.err, 1u);
 		return;
 	}
-	// position of the point: first position in [lo, hi) at or after (its dim1 key, tb)
-	const uint32_t tb = BuildCtx<T, HAS_ID>::tb_of(bj);
-	// the winner's dim1 key (needed to find its position) is known only from its
-	// point: one gather per node of the level
-	const Point<T, HAS_ID> top = c.point_of_tb(tb);
-	const K key1 = KeyOf<T>::key(top.dim1);
-	uint32_t a = lo, b = hi;
-	while (a < b) {
-		const uint32_t mid = a + (b - a) / 2;
-		const K km = c.k1s[mid];
-		if (km < key1 || (km == key1 && BuildCtx<T, HAS_ID>::tb_of(c.c2s[mid]) < tb))
-			a = mid + 1;
-		else
-			b = mid;
-	}
-	const uint32_t tp = a;
-	if (tp >= hi || c.c2s[tp] != bj) {
-		atomicOr(c.err, 8u);
-		return;
-	}
-	atomicOr(&c.taken[tp >> 5], 1u << (tp & 31));
-	c.top_pos[h] = tp;
-	uint32_t rem[33];
-	uint32_t nr = 0;
-	rem[nr++] = tp;
-	for (uint32_t an = h >> 1; an >= 1; an >>= 1) {
-		const uint32_t ta = c.top_pos[an];
-		if (ta >= lo && ta < hi)
-			rem[nr++] = ta;
-	}
-	for (uint32_t i = 1; i < nr; i++) {  // insertion sort, nr <= d + 1
-		const uint32_t x = rem[i];
-		uint32_t k = i;
-		while (k > 0 && rem[k - 1] > x) {
-			rem[k] = rem[k - 1];
-			k--;
+	uint64_t key = 0;
+	uint32_t at = 0;
+	auto see = [&](uint64_t k, uint32_t a) {
+		if (k > key) {
+			key = k;
+			at = a;
 		}
-		rem[k] = x;
+	};
+	// whole tiles [tf, tl), and the positions before and after them
+	const uint32_t tf = (uint32_t) (((uint64_t) lo + TM_TILE - 1) / TM_TILE), tl = hi / TM_TILE;
+	const bool tiles = tf < tl;
+	const uint32_t head = tiles ? tf * TM_TILE - lo : hi - lo, rest = tiles ? tl * TM_TILE : 0u;
+	const uint32_t np = tiles ? head + (hi - rest) : head;
+	constexpr int U = 8;  // loads in flight
+	for (uint32_t i0 = t; i0 < np; i0 += GROUP * U) {
+		uint64_t v[U];
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const uint32_t i = i0 + u * GROUP;
+			v[u] = i < np ? c.c2s[i < head ? lo + i : rest + (i - head)] : 0ull;
+		}
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const uint32_t i = i0 + u * GROUP;
+			see(v[u], i < head ? lo + i : rest + (i - head));
+		}
 	}
-	uint32_t pos = lo + (uint32_t) (cnt / 2) - 1;
-	for (uint32_t i = 0; i < nr; i++)
-		if (rem[i] <= pos)
-			pos++;
-	if (pos >= hi) {
-		atomicOr(c.err, 4u);
+	if (tiles) {
+		// whole groups of tiles [sf, sl), and the tiles before and after them
+		const uint32_t sf = (tf + TM_SUPER - 1) / TM_SUPER, sl = tl / TM_SUPER;
+		const bool supers = sf < sl;
+		const uint32_t th = supers ? sf * TM_SUPER : tl, tr = supers ? sl * TM_SUPER : tl;
+		for (uint32_t i = tf + t; i < th; i += GROUP)
+			see(c.tmax[i], AT_TILE | i);
+		for (uint32_t i = tr + t; i < tl; i += GROUP)
+			see(c.tmax[i], AT_TILE | i);
+		if (supers) {
+#pragma unroll 4
+			for (uint32_t i = sf + t; i < sl; i += GROUP)
+				see(c.smax[i], AT_SUPER | i);
+		}
+	}
+	uint64_t best = warp_max_key(key);
+	at = __shfl_sync(0xFFFFFFFFu, at, __ffs(__ballot_sync(0xFFFFFFFFu, key == best)) - 1);
+	if constexpr (GROUP > 32) {
+		if (lane == 0) {
+			s_key[threadIdx.x >> 5] = best;
+			s_at[threadIdx.x >> 5] = at;
+		}
+		__syncthreads();
+		if (threadIdx.x >= 32)
+			return;
+		key = lane < LV_THREADS / 32 ? s_key[lane] : 0ull;
+		best = warp_max_key(key);
+		at = s_at[(__ffs(__ballot_sync(0xFFFFFFFFu, key == best)) - 1) % (LV_THREADS / 32)];
+	}
+	// from here on one warp; every value below is the same in all its lanes, or a lane's own
+	if (best == 0) {
+		if (lane == 0)
+			atomicOr(c.err, 8u);
 		return;
 	}
-	Bn[2 * j] = lo;
-	Bn[2 * j + 1] = pos + 1;
-	if (j == nseg - 1)
-		Bn[2 * nseg] = hi;
-	c.write_node(h, top);
-	c.med[h] = c.point_at(pos).dim1;
-	atomicOr(&c.occ[h >> 5], 1u << (h & 31));
+	uint32_t tp = at;
+	if (at >= AT_TILE) {
+		uint64_t other = 0;  // maxima of the other tiles of the group
+		uint32_t tile = at & AT_INDEX;
+		if (at >= AT_SUPER) {
+			const uint64_t m = c.tmax[tile * TM_SUPER + lane];
+			const uint32_t w = __ffs(__ballot_sync(0xFFFFFFFFu, m == best)) - 1;
+			other = lane == w ? 0ull : m;
+			tile = tile * TM_SUPER + (w & 31u);
+		}
+		uint64_t v[TM_TILE / 32], m = 0;
+		load_tile(c.c2s, c.n, tile, v);
+		uint32_t k = TM_TILE / 32;
+#pragma unroll
+		for (uint32_t i = 0; i < TM_TILE / 32; i++) {
+			if (v[i] == best)
+				k = i;
+			else
+				m = max(m, v[i]);
+		}
+		const uint32_t w = __ffs(__ballot_sync(0xFFFFFFFFu, k < TM_TILE / 32));
+		if (w == 0) {
+			if (lane == 0)
+				atomicOr(c.err, 8u);
+			return;
+		}
+		tp = tile * TM_TILE + 32 * __shfl_sync(0xFFFFFFFFu, k, w - 1) + w - 1;
+		m = warp_max_key(m);
+		if (lane == 0)
+			c.tmax[tile] = m;
+		if (at >= AT_SUPER) {
+			m = max(m, warp_max_key(other));
+			if (lane == 0)
+				c.smax[at & AT_INDEX] = m;
+		}
+	}
+	// the median: the floor(cnt / 2)-th position of [lo, hi) that no ancestor's point, nor
+	// this node's, holds: the smallest pos = first + (positions taken up to pos)
+	const uint32_t mine = lane == 31 ? tp : anc;
+	const bool inside = (lane == 31 || lane < d) && mine >= lo && mine < hi;
+	const uint32_t first = lo + cnt / 2 - 1;
+	uint32_t pos = first;
+	for (;;) {
+		const uint32_t p = first + __popc(__ballot_sync(0xFFFFFFFFu, inside && mine <= pos));
+		if (p == pos)
+			break;
+		pos = p;
+	}
+	if (pos >= hi) {
+		if (lane == 0)
+			atomicOr(c.err, 4u);
+		return;
+	}
+	if (lane == 0) {
+		Bn[2 * j] = lo;
+		Bn[2 * j + 1] = pos + 1;
+		if (j == nseg - 1)
+			Bn[2 * nseg] = hi;
+		c.top_pos[h] = tp;
+		c.write_node(h, c.point_of(tp, best));
+		c.c2s[tp] = 0;
+		// every node of a wide level exists
+		if (nseg < 32)
+			atomicOr(&c.occ[0], 1u << h);
+		else if (j % 32 == 0)
+			c.occ[h >> 5] = 0xFFFFFFFFu;
+	}
+	if (lane == 1)
+		c.med[h] = c.point_of(pos, c.c2s[pos]).dim1;
 }
 
 // ---------------------------------------------------------------------------
@@ -585,15 +585,6 @@ constexpr int ST_GATHER = (ST_CAP + ST_THREADS - 1) / ST_THREADS + 1;
 // above the last level holds one), the left child keeps the first floor(c/2) of
 // the rest and the right child the others, so
 //   start(2t) = start(t) - t,  start(2t+1) = start(t) - t + floor(c/2).
-
-// The node count of node_count in 32 bits (trees hold fewer than 2^31 points).
-__device__ __forceinline__ uint32_t node_count32(uint32_t n, uint32_t d, uint32_t j)
-{
-	uint32_t c = n;
-	for (int b = (int) d - 1; b >= 0 && c != 0; b--)
-		c = ((j >> b) & 1u) ? c - 1u - (c >> 1) : c >> 1;
-	return c;
-}
 
 // Sub-node counts and warps come in powers of two: every quotient in the builder is
 // a shift (a run-time divisor costs a division sequence per use, and the builder is
@@ -647,21 +638,17 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(BuildCtx<T, HAS_ID> c, u
 	{
 		uint64_t v[ST_GATHER];
 		K v1[ST_GATHER];
-		uint32_t m[ST_GATHER], tw[ST_GATHER];
-		// the keys are read with the taken bits, not after them: one round trip
+		uint32_t m[ST_GATHER];
 #pragma unroll
 		for (int u = 0; u < ST_GATHER; u++) {
 			const uint32_t i = lo + (uint32_t) u * ST_THREADS + threadIdx.x;
 			const bool in = i < hi;
-			tw[u] = in ? c.taken[i >> 5] : 0u;
 			v[u] = in ? c.c2s[i] : 0;
 			v1[u] = (KEYS4 && c.recon && in) ? c.k1s[i] : K(0);
 		}
 #pragma unroll
 		for (int u = 0; u < ST_GATHER; u++) {
-			const uint32_t i = lo + (uint32_t) u * ST_THREADS + threadIdx.x;
-			const bool keep = i < hi && !((tw[u] >> (i & 31)) & 1u);
-			m[u] = __ballot_sync(0xFFFFFFFFu, keep);
+			m[u] = __ballot_sync(0xFFFFFFFFu, v[u] != 0);
 			if (lane == 0)
 				s_pre[u][warp] = __popc(m[u]);
 		}
@@ -928,7 +915,7 @@ T *as(void *p)
 
 // All construction scratch lives in one device allocation.
 struct ScratchLayout {
-	size_t k1, kalt, c2, valt, k2, v32a, v32b, P, rs_status, rs_misc, hist1, flags, Ba, Bb, best, top, taken, tmax;
+	size_t k1, kalt, c2, valt, k2, v32a, v32b, P, rs_status, rs_misc, hist1, flags, Ba, Bb, top, tmax, smax;
 	size_t total;
 };
 
@@ -962,10 +949,9 @@ ScratchLayout scratch_layout(pst_dtype dt, pst_idtype it, uint64_t n)
 	L.flags = take(256);
 	L.Ba = take((nodes_wide + 1) * 4);
 	L.Bb = take((nodes_wide + 1) * 4);
-	L.best = take(nodes_wide * 8);
 	L.top = take(nodes_wide * 4);
-	L.taken = take(((n + 31) / 32) * 4);
 	L.tmax = take(L0 ? ntiles * 8 : 0);
+	L.smax = take(L0 ? (ntiles + TM_SUPER - 1) / TM_SUPER * 8 : 0);
 	L.total = o;
 	return L;
 }
@@ -1114,8 +1100,6 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 	const uint32_t L0 = std::min(subtree_level(n), D - 1);
 	const uint64_t nodes_wide = 1ull << L0;
 	const uint64_t ntiles = (n + TM_TILE - 1) / TM_TILE;
-	unsigned long long *best = scr.at<unsigned long long>(SL.best);
-	PST_CUDA(cudaMemsetAsync(scr.at<void>(SL.taken), 0, ((n + 31) / 32) * 4, s));
 	BuildCtx<T, HAS_ID> c;
 	c.pts = pts;
 	c.P = P;
@@ -1123,8 +1107,8 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 	c.recon = !WIDE_KEY && !negzero && ids_are_indices && P == nullptr;
 	c.k1s = k1s;
 	c.c2s = c2s;
-	c.taken = scr.at<uint32_t>(SL.taken);
 	c.tmax = scr.at<uint64_t>(SL.tmax);
+	c.smax = scr.at<uint64_t>(SL.smax);
 	c.dim1 = as<T>(t.dim1);
 	c.dim2 = as<T>(t.dim2);
 	c.med = as<T>(t.med);
@@ -1140,21 +1124,23 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 		PST_CUDA(cudaMemcpyAsync(B, b0, 8, cudaMemcpyHostToDevice, s));
 	}
 	if (L0) {
-		const unsigned tgrid = (unsigned) std::max<uint64_t>(
-		    1, std::min<uint64_t>((ntiles + AM_THREADS / 32 - 1) / (AM_THREADS / 32), (uint64_t) device_info().sms * 8));
-		k_tile_max_all<<<tgrid, AM_THREADS, 0, s>>>(c2s, c.taken, n, c.tmax);
-		const unsigned am_grid = (unsigned) std::max<uint64_t>(
-		    1, std::min<uint64_t>((ntiles + AM_THREADS - 1) / AM_THREADS, (uint64_t) device_info().sms * 8));
+		k_tile_max<<<(unsigned) ((ntiles + TM_SUPER - 1) / TM_SUPER), LV_THREADS, 0, s>>>(c2s, n, c.tmax, c.smax);
+		PST_CUDA(cudaGetLastError());
 		for (uint32_t d = 0; d < L0; d++) {
 			const uint32_t nseg = 1u << d;
-			PST_CUDA(cudaMemsetAsync(best, 0, (size_t) nseg * 8, s));
-			k_level_argmax<<<am_grid, AM_THREADS, 0, s>>>(c2s, c.taken, c.tmax, n, B, nseg, best, c.err,
-			                                               (float) ((double) nseg / (double) n));
-			k_level_nodes<T, HAS_ID><<<(nseg + 127) / 128, 128, 0, s>>>(c, d, B, Bn, best);
-			if (d + 1 < L0)
-				k_tile_refresh<<<(unsigned) ((nseg * 32 + AM_THREADS - 1) / AM_THREADS), AM_THREADS, 0, s>>>(
-				    c2s, c.taken, n, c.top_pos, d, c.tmax, c.err);
-			PST_CUDA(cudaGetLastError());
+			// a CTA per node while the device holds them all at once, a warp per node below
+			const bool ctas = nseg <= (uint32_t) device_info().sms * 4;
+			cudaLaunchConfig_t cfg{};
+			cudaLaunchAttribute attr[1];
+			attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+			attr[0].val.programmaticStreamSerializationAllowed = 1;
+			cfg.gridDim = dim3(ctas ? nseg : (nseg + LV_THREADS / 32 - 1) / (LV_THREADS / 32));
+			cfg.blockDim = dim3(LV_THREADS);
+			cfg.stream = s;
+			cfg.attrs = attr;
+			cfg.numAttrs = 1;
+			PST_CUDA(ctas ? cudaLaunchKernelEx(&cfg, k_level<T, HAS_ID, LV_THREADS>, c, d, (const uint32_t *) B, Bn)
+			              : cudaLaunchKernelEx(&cfg, k_level<T, HAS_ID, 32>, c, d, (const uint32_t *) B, Bn));
 			std::swap(B, Bn);
 		}
 	}
