@@ -182,22 +182,24 @@ static uint64_t run_single(pst_tree *tr, const pst_query *q, pst_ret ret, void *
 	Batch &b = single_engine(tr);
 	b.stage_queries(q, 1, false, s);
 	uint64_t total = 0;
+	if (!alloc) {
+		// counted and written in one go, where the results fit
+		const EmitTo to{ret, *out_d, capacity, nullptr};
+		b.count_sync(s, &total, *out_d ? &to : nullptr);
+		if (total && total <= capacity && b.last_status() != PST_OK)
+			fail(b.last_status(), "search emit failed");
+		return total;
+	}
 	b.count_sync(s, &total);
 	if (total == 0)
 		return 0;
-	if (alloc) {
-		malloc_result(out_d, total * b.record_size(ret), s);
-	} else if (total > capacity) {
-		return total;
-	}
-	b.enqueue_emit(ret, *out_d, alloc ? total : capacity, s);
+	malloc_result(out_d, total * b.record_size(ret), s);
+	b.enqueue_emit(ret, *out_d, total, s);
 	uint64_t t2 = 0;
 	const pst_status st = b.read_ctl(s, &t2);
 	if (st != PST_OK) {
-		if (alloc) {
-			cudaFreeAsync(*out_d, s);  // after whatever the stream still holds
-			*out_d = nullptr;
-		}
+		cudaFreeAsync(*out_d, s);  // after whatever the stream still holds
+		*out_d = nullptr;
 		fail(st, "search emit failed");
 	}
 	return total;
@@ -488,23 +490,14 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 			fail(PST_ERR_INVALID, "bad return type");
 		if (ret == PST_RET_IDS && b.tree->idtype != PST_ID_U32)
 			fail(PST_ERR_UNSUPPORTED, "an id-less tree can only return points");
-		b.stage_queries(queries, nq, queries_on_device != 0, s);
+		b.stage_queries(queries, nq, queries_on_device != 0, s, !sync);
 		uint64_t tot = 0;
 		if (sync) {
-			b.count_sync(s, &tot);
-			if (offsets_d)
-				check_cuda(cudaMemcpyAsync(offsets_d, b.offsets, ((size_t) nq + 1) * 8, cudaMemcpyDeviceToDevice, s),
-				           "copy offsets");
+			const EmitTo to{ret, out_d, out_capacity, offsets_d};
+			b.count_sync(s, &tot, &to);
 			if (total)
 				*total = tot;
-			if (tot > out_capacity) {
-				check_cuda(cudaStreamSynchronize(s), "sync");
-				result = PST_ERR_CAPACITY;
-				return;
-			}
-			if (tot)
-				b.enqueue_emit(ret, out_d, out_capacity, s);
-			result = b.read_ctl(s, nullptr);
+			result = tot > out_capacity ? PST_ERR_CAPACITY : b.last_status();
 		} else {
 			b.launch_count(s);
 			b.enqueue_emit(ret, out_d, out_capacity, s);

@@ -86,6 +86,42 @@ __device__ __forceinline__ uint4 block_record(uint32_t pos32, uint32_t q, uint32
 	return make_uint4(pos32 & ~63u, q, upper ? 0u : bits32, upper ? bits32 : 0u);
 }
 
+// What a query does at a node of its boundary path (the reference's delegation): report it
+// (rep), go on to a child with a mode (pl, pr; 0 = no), report a child's subtree from above
+// (rl, rr).  v1, v2, m: the node's values and median; hl, hr: whether it has the children.
+template <typename T>
+__device__ __forceinline__ void path_rules(uint32_t kind, uint32_t mode, T min1, T max1, T min2, T v1, T v2, T m, bool hl,
+                                           bool hr, bool &rep, uint32_t &pl, uint32_t &pr, bool &rl, bool &rr)
+{
+	if (min2 <= v2) {
+		rep = kind == PST_Q_THREE ? (min1 <= v1 && v1 <= max1) : kind == PST_Q_LEFT ? (v1 <= max1) : (v1 >= min1);
+		if (mode == MODE_THREE) {
+			if (min1 <= m && m <= max1) {
+				pl = hl ? MODE_RIGHT : 0;
+				pr = hr ? MODE_LEFT : 0;
+			} else if (max1 < m && hl) {
+				pl = MODE_THREE;
+			} else if (m < min1 && hr) {
+				pr = MODE_THREE;
+			}
+		} else if (mode == MODE_LEFT) {
+			if (m <= max1) {
+				rl = hl;
+				pr = hr ? MODE_LEFT : 0;
+			} else if (hl) {
+				pl = MODE_LEFT;
+			}
+		} else {
+			if (m >= min1) {
+				pl = hl ? MODE_RIGHT : 0;
+				rr = hr;
+			} else if (hr) {
+				pr = MODE_RIGHT;
+			}
+		}
+	}
+}
+
 template <typename T>
 __device__ __forceinline__ void path_step(const TreeDev<T> &t, const QDev<T> &qd, const WorkDev &w, uint32_t d,
                                           uint4 task, bool valid)
@@ -108,34 +144,8 @@ __device__ __forceinline__ void path_step(const TreeDev<T> &t, const QDev<T> &qd
 		const T v1 = t.dim1[h];
 		const uint32_t ow = !inner ? 0u : d + 2 < t.levels ? FULL : t.occ[l >> 5];
 		const T m = inner ? t.med[h] : T(0);
-		if (min2 <= v2) {
-			rep = kind == PST_Q_THREE ? (min1 <= v1 && v1 <= max1) : kind == PST_Q_LEFT ? (v1 <= max1) : (v1 >= min1);
-			const bool hl = (ow >> (l & 31)) & 1u, hr = (ow >> (r & 31)) & 1u;
-			if (mode == MODE_THREE) {
-				if (min1 <= m && m <= max1) {
-					pl = hl ? MODE_RIGHT : 0;
-					pr = hr ? MODE_LEFT : 0;
-				} else if (max1 < m && hl) {
-					pl = MODE_THREE;
-				} else if (m < min1 && hr) {
-					pr = MODE_THREE;
-				}
-			} else if (mode == MODE_LEFT) {
-				if (m <= max1) {
-					rl = hl;
-					pr = hr ? MODE_LEFT : 0;
-				} else if (hl) {
-					pl = MODE_LEFT;
-				}
-			} else {
-				if (m >= min1) {
-					pl = hl ? MODE_RIGHT : 0;
-					rr = hr;
-				} else if (hr) {
-					pr = MODE_RIGHT;
-				}
-			}
-		}
+		path_rules<T>(kind, mode, min1, max1, min2, v1, v2, m, (ow >> (l & 31)) & 1u, (ow >> (r & 31)) & 1u, rep, pl, pr,
+		              rl, rr);
 	}
 	// The warp's reported nodes, next-level paths and seeds each take one reservation,
 	// and lane 0 issues the three together.  At most two boundary paths per query and
@@ -560,10 +570,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_bfs_level(TreeDev<T
 // its level-0 boundary path task (returned); a kind out of range raises
 // BATCH_FLAG_BAD_QUERY in *flags (the pass still runs, and the host reports it).
 template <typename T>
-__device__ __forceinline__ uint4 unpack_query(const pst_query *__restrict__ raw, uint32_t i, const QOut<T> &qo,
-                                              uint32_t *flags)
+__device__ __forceinline__ uint4 unpack_query(const pst_query &q, uint32_t i, const QOut<T> &qo, uint32_t *flags)
 {
-	const pst_query q = raw[i];
 	T a, b, c;
 	if constexpr (sizeof(T) == 8) {
 		a = q.min1.f64; b = q.max1.f64; c = q.min2.f64;
@@ -605,230 +613,12 @@ __global__ void k_prepare_queries(const pst_query *raw, BatchCtl *ctl, QOut<T> q
 	const uint32_t nq = ctl->nq;
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < max_q; i += gridDim.x * blockDim.x) {
 		if (i < nq)
-			path0[i] = unpack_query<T>(raw, i, qo, &ctl->flags);
+			path0[i] = unpack_query<T>(raw[i], i, qo, &ctl->flags);
 		counts[i] = 0;
 		cursor[i] = 0;
 	}
 	if (blockIdx.x == 0 && threadIdx.x == 0)
 		ctl->path_cnt[0] = nq;
-}
-
-// Small batches (a single query, or a few): one CTA takes the tree from the top,
-// level by level with a CTA barrier in place of a kernel boundary, while the
-// records to expand stay few enough for it (at most CTA_REC_CAP); it leaves
-// ctl->cta_levels = the levels done and the host launches the per-level kernels
-// for the rest only.  When it reaches the bottom it also scans the queries'
-// counts into offsets[0..max_q] and total, so no scan pass is needed.
-//
-// The pass works in shared memory: the control block, the boundary paths and
-// seeds (pcap of each of the four lists) and the alive records of every level it
-// takes (rcap) live in the dynamic shared array, so a level waits on its tree
-// loads alone, not on round trips to L2 for its counters, records and
-// reservations.  Where it stops, it writes the records, the control block and the
-// next level's paths and seeds to their global buffers, in the layout the
-// per-level kernels and the emit read.  It stops early when the next level might
-// not fit in rcap.
-constexpr uint32_t CTA_REC_CAP = 256;
-
-// Dynamic shared memory of k_bfs_cta: the control block, then the four path and
-// seed lists, then the records.
-__host__ __device__ constexpr size_t cta_smem_bytes(uint32_t pcap, uint32_t rcap)
-{
-	return sizeof(BatchCtl) + (size_t) (4 * pcap + rcap) * sizeof(uint4);
-}
-static_assert(sizeof(BatchCtl) % 16 == 0, "the lists after the control block stay 16-byte aligned");
-
-template <typename T>
-__global__ void __launch_bounds__(BFS_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T> qd, WorkDev wg, uint32_t max_q,
-                                                            uint32_t pcap, uint32_t rcap, const pst_query *raw,
-                                                            QOut<T> qo, const BatchCtl *ctl_src)
-{
-	extern __shared__ __align__(16) unsigned char s_dyn[];
-	__shared__ WarpStage<T> s_stage[BFS_THREADS / 32];
-	__shared__ uint64_t s_base[2];
-	__shared__ uint64_t s_wsum[BFS_THREADS / 32];
-	__shared__ uint32_t s_go, s_cnt[2];
-	BatchCtl *sc = reinterpret_cast<BatchCtl *>(s_dyn);
-	uint4 *sl = reinterpret_cast<uint4 *>(s_dyn + sizeof(BatchCtl));
-	// the shared-memory view of the work buffers (ids of reported boundary nodes,
-	// counts and offsets stay global)
-	WorkDev w = wg;
-	w.ctl = sc;
-	w.path0 = sl;
-	w.path1 = sl + pcap;
-	w.seed0 = sl + 2 * pcap;
-	w.seed1 = sl + 3 * pcap;
-	w.path_cap = pcap;
-	w.rec = sl + 4 * pcap;
-	w.rec_cap = rcap;
-	{
-		// the pass's starting control block: the engine's pinned host copy (or the
-		// no-alloc search's device copy), wg.ctl receives the final one
-		const uint32_t *src = reinterpret_cast<const uint32_t *>(ctl_src);
-		uint32_t *dst = reinterpret_cast<uint32_t *>(sc);
-		for (uint32_t i = threadIdx.x; i < sizeof(BatchCtl) / 4; i += BFS_THREADS)
-			dst[i] = src[i];
-	}
-	__syncthreads();
-	{
-		// the start of the pass (k_prepare_queries of a full pass): the queries
-		// unpacked and checked, their level-0 paths (at most pcap / 2 queries: the
-		// host runs this pass for small batches only), the counts and cursors zeroed
-		const uint32_t nq = min(sc->nq, pcap);
-		for (uint32_t i = threadIdx.x; i < max_q; i += BFS_THREADS) {
-			if (i < nq)
-				w.path0[i] = unpack_query<T>(raw, i, qo, &sc->flags);
-			wg.counts[i] = 0;
-			wg.cursor[i] = 0;
-		}
-		if (threadIdx.x == 0)
-			sc->path_cnt[0] = nq;
-	}
-	__syncthreads();
-	const uint64_t gwarps = BFS_THREADS / 32, gwarp = threadIdx.x >> 5;
-	uint64_t acc_prev = 0, acc = 0;  // (thread 0) start of the previous level's records, and of this level's
-	uint32_t d = 0;
-	for (; d < t.levels; d++) {
-		if (threadIdx.x == 0) {
-			const uint32_t prev = d ? sc->lvl_cnt[d - 1] : 0u;
-			const uint32_t np = min(sc->path_cnt[d], pcap), ns = min(sc->seed_cnt[d], pcap);
-			if (d) {
-				acc_prev = acc;
-				acc += prev;
-			}
-			s_base[0] = acc_prev;
-			s_base[1] = acc;
-			s_cnt[0] = np;
-			s_cnt[1] = ns;
-			// the level appends at most two children per record and one record per seed
-			s_go = !(sc->flags & BATCH_FLAG_TASK_OVERFLOW) && prev <= CTA_REC_CAP &&
-			       acc + 2 * (uint64_t) prev + ns <= rcap;
-			if (s_go)
-				sc->lvl_base[d] = acc;
-		}
-		__syncthreads();
-		if (!s_go)
-			break;
-		const uint64_t base_prev = s_base[0], base_cur = s_base[1];
-		const uint64_t n_prev = base_cur - base_prev;
-		if (d + 1 == t.levels && t.last_par)
-			level_body<T, true>(t, qd, w, d, gwarp, gwarps, base_prev, base_cur, n_prev, s_cnt, s_stage[gwarp]);
-		else
-			level_body<T, false>(t, qd, w, d, gwarp, gwarps, base_prev, base_cur, n_prev, s_cnt, s_stage[gwarp]);
-		__syncthreads();  // the level's records, paths, seeds and counts are visible to the CTA
-		if (threadIdx.x == 0)
-			sc->cta_levels = d + 1;
-	}
-	// Hand over: the records of the levels taken (acc of them, levels 0..d-1), and,
-	// where the pass stopped above the bottom, the paths and seeds of level d.
-	if (threadIdx.x == 0) {
-		// records written: at the bottom, acc is the start of the last level's region
-		// and that level's count follows it; where the pass stopped at level d, the
-		// top of the loop had already advanced acc past level d - 1, so acc is the
-		// number written (at most rcap in both cases: each level's bound was checked
-		// before it ran)
-		const uint64_t n = d == t.levels && d ? acc + sc->lvl_cnt[d - 1] : acc;
-		// (a refused reservation, which the bound rules out, would have raised the
-		// overflow flag and left the counts past what was stored: never copy beyond)
-		s_base[0] = min(n, (uint64_t) rcap);
-		if (n > wg.rec_cap) {
-			sc->need_tasks = max((unsigned long long) sc->need_tasks, (unsigned long long) n);
-			sc->flags |= BATCH_FLAG_TASK_OVERFLOW;
-		}
-		s_go = d == t.levels && !(sc->flags & BATCH_FLAG_TASK_OVERFLOW);
-	}
-	__syncthreads();
-	{
-		const uint64_t n = s_base[0];
-		if (n <= wg.rec_cap)
-			for (uint64_t i = threadIdx.x; i < n; i += BFS_THREADS)
-				wg.rec[i] = w.rec[i];
-		if (d < t.levels) {
-			const uint32_t np = min(sc->path_cnt[d], pcap), ns = min(sc->seed_cnt[d], pcap);
-			const uint4 *ps = (d & 1) ? w.path1 : w.path0, *ss = (d & 1) ? w.seed1 : w.seed0;
-			uint4 *pd = (d & 1) ? wg.path1 : wg.path0, *sd = (d & 1) ? wg.seed1 : wg.seed0;
-			for (uint32_t i = threadIdx.x; i < np; i += BFS_THREADS)
-				pd[i] = ps[i];
-			for (uint32_t i = threadIdx.x; i < ns; i += BFS_THREADS)
-				sd[i] = ss[i];
-		}
-	}
-	if (s_go) {
-		// exclusive scan of counts[0..max_q) in chunks of one count per thread
-		const uint32_t nq = sc->nq, lane = lane_id();
-		uint64_t *offsets = const_cast<uint64_t *>(w.offsets);
-		uint64_t carry = 0;
-		for (uint32_t b = 0; b < max_q; b += BFS_THREADS) {
-			const uint32_t q = b + threadIdx.x;
-			const uint64_t c = q < nq ? w.counts[q] : 0;
-			const uint64_t inc = warp_incl_scan(c);
-			if (lane == 31)
-				s_wsum[gwarp] = inc;
-			__syncthreads();
-			if (gwarp == 0) {
-				uint64_t v = lane < BFS_THREADS / 32 ? s_wsum[lane] : 0;
-				v = warp_incl_scan(v);
-				if (lane < BFS_THREADS / 32)
-					s_wsum[lane] = v;
-			}
-			__syncthreads();
-			if (q < max_q)
-				offsets[q] = carry + (gwarp ? s_wsum[gwarp - 1] : 0) + inc - c;
-			carry += s_wsum[BFS_THREADS / 32 - 1];
-			__syncthreads();  // s_wsum is rewritten by the next chunk
-		}
-		if (threadIdx.x == 0) {
-			offsets[max_q] = carry;
-			sc->total = carry;
-		}
-	}
-	__syncthreads();
-	// the control block last: every counter the host and the next kernels read
-	{
-		const uint32_t *src = reinterpret_cast<const uint32_t *>(sc);
-		uint32_t *dst = reinterpret_cast<uint32_t *>(wg.ctl);
-		for (uint32_t i = threadIdx.x; i < sizeof(BatchCtl) / 4; i += BFS_THREADS)
-			dst[i] = src[i];
-	}
-}
-
-// Shared memory the one-CTA top pass may take beyond its static arrays on the
-// current device, after allowing it for the kernel there (once per device; done
-// before any launch is captured into a graph).
-template <typename T>
-size_t cta_pass_budget()
-{
-	static std::mutex mu;
-	static size_t budget[64];
-	static bool done[64] = {};
-	const DeviceInfo &di = device_info();
-	std::lock_guard<std::mutex> lk(mu);
-	if (!done[di.device]) {
-		cudaFuncAttributes a{};
-		PST_CUDA(cudaFuncGetAttributes(&a, k_bfs_cta<T>));
-		const size_t b = di.smem_optin > a.sharedSizeBytes + 1024 ? di.smem_optin - a.sharedSizeBytes - 1024 : 0;
-		PST_CUDA(cudaFuncSetAttribute(k_bfs_cta<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b));
-		budget[di.device] = b;
-		done[di.device] = true;
-	}
-	return budget[di.device];
-}
-
-// Launches the one-CTA top pass with its shared-memory lists: pcap entries for each
-// path and seed list (at least two per query of the batch) and as many records as
-// the rest of the CTA's shared memory holds.
-template <typename T>
-void launch_cta_pass(const TreeDev<T> &tv, const QDev<T> &qd, const WorkDev &w, uint32_t max_q, uint32_t pcap,
-                     const pst_query *raw, const QOut<T> &qo, const BatchCtl *ctl_src, cudaStream_t s)
-{
-	const size_t budget = cta_pass_budget<T>();
-	const size_t fixed = cta_smem_bytes(pcap, 0);
-	// room for at least one level's records beyond the lists
-	if (budget < fixed + (size_t) (2 * CTA_REC_CAP + pcap) * sizeof(uint4))
-		fail(PST_ERR_INTERNAL, "shared memory too small for the top pass of " + std::to_string(max_q) + " queries");
-	const uint32_t rcap = (uint32_t) ((budget - fixed) / sizeof(uint4));
-	k_bfs_cta<T><<<1, BFS_THREADS, cta_smem_bytes(pcap, rcap), s>>>(tv, qd, w, max_q, pcap, rcap, raw, qo,
-	                                                                  ctl_src);
 }
 
 // Output slot of this lane's record inside its query's result: one atomic per run
@@ -999,6 +789,473 @@ __device__ __forceinline__ void emit_blocks(const TreeDev<T> &t, const uint4 &mi
 	else
 		emit_ids<U>(t.id, nrec, sm.st, static_cast<uint32_t *>(out));
 	__syncwarp();  // the stage is reused by the warp's next batch
+}
+
+// Small batches (a single query, or a few): one CTA takes the tree from the top,
+// level by level with a CTA barrier in place of a kernel boundary, while the
+// records to expand stay few enough for it (at most CTA_REC_CAP); it leaves
+// ctl->cta_levels = the levels done and the host launches the per-level kernels
+// for the rest only.  When it reaches the bottom it also scans the queries' counts
+// into their offsets, and writes the results itself when they are few
+// (CTA_EMIT_CAP), so that the call is this one kernel.
+//
+// The pass is a chain of levels, each a few dependent steps, so everything a level
+// touches but the tree is in shared memory: the control block, the paths and seeds (pcap
+// of each of the four lists), the counts (qcap) and the records of every level it takes
+// (rcap).  A record's children are read at once with the subtree minimum that may make
+// the reading needless (level_body asks for that first, to spare the loads: two round
+// trips a level); reservations are single shared-memory atomics, counts are sums of
+// one; and every thread keeps the level's bounds itself, so that one barrier ends a level.
+// One query on 64.5 k points (16 levels): 30 us with the per-level kernels' body between
+// two barriers a level, TOPUS us.  A few host queries and the arguments come as the kernel's
+// parameters (reading them from mapped host memory takes 3.7 us), and the control block goes
+// back to mapped host memory: a copy each way took 16 us of a call.
+// Where the pass stops, it writes the records, the counts and the next level's paths
+// and seeds to their global buffers, in the layout the per-level kernels and the emit
+// read.  It stops early when the next level might not fit in rcap.
+constexpr uint32_t CTA_REC_CAP = 256;
+constexpr uint32_t CTA_EMIT_CAP = 16384;
+constexpr int TOP_THREADS = 512, TOP_WARPS = TOP_THREADS / 32;
+
+// Dynamic shared memory of k_bfs_cta: the control block (built at the end), a cell of
+// counters per level, the queries' offsets, counts and cursors, the four path and seed
+// lists, then the records.
+constexpr uint32_t TOP_CELLS = 41;
+__host__ __device__ constexpr size_t cta_smem_bytes(uint32_t qcap, uint32_t pcap, uint32_t rcap)
+{
+	return sizeof(BatchCtl) + (size_t) (TOP_CELLS + qcap + 4 * pcap + rcap) * sizeof(uint4);
+}
+static_assert(sizeof(BatchCtl) % 16 == 0, "the lists after the control block stay 16-byte aligned");
+
+// Shared memory by its own 32-bit addresses: accesses through pointers that reach a level's
+// code in a struct were compiled as generic ones (130 cycles for a load, 30 as such).
+__device__ __forceinline__ uint4 sh_ld4(uint32_t a)
+{
+	uint4 v;
+	asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+	return v;
+}
+__device__ __forceinline__ void sh_st4(uint32_t a, const uint4 &v)
+{
+	asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint32_t sh_ld(uint32_t a)
+{
+	uint32_t v;
+	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+	return v;
+}
+__device__ __forceinline__ void sh_st(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ uint32_t sh_add(uint32_t a, uint32_t n)
+{
+	uint32_t v;
+	asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(v) : "r"(a), "r"(n) : "memory");
+	return v;
+}
+__device__ __forceinline__ void sh_or(uint32_t a, uint32_t m) { asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(a), "r"(m) : "memory"); }
+
+// The top pass's shared memory (addresses in it) and where its query bounds are.
+template <typename T>
+struct TopPass {
+	QDev<T> qd;
+	// cell d: records of level d - 1, paths and seeds of level d, start of level d's records
+	uint32_t cells;
+	uint32_t flags, rec_cnt;
+	uint32_t cnt, cur;  // a word per query
+	uint32_t lists, rec;
+	uint4 *ro;          // (global)
+	uint32_t pcap, ro_cap;
+
+	__device__ __forceinline__ uint32_t cell(uint32_t d) const { return cells + 16 * d; }
+	// entry i of the paths and of the seeds of level d
+	__device__ __forceinline__ uint32_t path(uint32_t d, uint32_t i) const { return lists + 16 * ((d & 1) * pcap + i); }
+	__device__ __forceinline__ uint32_t seed(uint32_t d, uint32_t i) const { return lists + 16 * ((2 + (d & 1)) * pcap + i); }
+};
+
+// 32 boundary-path tasks of level d (path_step's rules).  Every lane reserves for itself:
+// the lanes at work are few.
+template <typename T>
+__device__ __forceinline__ void top_paths(const TreeDev<T> &t, const TopPass<T> &p, uint32_t d, uint32_t at, uint32_t np)
+{
+	const uint32_t i = at + lane_id();
+	if (i >= np)
+		return;
+	const uint4 task = sh_ld4(p.path(d, i));
+	const uint32_t h = task.x, q = task.y, mode = task.z, l = 2 * h, r = l + 1;
+	bool rep = false, rl = false, rr = false;
+	uint32_t pl = 0, pr = 0;
+	const bool inner = d + 1 < t.levels;
+	const T v2 = t.dim2[h], v1 = t.dim1[h];
+	const T m = inner ? t.med[h] : T(0);
+	const uint32_t ow = !inner ? 0u : d + 2 < t.levels ? FULL : t.occ[l >> 5];
+	const T min2 = p.qd.min2[q], min1 = p.qd.min1[q], max1 = p.qd.max1[q];
+	const uint32_t kind = p.qd.kind[q];
+	path_rules<T>(kind, mode, min1, max1, min2, v1, v2, m, (ow >> (l & 31)) & 1u, (ow >> (r & 31)) & 1u, rep, pl, pr, rl,
+	              rr);
+	const uint32_t next = p.cell(d + 1), npl = (pl ? 1u : 0u) + (pr ? 1u : 0u);
+	const bool seed = rl || rr;
+	// the three reservations are on their way together
+	const uint32_t b_path = npl ? sh_add(next + 4, npl) : 0u, b_seed = seed ? sh_add(next + 8, 1) : 0u,
+	               b_rep = rep ? sh_add(p.rec_cnt, 1) : 0u;
+	// (the lists hold all there can be: two paths a query and level)
+	bool lost = b_path + npl > p.pcap;
+	if (!lost) {
+		if (pl)
+			sh_st4(p.path(d + 1, b_path), make_uint4(l, q, pl, 0));
+		if (pr)
+			sh_st4(p.path(d + 1, b_path + npl - 1), make_uint4(r, q, pr, 0));
+	}
+	if (seed) {
+		if (b_seed < p.pcap)
+			sh_st4(p.seed(d + 1, b_seed), make_uint4(l & ~31u, q, (rl ? 1u << (l & 31) : 0u) | (rr ? 1u << (r & 31) : 0u), 0u));
+		else
+			lost = true;
+	}
+	if (rep) {
+		if (b_rep < p.ro_cap)
+			p.ro[b_rep] = block_record(h & ~31u, q, 1u << (h & 31));
+		else
+			lost = true;
+		sh_add(p.cnt + 4 * q, 1);
+	}
+	if (lost)
+		sh_or(p.flags, BATCH_FLAG_INTERNAL);
+}
+
+// 32 report-above seeds of level d: each the aligned pair of one node's children.
+template <typename T>
+__device__ __forceinline__ void top_seeds(const TreeDev<T> &t, const TopPass<T> &p, uint32_t d, uint32_t at, uint32_t ns,
+                                          uint32_t base_cur)
+{
+	const uint32_t i = at + lane_id();
+	if (i >= ns)
+		return;
+	const uint4 sd = sh_ld4(p.seed(d, i));
+	const uint32_t b = (__ffs(sd.z) - 1) & ~1u;
+	const T v0 = t.dim2[sd.x + b], v1 = t.dim2[sd.x + b + 1];
+	const uint32_t cand = sd.z & (d + 1 < t.levels ? FULL : t.occ[sd.x >> 5]);
+	const T m2 = p.qd.min2[sd.y];
+	const uint32_t am =
+	    (((cand >> b) & 1u) && m2 <= v0 ? 1u << b : 0u) | (((cand >> (b + 1)) & 1u) && m2 <= v1 ? 2u << b : 0u);
+	if (am) {
+		sh_st4(p.rec + 16 * (base_cur + sh_add(p.cell(d + 1), 1)), block_record(sd.x, sd.y, am));
+		sh_add(p.cnt + 4 * sd.y, (uint32_t) __popc(am));
+	}
+}
+
+// The children of the records [at, end) of the level above (at most TOP_U): the warp takes
+// each record whole, lane l its child slots [2b + 4l, 2b + 4l + 4).
+constexpr int TOP_U = 4;
+
+template <typename T>
+__device__ __forceinline__ void top_records(const TreeDev<T> &t, const TopPass<T> &p, uint32_t d, uint32_t at,
+                                            uint32_t end, uint32_t base_cur)
+{
+	const uint32_t lane = lane_id();
+	const bool last = d + 1 == t.levels;
+	uint4 rc[TOP_U];
+	uint32_t nib[TOP_U];
+	T v[TOP_U][4], m2[TOP_U], sm[TOP_U];
+#pragma unroll
+	for (int u = 0; u < TOP_U; u++)
+		rc[u] = at + u < end ? sh_ld4(p.rec + 16 * (at + u)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+	for (int u = 0; u < TOP_U; u++) {
+		const uint32_t base = rc[u].x & ~63u;
+		const uint32_t two = ((lane < 16 ? rc[u].z : rc[u].w) >> ((2 * lane) & 31)) & 3u;  // the lane's parents
+		nib[u] = (two & 1u ? 3u : 0u) | (two & 2u ? 12u : 0u);
+		const bool look = (rc[u].x & RECORD_WHOLE) == 0 && (rc[u].z | rc[u].w) != 0;
+		m2[u] = look ? p.qd.min2[rc[u].y] : T(0);
+		sm[u] = look && t.sub_min && base >= 64 ? t.sub_min[base >> 6] : T(0);
+		const uint32_t c = 2 * base + 4 * lane;
+		const uint32_t ow = last && nib[u] ? t.occ[c >> 5] >> (c & 31) : FULL;
+		if (look && nib[u]) {
+			load_quad(t.dim2 + c, v[u]);
+		} else {
+#pragma unroll
+			for (int j = 0; j < 4; j++)
+				v[u][j] = T(0);
+		}
+		nib[u] &= ow;
+	}
+	// the lane's child record of the warp: half (lane & 1) of record lane >> 1
+	uint4 mine = make_uint4(0, 0, 0, 0);
+	uint32_t pts = 0, ptsq = 0;  // lane u: the points of record u, and its query
+#pragma unroll
+	for (int u = 0; u < TOP_U; u++) {
+		const uint32_t base = rc[u].x & ~63u;
+		const bool whole = (rc[u].x & RECORD_WHOLE) != 0 || (t.sub_min && base >= 64 && m2[u] <= sm[u]);
+		uint32_t ge = 0;
+#pragma unroll
+		for (int j = 0; j < 4; j++)
+			ge |= m2[u] <= v[u][j] ? 1u << j : 0u;
+		nib[u] &= whole ? 0xFu : ge;
+		const uint32_t n = __reduce_add_sync(FULL, __popc(nib[u]));
+		if (lane == (uint32_t) u) {
+			pts = n;
+			ptsq = rc[u].y;
+		}
+		// 8 lanes make a 32-slot row, two rows a child block
+		uint32_t row = nib[u] << (4 * (lane & 7));
+		row |= __shfl_xor_sync(FULL, row, 1);
+		row |= __shfl_xor_sync(FULL, row, 2);
+		row |= __shfl_xor_sync(FULL, row, 4);
+		const uint32_t lo = __shfl_sync(FULL, row, 16 * (lane & 1)), hi = __shfl_sync(FULL, row, 16 * (lane & 1) + 8);
+		if (lane >> 1 == (uint32_t) u)
+			mine = make_uint4(2 * base + 64 * (lane & 1) + (whole ? RECORD_WHOLE : 0u), rc[u].y, lo, hi);
+	}
+	if (mine.z | mine.w)
+		sh_st4(p.rec + 16 * (base_cur + sh_add(p.cell(d + 1), 1)), mine);
+	if (pts)
+		sh_add(p.cnt + 4 * ptsq, pts);
+}
+
+// Writes the slots of the blocks at[0 .. n) that their masks name, each from output place
+// rec.y on (the place the record has claimed), TOP_U blocks in flight.
+template <typename T>
+__device__ __forceinline__ void top_write(const TreeDev<T> &t, const uint4 *at, uint32_t n, uint32_t ret, void *out)
+{
+	const uint32_t lane = lane_id(), below = lanemask_lt();
+	uint4 rc[TOP_U];
+#pragma unroll
+	for (int u = 0; u < TOP_U; u++)
+		rc[u] = (uint32_t) u < n ? at[u] : make_uint4(0, 0, 0, 0);
+	if (ret == PST_RET_IDS) {
+		uint32_t id[TOP_U][2];
+#pragma unroll
+		for (int u = 0; u < TOP_U; u++)
+#pragma unroll
+			for (int j = 0; j < 2; j++)
+				id[u][j] = ((j ? rc[u].w : rc[u].z) >> lane) & 1u ? t.id[(rc[u].x & ~63u) + 32 * j + lane] : 0u;
+#pragma unroll
+		for (int u = 0; u < TOP_U; u++)
+#pragma unroll
+			for (int j = 0; j < 2; j++) {
+				const uint32_t m = j ? rc[u].w : rc[u].z;
+				if ((m >> lane) & 1u)
+					static_cast<uint32_t *>(out)[rc[u].y + (j ? __popc(rc[u].z) : 0) + __popc(m & below)] = id[u][j];
+			}
+		return;
+	}
+#pragma unroll
+	for (int u = 0; u < TOP_U; u++)
+#pragma unroll
+		for (int j = 0; j < 2; j++) {
+			const uint32_t m = j ? rc[u].w : rc[u].z;
+			if (!((m >> lane) & 1u))
+				continue;
+			const uint32_t h = (rc[u].x & ~63u) + 32 * j + lane;
+			const uint32_t k = rc[u].y + (j ? __popc(rc[u].z) : 0) + __popc(m & below);
+			if (t.id) {
+				Point<T, true> &pt = static_cast<Point<T, true> *>(out)[k];
+				pt.dim1 = t.dim1[h];
+				pt.dim2 = t.dim2[h];
+				pack_id(pt, t.id[h]);
+			} else {
+				Point<T, false> &pt = static_cast<Point<T, false> *>(out)[k];
+				pt.dim1 = t.dim1[h];
+				pt.dim2 = t.dim2[h];
+			}
+		}
+}
+
+template <typename T>
+__global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T> qd, WorkDev wg, uint32_t max_q,
+                                                            uint32_t qcap, uint32_t pcap, uint32_t rcap, QOut<T> qo,
+                                                            const __grid_constant__ TopIn in, BatchCtl *back)
+{
+	extern __shared__ __align__(16) unsigned char s_dyn[];
+	__shared__ uint64_t s_total;
+	__shared__ uint32_t s_word[2];  // flags, reported boundary nodes
+	BatchCtl *sc = reinterpret_cast<BatchCtl *>(s_dyn);
+	uint4 *s_cell = reinterpret_cast<uint4 *>(s_dyn + sizeof(BatchCtl));
+	uint64_t *s_offs = reinterpret_cast<uint64_t *>(s_cell + TOP_CELLS);
+	uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_offs + qcap), *s_cur = s_cnt + qcap;
+	uint4 *s_list = reinterpret_cast<uint4 *>(s_cur + qcap), *s_rec = s_list + 4 * pcap;
+	TopPass<T> p;
+	p.qd = qd;
+	auto addr = [](const void *x) { return static_cast<uint32_t>(__cvta_generic_to_shared(x)); };
+	p.cells = addr(s_cell);
+	p.flags = addr(&s_word[0]);
+	p.rec_cnt = addr(&s_word[1]);
+	p.cnt = addr(s_cnt);
+	p.cur = addr(s_cur);
+	p.lists = addr(s_list);
+	p.rec = addr(s_rec);
+	p.pcap = pcap;
+	p.ro = wg.ro;
+	p.ro_cap = wg.ro_cap;
+	// the start of the pass (k_prepare_queries of a full pass): the counters zeroed, the
+	// queries unpacked and checked, their level-0 paths (at most qcap queries: the host runs
+	// this pass for small batches only)
+	const uint32_t nq = min(in.args.nq, qcap);
+	if (threadIdx.x < 2)
+		s_word[threadIdx.x] = 0;
+	for (uint32_t i = threadIdx.x; i < TOP_CELLS; i += TOP_THREADS)
+		s_cell[i] = make_uint4(0, i ? 0u : nq, 0, 0);
+	for (uint32_t i = threadIdx.x; i < sizeof(BatchCtl) / 4; i += TOP_THREADS)
+		reinterpret_cast<uint32_t *>(sc)[i] = 0;
+	__syncthreads();
+	for (uint32_t i = threadIdx.x; i < qcap; i += TOP_THREADS) {
+		if (i < nq)
+			s_list[i] = unpack_query<T>(in.args.raw ? in.args.raw[i] : in.q[i], i, qo, &s_word[0]);
+		s_cnt[i] = 0;
+		s_cur[i] = 0;
+	}
+	__syncthreads();
+	const uint32_t warp = threadIdx.x >> 5;
+	uint32_t base_prev = 0, base_cur = 0, d = 0;
+	for (; d < t.levels; d++) {
+		const uint4 c = sh_ld4(p.cell(d));
+		const uint32_t prev = c.x, np = min(c.y, pcap), ns = min(c.z, pcap);
+		base_prev = base_cur;
+		base_cur += prev;
+		// the level appends at most two children per record and one record per seed
+		if (prev > CTA_REC_CAP || base_cur + 2 * prev + ns > rcap)
+			break;
+		if (prev + np + ns == 0) {
+			d = t.levels;  // nothing is left on any level below
+			break;
+		}
+		if (threadIdx.x == 0)
+			sh_st(p.cell(d) + 12, base_cur);
+		const uint32_t wp = (np + 31) / 32, ws = (ns + 31) / 32, wr = (prev + TOP_U - 1) / TOP_U;
+		for (uint32_t i = warp; i < wp + ws + wr; i += TOP_WARPS) {
+			if (i < wp)
+				top_paths<T>(t, p, d, 32 * i, np);
+			else if (i < wp + ws)
+				top_seeds<T>(t, p, d, 32 * (i - wp), ns, base_cur);
+			else
+				top_records<T>(t, p, d, base_prev + TOP_U * (i - wp - ws), base_cur, base_cur);
+		}
+		__syncthreads();  // the level's records, paths, seeds and counts are visible to the CTA
+	}
+	// records written: at the bottom the last level's follow base_cur (none, where the pass
+	// ended above it because nothing was left); where the pass stopped at level d, base_cur
+	// is already past level d - 1
+	const bool done = d == t.levels;
+	const uint32_t nrec = min(base_cur + (done ? s_cell[t.levels].x : 0u), rcap);
+	if (done && warp == 0) {
+		uint64_t run = 0;
+		for (uint32_t q0 = 0; q0 < nq; q0 += 32) {
+			const uint32_t q = q0 + lane_id();
+			const uint64_t c = q < nq ? s_cnt[q] : 0u;
+			const uint64_t inc = warp_incl_scan(c);
+			if (q < nq)
+				s_offs[q] = run + inc - c;
+			run += __shfl_sync(FULL, inc, 31);
+		}
+		if (lane_id() == 0)
+			s_total = run;
+	}
+	__syncthreads();
+	const uint64_t total = done ? s_total : 0;
+	const uint32_t flags = s_word[0], nro = min(s_word[1], p.ro_cap);
+	const bool emit = done && in.args.out && total <= in.args.out_cap && total <= CTA_EMIT_CAP &&
+	                  !(flags & (BATCH_FLAG_BAD_QUERY | BATCH_FLAG_INTERNAL));
+	const bool over = !emit && nrec > wg.rec_cap;
+	// the control block: every counter the host and the next kernels read
+	if (threadIdx.x < 40) {
+		const uint4 c = s_cell[threadIdx.x];
+		sc->lvl_cnt[threadIdx.x] = s_cell[threadIdx.x + 1].x;
+		sc->path_cnt[threadIdx.x] = c.y;
+		sc->seed_cnt[threadIdx.x] = c.z;
+		sc->lvl_base[threadIdx.x] = c.w;
+	} else if (threadIdx.x == 64) {
+		sc->rec_cnt = s_word[1];
+		sc->nq = nq;
+		sc->flags = flags | (over ? (uint32_t) BATCH_FLAG_TASK_OVERFLOW : 0u);
+		sc->cta_levels = d;
+		sc->need_tasks = over ? nrec : 0;
+		sc->total = total;
+		sc->emitted = emit;
+	}
+	uint64_t *offsets = const_cast<uint64_t *>(wg.offsets);
+	if (done) {
+		for (uint32_t q = threadIdx.x; q <= max_q; q += TOP_THREADS)
+			offsets[q] = q < nq ? s_offs[q] : total;
+		if (in.args.offsets)
+			for (uint32_t q = threadIdx.x; q <= nq; q += TOP_THREADS)
+				in.args.offsets[q] = q < nq ? s_offs[q] : total;
+	}
+	for (uint32_t q = threadIdx.x; q < max_q; q += TOP_THREADS) {
+		wg.counts[q] = q < nq ? s_cnt[q] : 0u;
+		wg.cursor[q] = 0;
+	}
+	if (emit) {
+		// every record claims its place (kept where its query was); the reported boundary
+		// nodes follow them as records of one slot
+		for (uint32_t i = threadIdx.x; i < nrec; i += TOP_THREADS) {
+			const uint4 x = s_rec[i];
+			s_rec[i].y = (uint32_t) s_offs[x.y] + sh_add(p.cur + 4 * x.y, (uint32_t) (__popc(x.z) + __popc(x.w)));
+		}
+		for (uint32_t i = threadIdx.x; i < nro; i += TOP_THREADS) {
+			const uint32_t q = p.ro[i].y;
+			p.ro[i].y = (uint32_t) s_offs[q] + sh_add(p.cur + 4 * q, 1);
+		}
+		__syncthreads();
+		for (uint32_t i = warp * TOP_U; i < nrec; i += TOP_WARPS * TOP_U)
+			top_write<T>(t, s_rec + i, min(nrec - i, (uint32_t) TOP_U), in.args.ret, in.args.out);
+		for (uint32_t i = warp * TOP_U; i < nro; i += TOP_WARPS * TOP_U)
+			top_write<T>(t, p.ro + i, min(nro - i, (uint32_t) TOP_U), in.args.ret, in.args.out);
+	} else {
+		for (uint32_t i = threadIdx.x; i < nrec && nrec <= wg.rec_cap; i += TOP_THREADS)
+			wg.rec[i] = s_rec[i];
+		if (!done) {
+			const uint32_t np = min(s_cell[d].y, pcap), ns = min(s_cell[d].z, pcap);
+			uint4 *pd = (d & 1) ? wg.path1 : wg.path0, *sd = (d & 1) ? wg.seed1 : wg.seed0;
+			for (uint32_t i = threadIdx.x; i < np; i += TOP_THREADS)
+				pd[i] = s_list[(d & 1) * pcap + i];
+			for (uint32_t i = threadIdx.x; i < ns; i += TOP_THREADS)
+				sd[i] = s_list[(2 + (d & 1)) * pcap + i];
+		}
+	}
+	__syncthreads();
+	if (threadIdx.x < sizeof(BatchCtl) / 4) {
+		const uint32_t x = reinterpret_cast<const uint32_t *>(sc)[threadIdx.x];
+		reinterpret_cast<uint32_t *>(wg.ctl)[threadIdx.x] = x;
+		if (back)
+			reinterpret_cast<uint32_t *>(back)[threadIdx.x] = x;
+	}
+}
+
+// Shared memory the one-CTA top pass may take beyond its static arrays on the
+// current device, after allowing it for the kernel there (once per device; done
+// before any launch is captured into a graph).
+template <typename T>
+size_t cta_pass_budget()
+{
+	static std::mutex mu;
+	static size_t budget[64];
+	static bool done[64] = {};
+	const DeviceInfo &di = device_info();
+	std::lock_guard<std::mutex> lk(mu);
+	if (!done[di.device]) {
+		cudaFuncAttributes a{};
+		PST_CUDA(cudaFuncGetAttributes(&a, k_bfs_cta<T>));
+		const size_t b = di.smem_optin > a.sharedSizeBytes + 1024 ? di.smem_optin - a.sharedSizeBytes - 1024 : 0;
+		PST_CUDA(cudaFuncSetAttribute(k_bfs_cta<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b));
+		budget[di.device] = b;
+		done[di.device] = true;
+	}
+	return budget[di.device];
+}
+
+// Launches the one-CTA top pass of at most qcap queries: two paths and two seeds for each
+// in the lists, and as many records as the rest of the CTA's shared memory holds.
+template <typename T>
+void launch_cta_pass(const TreeDev<T> &tv, const QDev<T> &qd, const WorkDev &w, uint32_t max_q, uint32_t qcap,
+                     const QOut<T> &qo, const TopIn &in, BatchCtl *back, cudaStream_t s)
+{
+	const size_t budget = cta_pass_budget<T>();
+	const uint32_t pcap = 2 * qcap;
+	const size_t fixed = cta_smem_bytes((qcap + 1) & ~1u, pcap, 0);
+	// room for at least one level's records beyond the lists
+	if (budget < fixed + (size_t) (2 * CTA_REC_CAP + pcap) * sizeof(uint4))
+		fail(PST_ERR_INTERNAL, "shared memory too small for the top pass of " + std::to_string(max_q) + " queries");
+	const uint32_t rcap = (uint32_t) ((budget - fixed) / sizeof(uint4));
+	k_bfs_cta<T><<<1, TOP_THREADS, cta_smem_bytes((qcap + 1) & ~1u, pcap, rcap), s>>>(
+	    tv, qd, w, max_q, (qcap + 1) & ~1u, pcap, rcap, qo, in, back);
 }
 
 // THREADS: the CTA size and U the records each warp has in flight (both tuning
@@ -1228,7 +1485,6 @@ void Batch::Graph::drop()
 void Batch::release()
 {
 	full_graph.drop();
-	top_graph.drop();
 	if (passes)
 		passes->wait(this);  // an asynchronous pass may still use the buffers
 	pool_release(work, device);
@@ -1302,10 +1558,18 @@ void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 		work = pool_alloc(off, "batch workspace");
 		layout();
 	}
-	ctl_host = static_cast<BatchCtl *>(pinned_alloc(sizeof(BatchCtl) + (size_t) max_q * sizeof(pst_query), "query staging"));
-	q_stage = reinterpret_cast<pst_query *>(ctl_host + 1);
-	memset(ctl_host, 0, sizeof(BatchCtl));
-	PST_CUDA(cudaHostGetDevicePointer((void **) &ctl_host_d, ctl_host, 0));
+	const size_t head = 2 * sizeof(BatchCtl);
+	ctl_host = static_cast<BatchCtl *>(pinned_alloc(head + (size_t) max_q * sizeof(pst_query), "query staging"));
+	back = ctl_host + 1;
+	q_stage = reinterpret_cast<pst_query *>(back + 1);
+	memset(ctl_host, 0, head);
+	void *mapped = nullptr;
+	PST_CUDA(cudaHostGetDevicePointer(&mapped, ctl_host, 0));
+	BatchCtl *ctl_d = static_cast<BatchCtl *>(mapped);
+	ctl_host_d = ctl_d;
+	back_d = ctl_d + 1;
+	q_stage_d = reinterpret_cast<const pst_query *>(back_d + 1);
+	idle = true;
 	const uint64_t want = o.task_capacity ? o.task_capacity : std::max<uint64_t>(1ull << 16, (uint64_t) max_q * 64);
 	rec = static_cast<uint4 *>(pool_alloc(want * sizeof(uint4), "frontier"));
 	task_cap = want;
@@ -1324,7 +1588,6 @@ void Batch::grow_tasks(uint64_t cap, cudaStream_t s)
 	task_cap = cap;
 	// the captured passes hold the old frontier's address
 	full_graph.drop();
-	top_graph.drop();
 }
 
 #define PST_WORKDEV                                                                                                   \
@@ -1352,10 +1615,9 @@ void Batch::enqueue_count_top(cudaStream_t s)
 	TreeDev<T> tv = tree->view<T>();
 	QDev<T> qd{kind, static_cast<const T *>(min1), static_cast<const T *>(max1), static_cast<const T *>(min2)};
 	PST_WORKDEV;
-	// one kernel: the control block read from its pinned host copy, the queries
-	// unpacked and the whole top pass
+	// one kernel: the queries unpacked and the whole top pass
 	const QOut<T> qo{kind, static_cast<T *>(min1), static_cast<T *>(max1), static_cast<T *>(min2)};
-	launch_cta_pass<T>(tv, qd, w, max_q, 2 * std::min(top_q, max_q), q_raw, qo, ctl_host_d, s);
+	launch_cta_pass<T>(tv, qd, w, max_q, std::min(top_q, max_q), qo, top_in, back_d, s);
 	PST_CUDA(cudaGetLastError());
 }
 
@@ -1462,7 +1724,7 @@ void Batch::launch_count_top(cudaStream_t s)
 {
 	if (ctl_host->nq > top_q)
 		fail(PST_ERR_INTERNAL, "top pass on a batch of more than " + std::to_string(top_q) + " queries");
-	launch_graph(top_graph, &Batch::enqueue_counting_top, s);
+	enqueue_counting_top(s);
 }
 
 void Batch::launch_count_rest(uint32_t from, cudaStream_t s)
@@ -1474,7 +1736,7 @@ void Batch::launch_count_rest(uint32_t from, cudaStream_t s)
 	}
 }
 
-void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s)
+void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, bool whole)
 {
 	if (nq > max_q)
 		fail(PST_ERR_INVALID, "batch of " + std::to_string(nq) + " queries exceeds max_queries " +
@@ -1482,49 +1744,67 @@ void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaS
 	if (nq && !q)
 		fail(PST_ERR_INVALID, "null query array");
 	// the pinned control block and query staging may still feed an earlier pass
-	PST_CUDA(cudaStreamSynchronize(s));
+	if (!idle)
+		PST_CUDA(cudaStreamSynchronize(s));
+	idle = false;
 	ctl_host->nq = nq;
-	if (nq) {
-		if (on_device) {
-			PST_CUDA(cudaMemcpyAsync(q_raw, q, (size_t) nq * sizeof(pst_query), cudaMemcpyDeviceToDevice, s));
-		} else {
-			memcpy(q_stage, q, (size_t) nq * sizeof(pst_query));
-			PST_CUDA(cudaMemcpyAsync(q_raw, q_stage, (size_t) nq * sizeof(pst_query), cudaMemcpyHostToDevice, s));
-		}
+	top_in.args = TopArgs{};
+	top_in.args.nq = nq;
+	if (!whole && nq <= TOP_IN_QUERIES && !on_device) {
+		std::copy(q, q + nq, top_in.q);
+		return;
+	}
+	if (!on_device && nq)
+		memcpy(q_stage, q, (size_t) nq * sizeof(pst_query));
+	if (!whole && nq <= top_q) {
+		top_in.args.raw = on_device ? q : q_stage_d;  // the top pass reads them where they are
+	} else if (nq) {
+		PST_CUDA(cudaMemcpyAsync(q_raw, on_device ? q : q_stage, (size_t) nq * sizeof(pst_query),
+		                         on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
 	}
 }
 
-pst_status Batch::read_ctl(cudaStream_t s, uint64_t *total)
+// The device's control block into `last`, once the work on `s` is done.
+void Batch::fetch_ctl(cudaStream_t s)
 {
-	BatchCtl h;
-	PST_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
+	PST_CUDA(cudaMemcpyAsync(back, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
 	PST_CUDA(cudaStreamSynchronize(s));
-	last = h;
-	if (total)
-		*total = h.total;
-	if (h.flags & BATCH_FLAG_BAD_QUERY)
+	last = *back;
+}
+
+pst_status Batch::last_status() const
+{
+	if (last.flags & BATCH_FLAG_BAD_QUERY)
 		return PST_ERR_INVALID;
-	if (h.flags & (BATCH_FLAG_TASK_OVERFLOW | BATCH_FLAG_INTERNAL))
+	if (last.flags & (BATCH_FLAG_TASK_OVERFLOW | BATCH_FLAG_INTERNAL))
 		return PST_ERR_INTERNAL;
-	if (h.flags & BATCH_FLAG_OUT_OVERFLOW)
+	if (last.flags & BATCH_FLAG_OUT_OVERFLOW)
 		return PST_ERR_CAPACITY;
 	return PST_OK;
 }
 
-// Count pass with the host waiting for it.
-void Batch::count_sync(cudaStream_t s, uint64_t *total)
+pst_status Batch::read_ctl(cudaStream_t s, uint64_t *total)
 {
-	if (ctl_host->nq <= top_q)
-		count_small_sync(s, total);
-	else
-		count_full_sync(s, total);
+	fetch_ctl(s);
+	if (total)
+		*total = last.total;
+	return last_status();
 }
 
-// Reads the control block after a pass; true when it is complete, false when the
-// frontier overflowed (and has been grown for another attempt).
-static bool settle(Batch &b, const BatchCtl &h, int attempt, cudaStream_t s, uint64_t *total)
+// Count pass with the host waiting for it.
+void Batch::count_sync(cudaStream_t s, uint64_t *total, const EmitTo *to)
 {
-	b.last = h;
+	if (ctl_host->nq <= top_q)
+		count_small_sync(s, total, to);
+	else
+		count_full_sync(s, total, to);
+}
+
+// Reads the control block of a pass (b.last); true when it is complete, false when the
+// frontier overflowed (and has been grown for another attempt).
+static bool settle(Batch &b, int attempt, cudaStream_t s, uint64_t *total)
+{
+	const BatchCtl &h = b.last;
 	if (h.flags & BATCH_FLAG_BAD_QUERY)
 		fail(PST_ERR_INVALID, "query kind must be PST_Q_THREE, PST_Q_LEFT or PST_Q_RIGHT");
 	if (h.flags & BATCH_FLAG_INTERNAL)
@@ -1539,15 +1819,26 @@ static bool settle(Batch &b, const BatchCtl &h, int attempt, cudaStream_t s, uin
 	return false;
 }
 
+// Queues the emit and the copy of the offsets behind a count pass: the emit writes
+// nothing when the pass did not fit the frontier or its results the buffer.
+void Batch::emit_to(const EmitTo &to, cudaStream_t s)
+{
+	if (to.offsets)
+		PST_CUDA(cudaMemcpyAsync(to.offsets, offsets, ((size_t) ctl_host->nq + 1) * 8, cudaMemcpyDeviceToDevice, s));
+	if (to.out && to.capacity)
+		enqueue_emit(to.ret, to.out, to.capacity, s);
+}
+
 // The whole pass, with automatic growth of the frontier buffer.
-void Batch::count_full_sync(cudaStream_t s, uint64_t *total)
+void Batch::count_full_sync(cudaStream_t s, uint64_t *total, const EmitTo *to)
 {
 	for (int attempt = 0;; attempt++) {
 		launch_count(s);
-		BatchCtl h;
-		PST_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
-		PST_CUDA(cudaStreamSynchronize(s));
-		if (settle(*this, h, attempt, s, total))
+		if (to)
+			emit_to(*to, s);
+		fetch_ctl(s);
+		idle = true;
+		if (settle(*this, attempt, s, total))
 			return;
 	}
 }
@@ -1555,20 +1846,31 @@ void Batch::count_full_sync(cudaStream_t s, uint64_t *total)
 // A small batch: the one-CTA top pass, then, if it stopped above the bottom, the
 // per-level kernels for the rest and the scan; with automatic growth of the
 // frontier buffer as in count_full_sync.
-void Batch::count_small_sync(cudaStream_t s, uint64_t *total)
+void Batch::count_small_sync(cudaStream_t s, uint64_t *total, const EmitTo *to)
 {
+	if (to) {
+		top_in.args.out = to->capacity ? to->out : nullptr;
+		top_in.args.out_cap = to->capacity;
+		top_in.args.offsets = to->offsets;
+		top_in.args.ret = to->ret;
+	}
 	for (int attempt = 0;; attempt++) {
 		launch_count_top(s);
-		BatchCtl h;
-		PST_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
 		PST_CUDA(cudaStreamSynchronize(s));
-		if (!(h.flags & (BATCH_FLAG_BAD_QUERY | BATCH_FLAG_INTERNAL | BATCH_FLAG_TASK_OVERFLOW)) &&
-		    h.cta_levels < tree->levels) {
-			launch_count_rest(h.cta_levels, s);
-			PST_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
-			PST_CUDA(cudaStreamSynchronize(s));
+		last = *back;
+		idle = true;
+		if (!(last.flags & (BATCH_FLAG_BAD_QUERY | BATCH_FLAG_INTERNAL | BATCH_FLAG_TASK_OVERFLOW))) {
+			if (last.cta_levels < tree->levels) {
+				launch_count_rest(last.cta_levels, s);
+				if (to)
+					emit_to(*to, s);
+				fetch_ctl(s);
+			} else if (to && to->out && !last.emitted && last.total && last.total <= to->capacity) {
+				enqueue_emit(to->ret, to->out, to->capacity, s);  // the pass wrote the offsets
+				fetch_ctl(s);
+			}
 		}
-		if (settle(*this, h, attempt, s, total))
+		if (settle(*this, attempt, s, total))
 			return;
 	}
 }
@@ -1598,8 +1900,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH
 
 // Sub-buffers of the scratch array, 256-byte aligned, in bytes.
 constexpr size_t NA_CTL = 0;
-constexpr size_t NA_QRAW = 1024;
-constexpr size_t NA_KIND = NA_QRAW + 256;
+constexpr size_t NA_KIND = 1024;
 constexpr size_t NA_MIN1 = NA_KIND + 256;
 constexpr size_t NA_MAX1 = NA_MIN1 + 256;
 constexpr size_t NA_MIN2 = NA_MAX1 + 256;
@@ -1616,7 +1917,7 @@ constexpr size_t NA_SCAN = NA_OFFSETS + 256;
 constexpr size_t NA_RECS = NA_SCAN + 256;
 // alive records (16 B each) take the rest
 constexpr uint64_t NA_REC_CAP = (NOALLOC_SCRATCH_BYTES - NA_RECS) / sizeof(uint4) / 64 * 64;
-static_assert(sizeof(BatchCtl) <= NA_QRAW, "control block");
+static_assert(sizeof(BatchCtl) <= NA_KIND, "control block");
 static_assert(NA_RECS + NA_REC_CAP * sizeof(uint4) <= NOALLOC_SCRATCH_BYTES, "scratch layout");
 // One query has at most one alive record per 64-slot block of every level, plus the
 // records of report-above subtrees that still share a block with another subtree:
@@ -1659,7 +1960,6 @@ uint64_t noalloc_run(TreeStorage &t, const pst_query &q, pst_ret ret, void *out,
                      unsigned char *base)
 {
 	BatchCtl *ctl = reinterpret_cast<BatchCtl *>(base + NA_CTL);
-	pst_query *qraw = reinterpret_cast<pst_query *>(base + NA_QRAW);
 	uint32_t *kind = reinterpret_cast<uint32_t *>(base + NA_KIND);
 	T *min1 = reinterpret_cast<T *>(base + NA_MIN1);
 	T *max1 = reinterpret_cast<T *>(base + NA_MAX1);
@@ -1675,12 +1975,15 @@ uint64_t noalloc_run(TreeStorage &t, const pst_query &q, pst_ret ret, void *out,
 	uint64_t *scan = reinterpret_cast<uint64_t *>(base + NA_SCAN);
 	uint4 *rec = reinterpret_cast<uint4 *>(base + NA_RECS);
 
-	// The array keeps the previous call's contents: the control block starts over
-	// (with nq = 1) here, and the top pass zeroes the query's count and output cursor.
+	// The array keeps the previous call's contents: the top pass starts the control block,
+	// the query's count and its output cursor over.
 	BatchCtl h{};
-	h.nq = 1;
-	PST_CUDA(cudaMemcpyAsync(ctl, &h, sizeof(BatchCtl), cudaMemcpyHostToDevice, s));
-	PST_CUDA(cudaMemcpyAsync(qraw, &q, sizeof(pst_query), cudaMemcpyHostToDevice, s));
+	TopIn in{};
+	in.q[0] = q;
+	in.args.nq = 1;
+	in.args.out = out;
+	in.args.out_cap = capacity;
+	in.args.ret = ret;
 
 	int occ = 0;
 	PST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bfs_kernel_ptr<T>(BFS_THREADS), BFS_THREADS, 0));
@@ -1690,7 +1993,7 @@ uint64_t noalloc_run(TreeStorage &t, const pst_query &q, pst_ret ret, void *out,
 	WorkDev w{rec, NA_REC_CAP, path0, path1, seed0, seed1, 2u, ro, NA_RO_CAP, counts, cursor, offsets, ctl};
 	// the one-CTA top pass (which unpacks the query and zeroes its count and output
 	// cursor), then the per-level kernels for whatever it left
-	launch_cta_pass<T>(tv, qd, w, 1u, 2u, qraw, QOut<T>{kind, min1, max1, min2}, ctl, s);
+	launch_cta_pass<T>(tv, qd, w, 1u, 1u, QOut<T>{kind, min1, max1, min2}, in, nullptr, s);
 	PST_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
 	PST_CUDA(cudaStreamSynchronize(s));
 	if (!(h.flags & (BATCH_FLAG_BAD_QUERY | BATCH_FLAG_INTERNAL | BATCH_FLAG_TASK_OVERFLOW)) &&
@@ -1705,7 +2008,7 @@ uint64_t noalloc_run(TreeStorage &t, const pst_query &q, pst_ret ret, void *out,
 		fail(PST_ERR_INVALID, "query kind must be PST_Q_THREE, PST_Q_LEFT or PST_Q_RIGHT");
 	if (h.flags & (BATCH_FLAG_TASK_OVERFLOW | BATCH_FLAG_INTERNAL))
 		fail(PST_ERR_INTERNAL, "no-alloc search: frontier consistency check failed");
-	if (h.total == 0 || h.total > capacity)
+	if (h.total == 0 || h.total > capacity || h.emitted)
 		return h.total;
 	const bool has_id = t.idtype == PST_ID_U32;
 	if (ret == PST_RET_IDS)

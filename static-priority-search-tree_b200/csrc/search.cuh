@@ -37,6 +37,33 @@ struct BatchCtl {
 	// kernel that fills the region, so the next kernel reads its bounds in one load
 	// each instead of summing every count before them
 	uint64_t lvl_base[40];
+	uint32_t emitted;       // the top pass wrote the results itself
+	uint32_t unused[3];
+};
+
+// What the top pass of a small batch works on (kernel parameters).
+struct TopArgs {
+	const pst_query *raw;   // the queries: null (they come along), mapped pinned memory or the
+	                        // caller's device array
+	void *out;              // where a pass that fits may write its results (null: count only)
+	uint64_t out_cap;       // records `out` holds
+	uint64_t *offsets;      // the caller's nq + 1 offsets, or null
+	uint32_t ret;           // pst_ret
+	uint32_t nq;
+};
+
+constexpr uint32_t TOP_IN_QUERIES = 32;  // host queries that come along
+struct TopIn {
+	TopArgs args;
+	pst_query q[TOP_IN_QUERIES];
+};
+
+// Where a waiting call wants its results.
+struct EmitTo {
+	pst_ret ret;
+	void *out;
+	uint64_t capacity;
+	uint64_t *offsets;      // nq + 1 on the device, or null
 };
 
 struct Batch {
@@ -66,41 +93,56 @@ struct Batch {
 	uint32_t ro_cap = 0;
 	uint64_t *counts = nullptr, *cursor = nullptr, *offsets = nullptr, *scan_tmp = nullptr;
 	BatchCtl *ctl = nullptr;
-	BatchCtl *ctl_host = nullptr;  // pinned, zeroed except nq
-	const BatchCtl *ctl_host_d = nullptr;  // its device address (mapped pinned memory)
+	// One mapped pinned block: the control block a whole pass starts from (zeroed except
+	// nq), the control block a pass ended with, the staged queries.  The _d pointers are
+	// device addresses.
+	BatchCtl *ctl_host = nullptr;
+	const BatchCtl *ctl_host_d = nullptr;
+	BatchCtl *back = nullptr;
+	BatchCtl *back_d = nullptr;
+	const pst_query *q_stage_d = nullptr;
+	TopIn top_in{};
+	bool idle = false;             // no pass that uses the block can be in flight
 	BatchCtl last{};
-	// captured passes, each for the stream it was captured for: the whole count pass,
-	// and the top pass of small batches
+	// the captured whole count pass, for the stream it was captured for
 	struct Graph {
 		cudaGraphExec_t exec = nullptr;
 		cudaStream_t stream = nullptr;
 		uint32_t direct = 0;  // passes launched on `stream` without it
 		void drop();
 	};
-	Graph full_graph, top_graph;
+	Graph full_graph;
 
 	~Batch();
 	void init(TreeStorage *t, const pst_batch_opts &o);
 	void release();
 	void grow_tasks(uint64_t cap, cudaStream_t s);
-	void stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s);
+	// whole: for a pass that never starts with the top pass.
+	void stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, bool whole = false);
 	// Whole count pass (every level kernel and the scan), asynchronous.
 	void launch_count(cudaStream_t s);
 	// Notes that work queued on `s` may still run when the call returns.
-	void mark_async(cudaStream_t s) { passes->mark(this, s); }
+	void mark_async(cudaStream_t s)
+	{
+		idle = false;
+		passes->mark(this, s);
+	}
 	// Top pass of a small batch (nq <= top_q), asynchronous: when it stops
 	// above the bottom (ctl->cta_levels < tree levels), launch_count_rest finishes it.
 	void launch_count_top(cudaStream_t s);
 	void launch_count_rest(uint32_t from, cudaStream_t s);
 	// Count pass with the host waiting for it: the top pass for small batches, the
-	// whole pass otherwise; grows the frontier buffer until the pass fits.
-	void count_sync(cudaStream_t s, uint64_t *total);
-	void count_full_sync(cudaStream_t s, uint64_t *total);
-	void count_small_sync(cudaStream_t s, uint64_t *total);
+	// whole pass otherwise; grows the frontier buffer until the pass fits.  With `to` the
+	// results (when they fit) and offsets are written too, before the one wait that the
+	// pass ends with; read_ctl's status of the last pass tells how that went.
+	void count_sync(cudaStream_t s, uint64_t *total, const EmitTo *to = nullptr);
+	void count_full_sync(cudaStream_t s, uint64_t *total, const EmitTo *to);
+	void count_small_sync(cudaStream_t s, uint64_t *total, const EmitTo *to);
 	void enqueue_counting(cudaStream_t s);
 	void enqueue_counting_top(cudaStream_t s);
 	void enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s);
 	pst_status read_ctl(cudaStream_t s, uint64_t *total);
+	pst_status last_status() const;  // of the control block read last
 	uint64_t record_size(pst_ret ret) const;
 
   private:
@@ -110,6 +152,8 @@ struct Batch {
 	void enqueue_count_top(cudaStream_t s);
 	template <typename T>
 	void enqueue_count_rest(uint32_t from, cudaStream_t s);
+	void emit_to(const EmitTo &to, cudaStream_t s);
+	void fetch_ctl(cudaStream_t s);
 	void launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStream_t s);
 	template <typename T>
 	void enqueue_emit_v(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s);

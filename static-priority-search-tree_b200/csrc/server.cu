@@ -594,10 +594,11 @@ uint32_t server_add_tree(Server *s, TreeStorage *t, const pst_batch_opts *tuning
 				q.min1.i32 = 1;
 				q.max1.i32 = 0;
 			}
-			sl->eng.stage_queries(&q, 1, false, sl->stream);
 			uint64_t total = 0;
-			sl->eng.count_full_sync(sl->stream, &total);
-			sl->eng.count_small_sync(sl->stream, &total);
+			sl->eng.stage_queries(&q, 1, false, sl->stream, true);
+			sl->eng.count_full_sync(sl->stream, &total, nullptr);
+			sl->eng.stage_queries(&q, 1, false, sl->stream);
+			sl->eng.count_small_sync(sl->stream, &total, nullptr);
 		}
 		check_cuda(cudaEventCreateWithFlags(&sl->ev, cudaEventDisableTiming), "cudaEventCreate");
 		check_cuda(cudaMallocHost((void **) &sl->ctl_h, sizeof(BatchCtl)), "cudaMallocHost");
