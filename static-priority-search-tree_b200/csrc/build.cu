@@ -1221,100 +1221,136 @@ void build_tree(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 
 namespace {
 
-// Block j of level L: positions [2^L + 64 j, 2^L + 64 j + 64); its children are the
-// 128 positions from 2^(L+1) + 128 j, i.e. occupancy words 2^(L+1)/32 + 4 j .. + 3.
-__global__ void k_last_par(const uint32_t *__restrict__ occ, uint32_t L, uint32_t *out)
-{
-	const uint64_t nb = (1ull << L) / 64;
-	const uint64_t w0 = (1ull << (L + 1)) / 32;
-	for (uint64_t j = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; j < ((nb + 31) & ~31ull);
-	     j += (uint64_t) gridDim.x * blockDim.x) {
-		bool any = false;
-		if (j < nb) {
-			const uint4 o = *reinterpret_cast<const uint4 *>(occ + w0 + 4 * j);
-			any = (o.x | o.y | o.z | o.w) != 0;
-		}
-		const uint32_t bits = __ballot_sync(0xFFFFFFFFu, any);
-		if ((threadIdx.x & 31) == 0)
-			out[j >> 5] = bits;
-	}
-}
-
 // Minimum of two dim2 values that keeps a NaN (so that no query's min2 compares
 // at most the minimum of a block with a NaN below it).
-template <typename T>
-__device__ __forceinline__ T min_keep_nan(T a, T b)
+__device__ __forceinline__ float min_keep_nan(float a, float b)
 {
-	if constexpr (std::is_floating_point<T>::value) {
-		if (a != a)
-			return a;
-		if (b != b)
-			return b;
-	}
-	return b < a ? b : a;
+	float r;
+	asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+__device__ __forceinline__ int32_t min_keep_nan(int32_t a, int32_t b) { return min(a, b); }
+__device__ __forceinline__ double min_keep_nan(double a, double b) { return a != a || a < b ? a : b; }
+
+// A block without descendants holds nothing to test: the largest value.
+template <typename T>
+__device__ __forceinline__ T min_of_none()
+{
+	if constexpr (std::is_floating_point<T>::value)
+		return std::numeric_limits<T>::infinity();
+	else
+		return std::numeric_limits<T>::max();
 }
 
-// sub_min of the 64-slot blocks of level e (one warp per block): its 128 children
-// on level e + 1 (positions 2^(e+1) + 128 j ..), only the occupied ones when that
-// is the last level, and the sub_min of the two child blocks below them.
+// sub_min of the 64-slot blocks of levels e, e - 1, .. e - depth + 1, and (where e is level
+// D - 2) one bit per block of level e: does any of its children exist (last_par).  A block's
+// value is the smallest dim2 of its 128 children on the level below it (positions
+// 2^(level + 1) + 128 j ..; only the occupied ones on the last level) and of the two child
+// blocks' values.  A CTA owns 2^(depth - 1) consecutive blocks of level e and all their
+// ancestors down to one: the minima of their own children are independent reads, whatever
+// the level, and the blocks' values are then folded up in shared memory.  SM_DEPTH levels a
+// launch in place of one each: 2^26 points 256 us in 21 launches, 148 in 3; 2^21 40, 21.  (Level by
+// level inside the CTA, with a barrier between them: 189 us.)
+constexpr int SM_DEPTH = 7, SM_THREADS = 256, SM_WARPS = SM_THREADS / 32;
+
 template <typename T>
-__global__ void k_sub_min(const T *__restrict__ dim2, const uint32_t *__restrict__ occ, T *sub_min, uint32_t D,
-                          uint32_t e)
+__global__ void __launch_bounds__(SM_THREADS) k_sub_min(const T *__restrict__ dim2, const uint32_t *__restrict__ occ,
+                                                        T *sub_min, uint32_t *last_par, uint32_t D, uint32_t e,
+                                                        uint32_t depth)
 {
-	const uint64_t nb = (1ull << e) / 64;
-	const uint32_t lane = threadIdx.x & 31;
-	for (uint64_t j = ((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < nb;
-	     j += ((uint64_t) gridDim.x * blockDim.x) >> 5) {
-		const uint64_t c0 = (1ull << (e + 1)) + 128 * j;  // first child position
-		const uint64_t p = c0 + 4 * lane;
-		T v[4];
-		if constexpr (sizeof(T) == 4) {
-			const uint4 x = *reinterpret_cast<const uint4 *>(dim2 + p);
-			memcpy(&v[0], &x.x, 4);
-			memcpy(&v[1], &x.y, 4);
-			memcpy(&v[2], &x.z, 4);
-			memcpy(&v[3], &x.w, 4);
-		} else {
-			const double2 a = reinterpret_cast<const double2 *>(dim2 + p)[0];
-			const double2 b = reinterpret_cast<const double2 *>(dim2 + p)[1];
-			v[0] = a.x;
-			v[1] = a.y;
-			v[2] = b.x;
-			v[3] = b.y;
-		}
-		// children on the last level exist where their occupancy bit is set
-		const uint32_t om = e + 2 == D ? (occ[p >> 5] >> (p & 31)) & 0xFu : 0xFu;
-		bool have = false;
-		T m = T(0);
+	// the blocks in order of their level, e first, and of their place: block b of n is the
+	// (2^(l + 1) - 1 - r)-th of 2^l blocks on level e - depth + 1 + l, r = n - b, l = log2 r
+	__shared__ T s_min[1 << SM_DEPTH];
+	__shared__ uint32_t s_any[2];
+	constexpr int U = sizeof(T) == 4 ? 4 : 2;  // blocks in flight per warp
+	const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+	const uint32_t n = (1u << depth) - 1, nb = 1u << (depth - 1);
+	const bool last = e + 2 == D;
+	if (threadIdx.x < 2)
+		s_any[threadIdx.x] = 0;
+	__syncthreads();
+	for (uint32_t b0 = warp * U; b0 < n; b0 += SM_WARPS * U) {
+		T v[U][4];
+		uint32_t om[U];
+		uint64_t p[U];
 #pragma unroll
-		for (int k = 0; k < 4; k++)
-			if ((om >> k) & 1u) {
-				m = have ? min_keep_nan(m, v[k]) : v[k];
-				have = true;
+		for (int u = 0; u < U; u++) {
+			const uint32_t b = b0 + u, r = b < n ? n - b : 1u, l = 31 - __clz(r), lv = e - depth + 1 + l;
+			const uint64_t j = ((uint64_t) blockIdx.x << l) + (2u << l) - 1 - r;
+			p[u] = (1ull << (lv + 1)) + 128 * j + 4 * lane;
+			om[u] = b >= n ? 0u : last && b < nb ? (occ[p[u] >> 5] >> (p[u] & 31)) & 0xFu : 0xFu;
+		}
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			if (!om[u])
+				continue;  // a last level is often almost empty
+			if constexpr (sizeof(T) == 4) {
+				const uint4 x = *reinterpret_cast<const uint4 *>(dim2 + p[u]);
+				memcpy(&v[u][0], &x.x, 4);
+				memcpy(&v[u][1], &x.y, 4);
+				memcpy(&v[u][2], &x.z, 4);
+				memcpy(&v[u][3], &x.w, 4);
+			} else {
+				const double2 a = reinterpret_cast<const double2 *>(dim2 + p[u])[0];
+				const double2 c = reinterpret_cast<const double2 *>(dim2 + p[u])[1];
+				v[u][0] = a.x;
+				v[u][1] = a.y;
+				v[u][2] = c.x;
+				v[u][3] = c.y;
 			}
-		if (lane == 0 && e + 2 < D) {
-			// the child blocks' own descendants (levels e + 2 .. D - 1)
-			const T a = sub_min[c0 >> 6], b = sub_min[(c0 >> 6) + 1];
-			m = have ? min_keep_nan(min_keep_nan(m, a), b) : min_keep_nan(a, b);
-			have = true;
 		}
 #pragma unroll
-		for (int o = 16; o > 0; o >>= 1) {
-			const T om2 = __shfl_xor_sync(0xFFFFFFFFu, m, o);
-			const bool oh = __shfl_xor_sync(0xFFFFFFFFu, have, o);
-			if (oh)
-				m = have ? min_keep_nan(m, om2) : om2;
-			have = have || oh;
+		for (int u = 0; u < U; u++) {
+			if (b0 + u >= n)
+				break;
+			T m = min_of_none<T>();
+			if (__any_sync(0xFFFFFFFFu, om[u])) {
+#pragma unroll
+				for (int q = 0; q < 4; q++)
+					m = (om[u] >> q) & 1u ? min_keep_nan(m, v[u][q]) : m;
+#pragma unroll
+				for (int o = 16; o > 0; o >>= 1)
+					m = min_keep_nan(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+				if (last && b0 + u < nb && lane == 0)
+					atomicOr(&s_any[(b0 + u) >> 5], 1u << ((b0 + u) & 31));
+			}
+			if (lane == 0)
+				s_min[b0 + u] = m;
 		}
-		if (lane == 0) {
-			// a block without descendants holds nothing to test: the largest value
-			T none;
-			if constexpr (std::is_floating_point<T>::value)
-				none = std::numeric_limits<T>::infinity();
-			else
-				none = std::numeric_limits<T>::max();
-			sub_min[((1ull << e) >> 6) + j] = have ? m : none;
+	}
+	__syncthreads();
+	// the child blocks' values: of the launch before, then of the level just folded
+	for (uint32_t l = depth; l-- > 0;) {
+		const uint32_t on = 1u << l, at = n + 1 - (2u << l);  // blocks of the level, and their place
+		for (uint32_t i = threadIdx.x; i < on; i += SM_THREADS) {
+			T m = s_min[at + i];
+			const uint64_t j = ((1ull << (e - depth + 1 + l)) >> 6) + ((uint64_t) blockIdx.x << l) + i;
+			if (l + 1 < depth)
+				m = min_keep_nan(m, min_keep_nan(s_min[at - 2 * on + 2 * i], s_min[at - 2 * on + 2 * i + 1]));
+			else if (!last)
+				m = min_keep_nan(m, min_keep_nan(sub_min[2 * j], sub_min[2 * j + 1]));
+			s_min[at + i] = m;
+			sub_min[j] = m;
 		}
+		__syncthreads();
+	}
+	// the CTA's bits: whole words of last_par, or (below 32 blocks in all) the start of one
+	if (last && threadIdx.x < (nb + 31) / 32)
+		last_par[(uint64_t) blockIdx.x * nb / 32 + threadIdx.x] = s_any[threadIdx.x];
+}
+static_assert(SM_DEPTH <= 7, "two words of last_par bits per CTA");
+
+template <typename T>
+void sub_min_launch(const TreeStorage &t, cudaStream_t s)
+{
+	// from the bottom up; a run ends at level 6, whose one block is level 6's
+	for (uint32_t e = t.levels - 2; e >= 6;) {
+		const uint32_t depth = std::min<uint32_t>(SM_DEPTH, e - 5);
+		const uint64_t ctas = ((1ull << e) / 64) >> (depth - 1);
+		k_sub_min<T><<<(unsigned) ctas, SM_THREADS, 0, s>>>(static_cast<const T *>(t.dim2), t.occ,
+		                                                    static_cast<T *>(t.sub_min), t.last_par, t.levels, e, depth);
+		PST_CUDA(cudaGetLastError());
+		e -= depth;
 	}
 }
 
@@ -1332,29 +1368,11 @@ void finish_tree_aux(TreeStorage &t, cudaStream_t s)
 	t.aux = pool_alloc(par_bytes + ((1ull << (t.levels - 1)) / 64) * vs, "search index");
 	t.last_par = static_cast<uint32_t *>(t.aux);
 	t.sub_min = static_cast<char *>(t.aux) + par_bytes;
-	const unsigned g = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((nb + 255) / 256, 65535));
-	k_last_par<<<g, 256, 0, s>>>(t.occ, L, t.last_par);
-	PST_CUDA(cudaGetLastError());
-	// sub_min: one value per 64-slot block of positions [64, 2^(D-1)), levels
-	// 6..D-2, built from the bottom up
-	for (uint32_t lv = t.levels - 2; lv >= 6; lv--) {
-		const uint64_t warps = (1ull << lv) / 64;
-		const unsigned gb = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((warps * 32 + 255) / 256, 1u << 20));
-		switch (t.dtype) {
-		case PST_F32:
-			k_sub_min<float><<<gb, 256, 0, s>>>(static_cast<const float *>(t.dim2), t.occ,
-			                                    static_cast<float *>(t.sub_min), t.levels, lv);
-			break;
-		case PST_F64:
-			k_sub_min<double><<<gb, 256, 0, s>>>(static_cast<const double *>(t.dim2), t.occ,
-			                                     static_cast<double *>(t.sub_min), t.levels, lv);
-			break;
-		case PST_I32:
-			k_sub_min<int32_t><<<gb, 256, 0, s>>>(static_cast<const int32_t *>(t.dim2), t.occ,
-			                                      static_cast<int32_t *>(t.sub_min), t.levels, lv);
-			break;
-		}
-		PST_CUDA(cudaGetLastError());
+	// sub_min: one value per 64-slot block of positions [64, 2^(D-1)), levels 6..D-2
+	switch (t.dtype) {
+	case PST_F32: sub_min_launch<float>(t, s); break;
+	case PST_F64: sub_min_launch<double>(t, s); break;
+	case PST_I32: sub_min_launch<int32_t>(t, s); break;
 	}
 }
 

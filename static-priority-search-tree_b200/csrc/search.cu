@@ -806,14 +806,18 @@ __device__ __forceinline__ void emit_blocks(const TreeDev<T> &t, const uint4 &mi
 // the reading needless (level_body asks for that first, to spare the loads: two round
 // trips a level); reservations are single shared-memory atomics, counts are sums of
 // one; and every thread keeps the level's bounds itself, so that one barrier ends a level.
-// One query on 64.5 k points (16 levels): 30 us with the per-level kernels' body between
-// two barriers a level, TOPUS us.  A few host queries and the arguments come as the kernel's
+// One query on 64.5 k points (16 levels, 6.5 k ids): 30 us with the per-level kernels' body
+// between two barriers a level and 7 for the emit, 21 us with its results written; the
+// call 88 -> 41 us.  A few host queries and the arguments come as the kernel's
 // parameters (reading them from mapped host memory takes 3.7 us), and the control block goes
 // back to mapped host memory: a copy each way took 16 us of a call.
 // Where the pass stops, it writes the records, the counts and the next level's paths
 // and seeds to their global buffers, in the layout the per-level kernels and the emit
 // read.  It stops early when the next level might not fit in rcap.
-constexpr uint32_t CTA_REC_CAP = 256;
+// With 256 records instead of 160, 16 isovalues over 2^21 metacells took 108 us, and with
+// 96 one query for 1 % of 2^24 points took 87; with 160 they take 106 and 83.
+constexpr uint32_t CTA_REC_CAP = 160;
+// A single query's 6.5 k ids from a kernel of their own: 69 us a call instead of 45.
 constexpr uint32_t CTA_EMIT_CAP = 16384;
 constexpr int TOP_THREADS = 512, TOP_WARPS = TOP_THREADS / 32;
 
