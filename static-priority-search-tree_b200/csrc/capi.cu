@@ -555,12 +555,13 @@ pst_status pst_batch_last_stats(pst_batch *batch, pst_batch_stats *stats, uint32
 		pst_batch_stats st{};
 		st.levels = batch->b.tree->levels;
 		for (uint32_t d = 0; d < 40; d++) {
-			st.records += c.lvl_cnt[d];
+			st.records += c.lvl_cnt[d] + c.top_cnt[d];
 			st.seeds += c.seed_cnt[d];
+			st.boundary -= c.top_cnt[d];
 			if (per_level)
-				per_level[d] = c.lvl_cnt[d];
+				per_level[d] = c.lvl_cnt[d] + c.top_cnt[d];
 		}
-		st.boundary = c.rec_cnt;
+		st.boundary += c.rec_cnt;
 		st.points = c.total;
 		*stats = st;
 	});

@@ -865,9 +865,10 @@ struct TopPass {
 	// cell d: records of level d - 1, paths and seeds of level d, start of level d's records
 	uint32_t cells;
 	uint32_t flags, rec_cnt;
-	uint32_t cnt, cur;  // a word per query
+	uint32_t cnt, cur;  // a word per query, from query q0 on
+	uint32_t q0;
 	uint32_t lists, rec;
-	uint4 *ro;          // (global)
+	uint4 *ro;          // reported boundary nodes
 	uint32_t pcap, ro_cap;
 
 	__device__ __forceinline__ uint32_t cell(uint32_t d) const { return cells + 16 * d; }
@@ -920,7 +921,7 @@ __device__ __forceinline__ void top_paths(const TreeDev<T> &t, const TopPass<T> 
 			p.ro[b_rep] = block_record(h & ~31u, q, 1u << (h & 31));
 		else
 			lost = true;
-		sh_add(p.cnt + 4 * q, 1);
+		sh_add(p.cnt + 4 * (q - p.q0), 1);
 	}
 	if (lost)
 		sh_or(p.flags, BATCH_FLAG_INTERNAL);
@@ -943,7 +944,7 @@ __device__ __forceinline__ void top_seeds(const TreeDev<T> &t, const TopPass<T> 
 	    (((cand >> b) & 1u) && m2 <= v0 ? 1u << b : 0u) | (((cand >> (b + 1)) & 1u) && m2 <= v1 ? 2u << b : 0u);
 	if (am) {
 		sh_st4(p.rec + 16 * (base_cur + sh_add(p.cell(d + 1), 1)), block_record(sd.x, sd.y, am));
-		sh_add(p.cnt + 4 * sd.y, (uint32_t) __popc(am));
+		sh_add(p.cnt + 4 * (sd.y - p.q0), (uint32_t) __popc(am));
 	}
 }
 
@@ -1011,7 +1012,24 @@ __device__ __forceinline__ void top_records(const TreeDev<T> &t, const TopPass<T
 	if (mine.z | mine.w)
 		sh_st4(p.rec + 16 * (base_cur + sh_add(p.cell(d + 1), 1)), mine);
 	if (pts)
-		sh_add(p.cnt + 4 * ptsq, pts);
+		sh_add(p.cnt + 4 * (ptsq - p.q0), pts);
+}
+
+// Level d of the pass, shared out over the CTA's warps: np paths, ns seeds, and the records
+// [base_prev, base_cur) of the level above.
+template <typename T>
+__device__ __forceinline__ void top_level(const TreeDev<T> &t, const TopPass<T> &p, uint32_t d, uint32_t np, uint32_t ns,
+                                          uint32_t base_prev, uint32_t base_cur)
+{
+	const uint32_t wp = (np + 31) / 32, ws = (ns + 31) / 32, wr = (base_cur - base_prev + TOP_U - 1) / TOP_U;
+	for (uint32_t i = threadIdx.x >> 5; i < wp + ws + wr; i += TOP_WARPS) {
+		if (i < wp)
+			top_paths<T>(t, p, d, 32 * i, np);
+		else if (i < wp + ws)
+			top_seeds<T>(t, p, d, 32 * (i - wp), ns, base_cur);
+		else
+			top_records<T>(t, p, d, base_prev + TOP_U * (i - wp - ws), base_cur, base_cur);
+	}
 }
 
 // Writes the slots of the blocks at[0 .. n) that their masks name, each from output place
@@ -1084,6 +1102,7 @@ __global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T
 	p.rec_cnt = addr(&s_word[1]);
 	p.cnt = addr(s_cnt);
 	p.cur = addr(s_cur);
+	p.q0 = 0;
 	p.lists = addr(s_list);
 	p.rec = addr(s_rec);
 	p.pcap = pcap;
@@ -1123,15 +1142,7 @@ __global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T
 		}
 		if (threadIdx.x == 0)
 			sh_st(p.cell(d) + 12, base_cur);
-		const uint32_t wp = (np + 31) / 32, ws = (ns + 31) / 32, wr = (prev + TOP_U - 1) / TOP_U;
-		for (uint32_t i = warp; i < wp + ws + wr; i += TOP_WARPS) {
-			if (i < wp)
-				top_paths<T>(t, p, d, 32 * i, np);
-			else if (i < wp + ws)
-				top_seeds<T>(t, p, d, 32 * (i - wp), ns, base_cur);
-			else
-				top_records<T>(t, p, d, base_prev + TOP_U * (i - wp - ws), base_cur, base_cur);
-		}
+		top_level<T>(t, p, d, np, ns, base_prev, base_cur);
 		__syncthreads();  // the level's records, paths, seeds and counts are visible to the CTA
 	}
 	// records written: at the bottom the last level's follow base_cur (none, where the pass
@@ -1223,26 +1234,173 @@ __global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T
 	}
 }
 
-// Shared memory the one-CTA top pass may take beyond its static arrays on the
-// current device, after allowing it for the kernel there (once per device; done
-// before any launch is captured into a graph).
+// The first `stop` levels of a whole pass, in place of as many level kernels: a CTA per
+// group of g queries, which walks them as k_bfs_cta does and waits for no other CTA.  What
+// it leaves: the records of the last level it took, in that level's region, and the paths
+// and seeds of the next, for the level kernels; the records above, which nobody expands
+// again, with the reported boundary nodes.  (After the control block's load; it unpacks
+// the queries and zeroes the counts and cursors too.)
+//
+// A narrow level is a launch and one warp's chain of loads, 5 to 6 us whatever its size; in
+// here it takes 1.1 to 1.5 us.  How far that reaches is a bound on the records (top_levels
+// below), not a look at the queries: the pass is queued without waiting.
 template <typename T>
-size_t cta_pass_budget()
+__global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_groups(TreeDev<T> t, QDev<T> qd, WorkDev wg, const pst_query *raw,
+                                                               QOut<T> qo, uint32_t max_q, uint32_t g, uint32_t rocap,
+                                                               uint32_t rcap, uint32_t stop)
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	extern __shared__ __align__(16) unsigned char s_dyn[];
+	__shared__ uint32_t s_word[2];  // flags, reported boundary nodes
+	__shared__ uint32_t s_at[4];    // places taken in the global lists
+	uint4 *s_cell = reinterpret_cast<uint4 *>(s_dyn);
+	uint4 *s_list = s_cell + TOP_CELLS, *s_ro = s_list + 8 * g, *s_rec = s_ro + rocap;
+	uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_rec + rcap);
+	const uint32_t q0 = blockIdx.x * g, nq = wg.ctl->nq;
+	const uint32_t mine = nq > q0 ? min(nq - q0, g) : 0u;
+	TopPass<T> p;
+	p.qd = qd;
+	auto addr = [](const void *x) { return static_cast<uint32_t>(__cvta_generic_to_shared(x)); };
+	p.cells = addr(s_cell);
+	p.flags = addr(&s_word[0]);
+	p.rec_cnt = addr(&s_word[1]);
+	p.cnt = addr(s_cnt);
+	p.cur = 0;
+	p.q0 = q0;
+	p.lists = addr(s_list);
+	p.rec = addr(s_rec);
+	p.pcap = 2 * g;
+	p.ro = s_ro;
+	p.ro_cap = rocap;
+	if (threadIdx.x < 2)
+		s_word[threadIdx.x] = 0;
+	for (uint32_t i = threadIdx.x; i < TOP_CELLS; i += TOP_THREADS)
+		s_cell[i] = make_uint4(0, i ? 0u : mine, 0, 0);
+	for (uint32_t i = threadIdx.x; i < g; i += TOP_THREADS)
+		s_cnt[i] = 0;
+	__syncthreads();
+	for (uint32_t i = threadIdx.x; i < mine; i += TOP_THREADS)
+		s_list[i] = unpack_query<T>(raw[q0 + i], q0 + i, qo, &s_word[0]);
+	__syncthreads();
+	uint32_t base_prev = 0, base_cur = 0;
+	for (uint32_t d = 0; d < stop; d++) {
+		const uint4 c = sh_ld4(p.cell(d));
+		const uint32_t np = min(c.y, p.pcap), ns = min(c.z, p.pcap);
+		base_prev = base_cur;
+		base_cur += c.x;
+		// (the records of the levels taken fit, by the bound that chose `stop`)
+		if (base_cur + 2 * c.x + ns > rcap) {
+			if (threadIdx.x == 0)
+				sh_or(p.flags, BATCH_FLAG_INTERNAL);
+			break;
+		}
+		if (c.x + np + ns == 0)
+			continue;
+		top_level<T>(t, p, d, np, ns, base_prev, base_cur);
+		__syncthreads();
+	}
+	__syncthreads();
+	const uint32_t flags = s_word[0];
+	const uint32_t open = flags & BATCH_FLAG_INTERNAL ? 0u : s_cell[stop].x, nro = min(s_word[1], rocap);
+	const uint32_t np = min(s_cell[stop].y, p.pcap), ns = min(s_cell[stop].z, p.pcap);
+	if (threadIdx.x < 4) {
+		const uint32_t n = threadIdx.x == 0 ? open : threadIdx.x == 1 ? base_cur + nro : threadIdx.x == 2 ? np : ns;
+		uint32_t *c = threadIdx.x == 0   ? &wg.ctl->lvl_cnt[stop - 1]
+		              : threadIdx.x == 1 ? &wg.ctl->rec_cnt
+		              : threadIdx.x == 2 ? &wg.ctl->path_cnt[stop]
+		                                 : &wg.ctl->seed_cnt[stop];
+		s_at[threadIdx.x] = n ? atomicAdd(c, n) : 0u;
+	}
+	if (threadIdx.x >= 64 && threadIdx.x < 64 + stop) {
+		// what the level kernels would have counted
+		const uint32_t d = threadIdx.x - 64;
+		if (d + 1 < stop && s_cell[d + 1].x)
+			atomicAdd(&wg.ctl->top_cnt[d], s_cell[d + 1].x);
+		if (s_cell[d].z)
+			atomicAdd(&wg.ctl->seed_cnt[d], s_cell[d].z);
+	}
+	if (threadIdx.x == 32 && flags)
+		atomicOr(&wg.ctl->flags, flags);
+	for (uint32_t i = threadIdx.x; i < g && q0 + i < max_q; i += TOP_THREADS) {
+		wg.counts[q0 + i] = s_cnt[i];
+		wg.cursor[q0 + i] = 0;
+	}
+	__syncthreads();
+	// (the region of the last level taken starts the frontier: lvl_base is 0 there)
+	const uint64_t b_open = s_at[0];
+	if (b_open + open > wg.rec_cap) {
+		if (threadIdx.x == 0) {
+			atomicMax((unsigned long long *) &wg.ctl->need_tasks, (unsigned long long) (b_open + open));
+			atomicOr(&wg.ctl->flags, BATCH_FLAG_TASK_OVERFLOW);
+		}
+	} else {
+		for (uint32_t i = threadIdx.x; i < open; i += TOP_THREADS)
+			wg.rec[b_open + i] = s_rec[base_cur + i];
+	}
+	const uint32_t b_ro = s_at[1];
+	if (b_ro + base_cur + nro > wg.ro_cap) {
+		if (threadIdx.x == 0)
+			atomicOr(&wg.ctl->flags, BATCH_FLAG_INTERNAL);
+	} else {
+		for (uint32_t i = threadIdx.x; i < base_cur + nro; i += TOP_THREADS)
+			wg.ro[b_ro + i] = i < base_cur ? s_rec[i] : s_ro[i - base_cur];
+	}
+	uint4 *pd = (stop & 1) ? wg.path1 : wg.path0, *sd = (stop & 1) ? wg.seed1 : wg.seed0;
+	for (uint32_t i = threadIdx.x; i < np && s_at[2] + i < wg.path_cap; i += TOP_THREADS)
+		pd[s_at[2] + i] = s_list[(stop & 1) * p.pcap + i];
+	for (uint32_t i = threadIdx.x; i < ns && s_at[3] + i < wg.path_cap; i += TOP_THREADS)
+		sd[s_at[3] + i] = s_list[(2 + (stop & 1)) * p.pcap + i];
+}
+
+// Shared memory a top-pass kernel may take beyond its static arrays on the current device,
+// after allowing it for the kernel there (once per device; done before any launch is
+// captured into a graph).
+template <typename T>
+size_t cta_pass_budget(bool groups = false)
 {
 	static std::mutex mu;
-	static size_t budget[64];
+	static size_t budget[64][2];
 	static bool done[64] = {};
 	const DeviceInfo &di = device_info();
 	std::lock_guard<std::mutex> lk(mu);
 	if (!done[di.device]) {
-		cudaFuncAttributes a{};
-		PST_CUDA(cudaFuncGetAttributes(&a, k_bfs_cta<T>));
-		const size_t b = di.smem_optin > a.sharedSizeBytes + 1024 ? di.smem_optin - a.sharedSizeBytes - 1024 : 0;
-		PST_CUDA(cudaFuncSetAttribute(k_bfs_cta<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b));
-		budget[di.device] = b;
+		auto allow = [&](auto *kernel) {
+			cudaFuncAttributes a{};
+			PST_CUDA(cudaFuncGetAttributes(&a, kernel));
+			const size_t b = di.smem_optin > a.sharedSizeBytes + 1024 ? di.smem_optin - a.sharedSizeBytes - 1024 : 0;
+			PST_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b));
+			return b;
+		};
+		budget[di.device][0] = allow(k_bfs_cta<T>);
+		budget[di.device][1] = allow(k_bfs_groups<T>);
 		done[di.device] = true;
 	}
-	return budget[di.device];
+	return budget[di.device][groups];
+}
+
+// How far k_bfs_groups goes with groups of g queries: the levels on which a CTA's records
+// stay below GROUP_REC_CAP whatever the queries, and within its shared memory.  A query has
+// at most a record per 64-slot block of a level and 14 more (the bound of
+// NOALLOC_MAX_LEVELS).  1024 records are 16 rounds of the CTA's warps, which a level kernel
+// would beat, but only queries for most of the tree come near: 64 queries for 30 % of 2^22
+// points each take 260 us without the groups and 213, 210 and 210 with limits of 512, 1024
+// and 2048; 601 mixed ones on 12.3 M doubles 248, and 214, 213 and 210; 4096 on 2^28 points
+// 2091, and 2069, 2057 and 2070.
+constexpr uint32_t GROUP_REC_CAP = 1024, GROUP_MIN_LEVELS = 6;
+constexpr size_t GROUP_SMEM = size_t(200) << 10;
+// Records of the first s levels of one query, and its boundary nodes.
+constexpr uint32_t group_records(uint32_t s) { return (1u << s) / 32 + 14 * s + 64; }
+constexpr size_t group_smem_bytes(uint32_t g, uint32_t s)
+{
+	return (size_t) (TOP_CELLS + g * (8 + 2 * s + group_records(s))) * sizeof(uint4) + (size_t) g * 4;
+}
+inline uint32_t group_levels(uint32_t levels, uint32_t g)
+{
+	uint32_t s = 0;
+	while (s < levels && s < 20 && (uint64_t) g * ((1u << s) / 64 + 14) <= GROUP_REC_CAP &&
+	       group_smem_bytes(g, s + 1) <= GROUP_SMEM)
+		s++;
+	return s;
 }
 
 // Launches the one-CTA top pass of at most qcap queries: two paths and two seeds for each
@@ -1531,7 +1689,12 @@ void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 	grid = (uint32_t) device_info().sms * blocks_per_sm;
 	const size_t vs = value_size(t->dtype);
 	path_cap = 2 * max_q;
-	ro_cap = 2 * max_q * 32;
+	// groups of queries for the first levels of a whole pass, a CTA each
+	group = (max_q + (uint32_t) device_info().sms - 1) / (uint32_t) device_info().sms;
+	group_stop = group_levels(t->levels, group);
+	if (group_stop < GROUP_MIN_LEVELS || max_q <= top_q)
+		group_stop = 0;
+	ro_cap = max_q * (2 * 32 + (group_stop ? group_records(group_stop) : 0));
 	{
 		// laid out twice: once for the size, once for the addresses
 		size_t off = 0;
@@ -1604,10 +1767,20 @@ void Batch::enqueue_count(cudaStream_t s)
 	QDev<T> qd{kind, static_cast<const T *>(min1), static_cast<const T *>(max1), static_cast<const T *>(min2)};
 	PST_WORKDEV;
 	k_load_ctl<<<1, 256, 0, s>>>(ctl_host_d, ctl);
-	const unsigned ug = (unsigned) std::min<uint64_t>((max_q + 255) / 256, (uint64_t) device_info().sms * 4);
 	const QOut<T> qo{kind, static_cast<T *>(min1), static_cast<T *>(max1), static_cast<T *>(min2)};
-	k_prepare_queries<T><<<ug, 256, 0, s>>>(q_raw, ctl, qo, path0, counts, cursor, max_q);
-	for (uint32_t d = 0; d < tv.levels; d++)
+	if (group_stop) {
+		const uint32_t rocap = 2 * group_stop * group, rcap = group * group_records(group_stop);
+		DependentLaunch l((max_q + group - 1) / group, TOP_THREADS, s);
+		l.cfg.dynamicSmemBytes = group_smem_bytes(group, group_stop);
+		if (l.cfg.dynamicSmemBytes > cta_pass_budget<T>(true))
+			fail(PST_ERR_INTERNAL, "shared memory too small for groups of " + std::to_string(group) + " queries");
+		PST_CUDA(cudaLaunchKernelEx(&l.cfg, k_bfs_groups<T>, tv, qd, w, (const pst_query *) q_raw, qo, max_q, group, rocap,
+		                            rcap, group_stop));
+	} else {
+		const unsigned ug = (unsigned) std::min<uint64_t>((max_q + 255) / 256, (uint64_t) device_info().sms * 4);
+		k_prepare_queries<T><<<ug, 256, 0, s>>>(q_raw, ctl, qo, path0, counts, cursor, max_q);
+	}
+	for (uint32_t d = group_stop; d < tv.levels; d++)
 		launch_level<T>(tv, qd, w, d, grid, threads, s);
 	scan_offsets(counts, offsets, max_q, scan_tmp, ctl, s);
 	PST_CUDA(cudaGetLastError());

@@ -39,6 +39,7 @@ struct BatchCtl {
 	uint64_t lvl_base[40];
 	uint32_t emitted;       // the top pass wrote the results itself
 	uint32_t unused[3];
+	uint32_t top_cnt[40];   // records per level that k_bfs_groups put with the boundary nodes
 };
 
 // What the top pass of a small batch works on (kernel parameters).
@@ -91,6 +92,7 @@ struct Batch {
 	uint32_t path_cap = 0;
 	uint4 *ro = nullptr;        // reported boundary nodes, as one-bit records
 	uint32_t ro_cap = 0;
+	uint32_t group = 0, group_stop = 0;  // queries a CTA of k_bfs_groups takes, and its levels (0: not used)
 	uint64_t *counts = nullptr, *cursor = nullptr, *offsets = nullptr, *scan_tmp = nullptr;
 	BatchCtl *ctl = nullptr;
 	// One mapped pinned block: the control block a whole pass starts from (zeroed except
