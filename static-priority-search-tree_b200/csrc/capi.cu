@@ -184,7 +184,7 @@ static uint64_t run_single(pst_tree *tr, const pst_query *q, pst_ret ret, void *
 	uint64_t total = 0;
 	if (!alloc) {
 		// counted and written in one go, where the results fit
-		const EmitTo to{ret, *out_d, capacity, nullptr};
+		const EmitTo to{ret, *out_d, capacity};
 		b.count_sync(s, &total, *out_d ? &to : nullptr);
 		if (total && total <= capacity && b.last_status() != PST_OK)
 			fail(b.last_status(), "search emit failed");
@@ -195,8 +195,7 @@ static uint64_t run_single(pst_tree *tr, const pst_query *q, pst_ret ret, void *
 		return 0;
 	malloc_result(out_d, total * b.record_size(ret), s);
 	b.enqueue_emit(ret, *out_d, total, s);
-	uint64_t t2 = 0;
-	const pst_status st = b.read_ctl(s, &t2);
+	const pst_status st = b.finish(s);
 	if (st != PST_OK) {
 		cudaFreeAsync(*out_d, s);  // after whatever the stream still holds
 		*out_d = nullptr;
@@ -490,10 +489,10 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 			fail(PST_ERR_INVALID, "bad return type");
 		if (ret == PST_RET_IDS && b.tree->idtype != PST_ID_U32)
 			fail(PST_ERR_UNSUPPORTED, "an id-less tree can only return points");
-		b.stage_queries(queries, nq, queries_on_device != 0, s, !sync);
+		b.stage_queries(queries, nq, queries_on_device != 0, s, offsets_d);
 		uint64_t tot = 0;
 		if (sync) {
-			const EmitTo to{ret, out_d, out_capacity, offsets_d};
+			const EmitTo to{ret, out_d, out_capacity};
 			b.count_sync(s, &tot, &to);
 			if (total)
 				*total = tot;
@@ -501,9 +500,6 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 		} else {
 			b.launch_count(s);
 			b.enqueue_emit(ret, out_d, out_capacity, s);
-			if (offsets_d)
-				check_cuda(cudaMemcpyAsync(offsets_d, b.offsets, ((size_t) nq + 1) * 8, cudaMemcpyDeviceToDevice, s),
-				           "copy offsets");
 			if (total)
 				check_cuda(cudaMemcpyAsync(total, &b.ctl->total, 8, cudaMemcpyDeviceToHost, s), "copy total");
 			b.mark_async(s);

@@ -607,10 +607,11 @@ __global__ void k_load_ctl(const BatchCtl *src, BatchCtl *dst)
 // unpacked and checked, their level-0 paths, and the per-query counts and output
 // cursors zeroed (all max_q of them: the scan reads every count).
 template <typename T>
-__global__ void k_prepare_queries(const pst_query *raw, BatchCtl *ctl, QOut<T> qo, uint4 *path0, uint64_t *counts,
-                                  uint64_t *cursor, uint32_t max_q)
+__global__ void k_prepare_queries(BatchCtl *ctl, QOut<T> qo, uint4 *path0, uint64_t *counts, uint64_t *cursor,
+                                  uint32_t max_q)
 {
 	const uint32_t nq = ctl->nq;
+	const pst_query *raw = ctl->raw;
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < max_q; i += gridDim.x * blockDim.x) {
 		if (i < nq)
 			path0[i] = unpack_query<T>(raw[i], i, qo, &ctl->flags);
@@ -645,6 +646,8 @@ __device__ __forceinline__ void guard_claim(const WorkDev &w, uint4 &rec, uint64
 {
 	if (out_base + __popc(rec.z) + __popc(rec.w) > capacity) {
 		atomicOr(&w.ctl->flags, BATCH_FLAG_INTERNAL);
+		if (uint32_t *host = w.ctl->host_fault)
+			*host = 1;
 		rec.z = rec.w = 0;
 	}
 }
@@ -1184,6 +1187,9 @@ __global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T
 		sc->need_tasks = over ? nrec : 0;
 		sc->total = total;
 		sc->emitted = emit;
+		sc->user_offsets = in.args.offsets;  // for a scan that follows
+		sc->host_fault = back ? &back->fault : nullptr;
+		sc->emit_follows = in.args.out != nullptr;
 	}
 	uint64_t *offsets = const_cast<uint64_t *>(wg.offsets);
 	if (done) {
@@ -1245,8 +1251,8 @@ __global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T
 // here it takes 1.1 to 1.5 us.  How far that reaches is a bound on the records (top_levels
 // below), not a look at the queries: the pass is queued without waiting.
 template <typename T>
-__global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_groups(TreeDev<T> t, QDev<T> qd, WorkDev wg, const pst_query *raw,
-                                                               QOut<T> qo, uint32_t max_q, uint32_t g, uint32_t rocap,
+__global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_groups(TreeDev<T> t, QDev<T> qd, WorkDev wg, QOut<T> qo,
+                                                               uint32_t max_q, uint32_t g, uint32_t rocap,
                                                                uint32_t rcap, uint32_t stop)
 {
 	asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -1257,6 +1263,7 @@ __global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_groups(TreeDev<T> t, QDe
 	uint4 *s_list = s_cell + TOP_CELLS, *s_ro = s_list + 8 * g, *s_rec = s_ro + rocap;
 	uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_rec + rcap);
 	const uint32_t q0 = blockIdx.x * g, nq = wg.ctl->nq;
+	const pst_query *raw = wg.ctl->raw;
 	const uint32_t mine = nq > q0 ? min(nq - q0, g) : 0u;
 	TopPass<T> p;
 	p.qd = qd;
@@ -1420,15 +1427,26 @@ void launch_cta_pass(const TreeDev<T> &tv, const QDev<T> &qd, const WorkDev &w, 
 	    tv, qd, w, max_q, (qcap + 1) & ~1u, pcap, rcap, qo, in, back);
 }
 
+// The host's copy of a finished pass's control block (by the whole CTA; `back` may be null).
+__device__ __forceinline__ void ctl_to_host(const BatchCtl *ctl, BatchCtl *back)
+{
+	if (back)
+		for (uint32_t i = threadIdx.x; i < sizeof(BatchCtl) / 4; i += blockDim.x)
+			reinterpret_cast<uint32_t *>(back)[i] = reinterpret_cast<const uint32_t *>(ctl)[i];
+}
+
 // THREADS: the CTA size and U the records each warp has in flight (both tuning
 // choices; point records keep U = 4).
 template <typename T, bool HAS_ID, bool POINTS, int THREADS, int U>
-__global__ void __launch_bounds__(THREADS) k_emit(TreeDev<T> t, WorkDev w, void *out, uint64_t capacity)
+__global__ void __launch_bounds__(THREADS) k_emit(TreeDev<T> t, WorkDev w, void *out, uint64_t capacity,
+                                                 BatchCtl *back)
 {
 	// a programmatic dependent of the scan (a no-op after any other predecessor)
 	asm volatile("griddepcontrol.wait;" ::: "memory");
 	__shared__ uint64_t s_total;
 	__shared__ EmitWarp<Point<T, HAS_ID>, POINTS> s_warp[THREADS / 32];
+	if (blockIdx.x == 0)
+		ctl_to_host(w.ctl, back);
 	if (threadIdx.x == 0) {
 		uint64_t b = 0;
 		for (uint32_t e = 0; e < t.levels; e++)
@@ -1479,14 +1497,18 @@ __global__ void __launch_bounds__(THREADS) k_emit(TreeDev<T> t, WorkDev w, void 
 // Result offsets of a batch in one launch: offsets[q] = the counts of the queries
 // before q, offsets[max_q] = ctl->total = all of them.  One CTA walks the counts a
 // tile at a time (batches of up to OFFSETS_ONE_CTA queries; larger ones take the
-// three-kernel scan).  Launched as a programmatic dependent of the last level.
+// three-kernel scan and k_pass_end).  Launched as a programmatic dependent of the last
+// level.  It also writes the caller's offsets and the host's copy of the control block,
+// which spares a copy of each (2 to 3 us on the device).
 constexpr uint32_t OFFSETS_ONE_CTA = 4 * SCAN_TILE;
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_offsets(const uint64_t *counts, uint64_t *offsets, uint32_t n,
-                                                          BatchCtl *ctl)
+                                                          BatchCtl *ctl, BatchCtl *back)
 {
 	asm volatile("griddepcontrol.wait;" ::: "memory");
 	__shared__ uint64_t ws[33];
+	const uint32_t nq = ctl->nq;
+	uint64_t *user = ctl->user_offsets;
 	uint64_t carry = 0;
 	for (uint32_t c0 = 0; c0 < n; c0 += SCAN_TILE) {
 		const uint32_t base = c0 + threadIdx.x * SCAN_ITEMS;
@@ -1503,14 +1525,31 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_offsets(const uint64_t *counts
 		for (int i = 0; i < SCAN_ITEMS; i++) {
 			if (base + i < n)
 				offsets[base + i] = ex;
+			if (user && base + i < n && base + i <= nq)
+				user[base + i] = ex;
 			ex += v[i];
 		}
 		carry += tot;
 	}
 	if (threadIdx.x == 0) {
 		offsets[n] = carry;
+		if (user && nq == n)
+			user[n] = carry;
 		ctl->total = carry;
 	}
+	__syncthreads();
+	if (!ctl->emit_follows)
+		ctl_to_host(ctl, back);
+}
+
+// The end of a pass of more queries, after its scan.
+__global__ void __launch_bounds__(SCAN_THREADS) k_pass_end(const uint64_t *offsets, const BatchCtl *ctl, BatchCtl *back)
+{
+	if (ctl->user_offsets)
+		for (uint64_t q = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; q <= ctl->nq; q += (uint64_t) gridDim.x * blockDim.x)
+			ctl->user_offsets[q] = offsets[q];
+	if (blockIdx.x == 0 && !ctl->emit_follows)
+		ctl_to_host(ctl, back);
 }
 
 // Launch configuration of a programmatic dependent of the kernel before it on `s`:
@@ -1534,15 +1573,17 @@ struct DependentLaunch {
 
 // The batch's result offsets and total (exclusive scan of its counts).
 inline void scan_offsets(uint64_t *counts, uint64_t *offsets, uint32_t max_q, uint64_t *scan_tmp, BatchCtl *ctl,
-                         cudaStream_t s)
+                         BatchCtl *back, cudaStream_t s)
 {
 	if (max_q <= OFFSETS_ONE_CTA) {
 		DependentLaunch l(1, SCAN_THREADS, s);
-		PST_CUDA(cudaLaunchKernelEx(&l.cfg, k_offsets, (const uint64_t *) counts, offsets, max_q, ctl));
+		PST_CUDA(cudaLaunchKernelEx(&l.cfg, k_offsets, (const uint64_t *) counts, offsets, max_q, ctl, back));
 		return;
 	}
 	exclusive_scan<uint64_t>(counts, offsets, max_q, scan_tmp, &ctl->total, s);
 	PST_CUDA(cudaMemcpyAsync(offsets + max_q, &ctl->total, 8, cudaMemcpyDeviceToDevice, s));
+	k_pass_end<<<32, SCAN_THREADS, 0, s>>>(offsets, ctl, back);
+	PST_CUDA(cudaGetLastError());
 }
 
 // Grid of k_emit: as many CTAs as fit on the device at once (its own occupancy,
@@ -1598,35 +1639,36 @@ const void *bfs_kernel_ptr(unsigned threads)
 
 // Launches the emit with the batch's CTA size and records in flight.
 template <typename T, bool HAS_ID, bool POINTS, int THREADS, int U>
-void launch_emit_tu(const TreeDev<T> &tv, const WorkDev &w, void *out, uint64_t capacity, cudaStream_t s)
+void launch_emit_tu(const TreeDev<T> &tv, const WorkDev &w, void *out, uint64_t capacity, BatchCtl *back, cudaStream_t s)
 {
 	DependentLaunch l(emit_grid<T, HAS_ID, POINTS, THREADS, U>(), THREADS, s);
-	PST_CUDA(cudaLaunchKernelEx(&l.cfg, k_emit<T, HAS_ID, POINTS, THREADS, U>, tv, w, out, capacity));
+	PST_CUDA(cudaLaunchKernelEx(&l.cfg, k_emit<T, HAS_ID, POINTS, THREADS, U>, tv, w, out, capacity, back));
 }
 
 template <typename T, bool HAS_ID, bool POINTS, int THREADS>
-void launch_emit_t(const TreeDev<T> &tv, const WorkDev &w, void *out, uint64_t capacity, uint32_t u, cudaStream_t s)
+void launch_emit_t(const TreeDev<T> &tv, const WorkDev &w, void *out, uint64_t capacity, uint32_t u, BatchCtl *back,
+                   cudaStream_t s)
 {
 	if constexpr (POINTS) {
 		(void) u;
-		launch_emit_tu<T, HAS_ID, POINTS, THREADS, 4>(tv, w, out, capacity, s);
+		launch_emit_tu<T, HAS_ID, POINTS, THREADS, 4>(tv, w, out, capacity, back, s);
 	} else if (u == 4) {
-		launch_emit_tu<T, HAS_ID, POINTS, THREADS, 4>(tv, w, out, capacity, s);
+		launch_emit_tu<T, HAS_ID, POINTS, THREADS, 4>(tv, w, out, capacity, back, s);
 	} else if (u == 16) {
-		launch_emit_tu<T, HAS_ID, POINTS, THREADS, 16>(tv, w, out, capacity, s);
+		launch_emit_tu<T, HAS_ID, POINTS, THREADS, 16>(tv, w, out, capacity, back, s);
 	} else {
-		launch_emit_tu<T, HAS_ID, POINTS, THREADS, 8>(tv, w, out, capacity, s);
+		launch_emit_tu<T, HAS_ID, POINTS, THREADS, 8>(tv, w, out, capacity, back, s);
 	}
 }
 
 template <typename T, bool HAS_ID, bool POINTS>
 void launch_emit(const TreeDev<T> &tv, const WorkDev &w, void *out, uint64_t capacity, uint32_t threads, uint32_t u,
-                 cudaStream_t s)
+                 BatchCtl *back, cudaStream_t s)
 {
 	switch (threads) {
-	case 128: launch_emit_t<T, HAS_ID, POINTS, 128>(tv, w, out, capacity, u, s); break;
-	case 512: launch_emit_t<T, HAS_ID, POINTS, 512>(tv, w, out, capacity, u, s); break;
-	default: launch_emit_t<T, HAS_ID, POINTS, BFS_THREADS>(tv, w, out, capacity, u, s);
+	case 128: launch_emit_t<T, HAS_ID, POINTS, 128>(tv, w, out, capacity, u, back, s); break;
+	case 512: launch_emit_t<T, HAS_ID, POINTS, 512>(tv, w, out, capacity, u, back, s); break;
+	default: launch_emit_t<T, HAS_ID, POINTS, BFS_THREADS>(tv, w, out, capacity, u, back, s);
 	}
 }
 
@@ -1653,7 +1695,6 @@ void Batch::release()
 	pool_release(rec, device);
 	work = nullptr;
 	pinned_release(ctl_host, device);  // the staged queries lie behind the control block
-	q_raw = nullptr;
 	ctl_host = nullptr;
 	ctl_host_d = nullptr;
 	q_stage = nullptr;
@@ -1705,7 +1746,6 @@ void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 		};
 		auto layout = [&] {
 			off = 0;
-			take(&q_raw, (size_t) max_q * sizeof(pst_query));
 			take(&kind, (size_t) max_q * 4);
 			take(&min1, (size_t) max_q * vs);
 			take(&max1, (size_t) max_q * vs);
@@ -1774,15 +1814,14 @@ void Batch::enqueue_count(cudaStream_t s)
 		l.cfg.dynamicSmemBytes = group_smem_bytes(group, group_stop);
 		if (l.cfg.dynamicSmemBytes > cta_pass_budget<T>(true))
 			fail(PST_ERR_INTERNAL, "shared memory too small for groups of " + std::to_string(group) + " queries");
-		PST_CUDA(cudaLaunchKernelEx(&l.cfg, k_bfs_groups<T>, tv, qd, w, (const pst_query *) q_raw, qo, max_q, group, rocap,
-		                            rcap, group_stop));
+		PST_CUDA(cudaLaunchKernelEx(&l.cfg, k_bfs_groups<T>, tv, qd, w, qo, max_q, group, rocap, rcap, group_stop));
 	} else {
 		const unsigned ug = (unsigned) std::min<uint64_t>((max_q + 255) / 256, (uint64_t) device_info().sms * 4);
-		k_prepare_queries<T><<<ug, 256, 0, s>>>(q_raw, ctl, qo, path0, counts, cursor, max_q);
+		k_prepare_queries<T><<<ug, 256, 0, s>>>(ctl, qo, path0, counts, cursor, max_q);
 	}
 	for (uint32_t d = group_stop; d < tv.levels; d++)
 		launch_level<T>(tv, qd, w, d, grid, threads, s);
-	scan_offsets(counts, offsets, max_q, scan_tmp, ctl, s);
+	scan_offsets(counts, offsets, max_q, scan_tmp, ctl, back_d, s);
 	PST_CUDA(cudaGetLastError());
 }
 
@@ -1806,31 +1845,31 @@ void Batch::enqueue_count_rest(uint32_t from, cudaStream_t s)
 	PST_WORKDEV;
 	for (uint32_t d = from; d < tv.levels; d++)
 		launch_level<T>(tv, qd, w, d, grid, threads, s);
-	scan_offsets(counts, offsets, max_q, scan_tmp, ctl, s);
+	scan_offsets(counts, offsets, max_q, scan_tmp, ctl, back_d, s);
 	PST_CUDA(cudaGetLastError());
 }
 
 template <typename T, bool HAS_ID, bool POINTS>
-void Batch::enqueue_emit_t(void *out, uint64_t capacity, cudaStream_t s)
+void Batch::enqueue_emit_t(void *out, uint64_t capacity, cudaStream_t s, bool to_host)
 {
 	TreeDev<T> tv = tree->view<T>();
 	PST_WORKDEV;
-	launch_emit<T, HAS_ID, POINTS>(tv, w, out, capacity, threads, emit_u, s);
+	launch_emit<T, HAS_ID, POINTS>(tv, w, out, capacity, threads, emit_u, to_host ? back_d : nullptr, s);
 	PST_CUDA(cudaGetLastError());
 }
 
 template <typename T>
-void Batch::enqueue_emit_v(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s)
+void Batch::enqueue_emit_v(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s, bool to_host)
 {
 	const bool has_id = tree->idtype == PST_ID_U32;
 	if (ret == PST_RET_IDS) {
 		if (!has_id)
 			fail(PST_ERR_UNSUPPORTED, "an id-less tree can only return points");
-		enqueue_emit_t<T, true, false>(out, capacity, s);
+		enqueue_emit_t<T, true, false>(out, capacity, s, to_host);
 	} else if (has_id) {
-		enqueue_emit_t<T, true, true>(out, capacity, s);
+		enqueue_emit_t<T, true, true>(out, capacity, s, to_host);
 	} else {
-		enqueue_emit_t<T, false, true>(out, capacity, s);
+		enqueue_emit_t<T, false, true>(out, capacity, s, to_host);
 	}
 }
 
@@ -1852,12 +1891,12 @@ void Batch::enqueue_counting_top(cudaStream_t s)
 	}
 }
 
-void Batch::enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s)
+void Batch::enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s, bool to_host)
 {
 	switch (tree->dtype) {
-	case PST_F32: enqueue_emit_v<float>(ret, out, capacity, s); break;
-	case PST_F64: enqueue_emit_v<double>(ret, out, capacity, s); break;
-	case PST_I32: enqueue_emit_v<int32_t>(ret, out, capacity, s); break;
+	case PST_F32: enqueue_emit_v<float>(ret, out, capacity, s, to_host); break;
+	case PST_F64: enqueue_emit_v<double>(ret, out, capacity, s, to_host); break;
+	case PST_I32: enqueue_emit_v<int32_t>(ret, out, capacity, s, to_host); break;
 	}
 }
 
@@ -1913,7 +1952,7 @@ void Batch::launch_count_rest(uint32_t from, cudaStream_t s)
 	}
 }
 
-void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, bool whole)
+void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, uint64_t *to_offsets)
 {
 	if (nq > max_q)
 		fail(PST_ERR_INVALID, "batch of " + std::to_string(nq) + " queries exceeds max_queries " +
@@ -1924,29 +1963,22 @@ void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaS
 	if (!idle)
 		PST_CUDA(cudaStreamSynchronize(s));
 	idle = false;
-	ctl_host->nq = nq;
-	top_in.args = TopArgs{};
-	top_in.args.nq = nq;
-	if (!whole && nq <= TOP_IN_QUERIES && !on_device) {
-		std::copy(q, q + nq, top_in.q);
-		return;
-	}
+	// the kernels read the queries where they are, the staged ones through their mapping
 	if (!on_device && nq)
 		memcpy(q_stage, q, (size_t) nq * sizeof(pst_query));
-	if (!whole && nq <= top_q) {
-		top_in.args.raw = on_device ? q : q_stage_d;  // the top pass reads them where they are
-	} else if (nq) {
-		PST_CUDA(cudaMemcpyAsync(q_raw, on_device ? q : q_stage, (size_t) nq * sizeof(pst_query),
-		                         on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
-	}
-}
-
-// The device's control block into `last`, once the work on `s` is done.
-void Batch::fetch_ctl(cudaStream_t s)
-{
-	PST_CUDA(cudaMemcpyAsync(back, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
-	PST_CUDA(cudaStreamSynchronize(s));
-	last = *back;
+	ctl_host->nq = nq;
+	ctl_host->raw = on_device ? q : q_stage_d;
+	ctl_host->user_offsets = to_offsets;
+	ctl_host->host_fault = &back_d->fault;
+	ctl_host->emit_follows = 0;
+	back->fault = 0;
+	top_in.args = TopArgs{};
+	top_in.args.nq = nq;
+	top_in.args.offsets = to_offsets;
+	if (!on_device && nq <= TOP_IN_QUERIES)
+		std::copy(q, q + nq, top_in.q);
+	else
+		top_in.args.raw = ctl_host->raw;
 }
 
 pst_status Batch::last_status() const
@@ -1962,9 +1994,20 @@ pst_status Batch::last_status() const
 
 pst_status Batch::read_ctl(cudaStream_t s, uint64_t *total)
 {
-	fetch_ctl(s);
+	PST_CUDA(cudaMemcpyAsync(&last, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
+	PST_CUDA(cudaStreamSynchronize(s));
 	if (total)
 		*total = last.total;
+	return last_status();
+}
+
+pst_status Batch::finish(cudaStream_t s)
+{
+	PST_CUDA(cudaStreamSynchronize(s));
+	last = *back;
+	if (last.fault)
+		last.flags |= BATCH_FLAG_INTERNAL;
+	idle = true;
 	return last_status();
 }
 
@@ -1977,8 +2020,8 @@ void Batch::count_sync(cudaStream_t s, uint64_t *total, const EmitTo *to)
 		count_full_sync(s, total, to);
 }
 
-// Reads the control block of a pass (b.last); true when it is complete, false when the
-// frontier overflowed (and has been grown for another attempt).
+// Looks at a finished pass (b.last); true when it is complete, false when the frontier
+// overflowed (and has been grown for another attempt).
 static bool settle(Batch &b, int attempt, cudaStream_t s, uint64_t *total)
 {
 	const BatchCtl &h = b.last;
@@ -1996,25 +2039,18 @@ static bool settle(Batch &b, int attempt, cudaStream_t s, uint64_t *total)
 	return false;
 }
 
-// Queues the emit and the copy of the offsets behind a count pass: the emit writes
-// nothing when the pass did not fit the frontier or its results the buffer.
-void Batch::emit_to(const EmitTo &to, cudaStream_t s)
-{
-	if (to.offsets)
-		PST_CUDA(cudaMemcpyAsync(to.offsets, offsets, ((size_t) ctl_host->nq + 1) * 8, cudaMemcpyDeviceToDevice, s));
-	if (to.out && to.capacity)
-		enqueue_emit(to.ret, to.out, to.capacity, s);
-}
-
-// The whole pass, with automatic growth of the frontier buffer.
+// The whole pass, with automatic growth of the frontier buffer.  An emit queued behind a
+// count pass writes nothing when the pass did not fit the frontier or its results the
+// buffer.
 void Batch::count_full_sync(cudaStream_t s, uint64_t *total, const EmitTo *to)
 {
+	const bool emits = to && to->out && to->capacity;
+	ctl_host->emit_follows = emits;
 	for (int attempt = 0;; attempt++) {
 		launch_count(s);
-		if (to)
-			emit_to(*to, s);
-		fetch_ctl(s);
-		idle = true;
+		if (emits)
+			enqueue_emit(to->ret, to->out, to->capacity, s, true);
+		finish(s);
 		if (settle(*this, attempt, s, total))
 			return;
 	}
@@ -2025,27 +2061,24 @@ void Batch::count_full_sync(cudaStream_t s, uint64_t *total, const EmitTo *to)
 // frontier buffer as in count_full_sync.
 void Batch::count_small_sync(cudaStream_t s, uint64_t *total, const EmitTo *to)
 {
-	if (to) {
-		top_in.args.out = to->capacity ? to->out : nullptr;
+	const bool emits = to && to->out && to->capacity;
+	if (emits) {
+		top_in.args.out = to->out;
 		top_in.args.out_cap = to->capacity;
-		top_in.args.offsets = to->offsets;
 		top_in.args.ret = to->ret;
 	}
 	for (int attempt = 0;; attempt++) {
 		launch_count_top(s);
-		PST_CUDA(cudaStreamSynchronize(s));
-		last = *back;
-		idle = true;
+		finish(s);
 		if (!(last.flags & (BATCH_FLAG_BAD_QUERY | BATCH_FLAG_INTERNAL | BATCH_FLAG_TASK_OVERFLOW))) {
-			if (last.cta_levels < tree->levels) {
+			const bool rest = last.cta_levels < tree->levels;
+			if (rest)
 				launch_count_rest(last.cta_levels, s);
-				if (to)
-					emit_to(*to, s);
-				fetch_ctl(s);
-			} else if (to && to->out && !last.emitted && last.total && last.total <= to->capacity) {
-				enqueue_emit(to->ret, to->out, to->capacity, s);  // the pass wrote the offsets
-				fetch_ctl(s);
-			}
+			const bool emit = emits && (rest || (!last.emitted && last.total && last.total <= to->capacity));
+			if (emit)
+				enqueue_emit(to->ret, to->out, to->capacity, s, true);
+			if (rest || emit)
+				finish(s);
 		}
 		if (settle(*this, attempt, s, total))
 			return;
@@ -2077,7 +2110,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH
 
 // Sub-buffers of the scratch array, 256-byte aligned, in bytes.
 constexpr size_t NA_CTL = 0;
-constexpr size_t NA_KIND = 1024;
+constexpr size_t NA_KIND = 1280;
 constexpr size_t NA_MIN1 = NA_KIND + 256;
 constexpr size_t NA_MAX1 = NA_MIN1 + 256;
 constexpr size_t NA_MIN2 = NA_MAX1 + 256;
@@ -2177,7 +2210,7 @@ uint64_t noalloc_run(TreeStorage &t, const pst_query &q, pst_ret ret, void *out,
 	    h.cta_levels < tv.levels) {
 		for (uint32_t d = h.cta_levels; d < tv.levels; d++)
 			launch_level<T>(tv, qd, w, d, grid, BFS_THREADS, s);
-		scan_offsets(counts, offsets, 1, scan, ctl, s);
+		scan_offsets(counts, offsets, 1, scan, ctl, nullptr, s);
 		PST_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
 		PST_CUDA(cudaStreamSynchronize(s));
 	}
@@ -2189,11 +2222,11 @@ uint64_t noalloc_run(TreeStorage &t, const pst_query &q, pst_ret ret, void *out,
 		return h.total;
 	const bool has_id = t.idtype == PST_ID_U32;
 	if (ret == PST_RET_IDS)
-		launch_emit<T, true, false>(tv, w, out, capacity, BFS_THREADS, 8, s);
+		launch_emit<T, true, false>(tv, w, out, capacity, BFS_THREADS, 8, nullptr, s);
 	else if (has_id)
-		launch_emit<T, true, true>(tv, w, out, capacity, BFS_THREADS, 4, s);
+		launch_emit<T, true, true>(tv, w, out, capacity, BFS_THREADS, 4, nullptr, s);
 	else
-		launch_emit<T, false, true>(tv, w, out, capacity, BFS_THREADS, 4, s);
+		launch_emit<T, false, true>(tv, w, out, capacity, BFS_THREADS, 4, nullptr, s);
 	PST_CUDA(cudaGetLastError());
 	PST_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, s));
 	PST_CUDA(cudaStreamSynchronize(s));

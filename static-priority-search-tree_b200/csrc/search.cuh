@@ -38,8 +38,13 @@ struct BatchCtl {
 	// each instead of summing every count before them
 	uint64_t lvl_base[40];
 	uint32_t emitted;       // the top pass wrote the results itself
-	uint32_t unused[3];
+	uint32_t fault;         // (host copy) the emit's consistency check failed
+	uint32_t unused[2];
 	uint32_t top_cnt[40];   // records per level that k_bfs_groups put with the boundary nodes
+	const pst_query *raw;   // the queries: mapped pinned memory or the caller's device array
+	uint64_t *user_offsets; // the caller's nq + 1 offsets, or null
+	uint32_t *host_fault;   // `fault` of the host's copy, or null
+	uint64_t emit_follows;  // the emit hands the host its copy, while it runs, not the scan
 };
 
 // What the top pass of a small batch works on (kernel parameters).
@@ -64,7 +69,6 @@ struct EmitTo {
 	pst_ret ret;
 	void *out;
 	uint64_t capacity;
-	uint64_t *offsets;      // nq + 1 on the device, or null
 };
 
 struct Batch {
@@ -80,7 +84,6 @@ struct Batch {
 	uint32_t blocks_per_sm = 0;
 	uint32_t grid = 0;
 	// queries
-	pst_query *q_raw = nullptr;
 	pst_query *q_stage = nullptr;  // pinned staging for host query arrays
 	uint32_t *kind = nullptr;
 	void *min1 = nullptr, *max1 = nullptr, *min2 = nullptr;
@@ -119,8 +122,8 @@ struct Batch {
 	void init(TreeStorage *t, const pst_batch_opts &o);
 	void release();
 	void grow_tasks(uint64_t cap, cudaStream_t s);
-	// whole: for a pass that never starts with the top pass.
-	void stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, bool whole = false);
+	// offsets: where the pass also writes the result offsets (nq + 1 on the device, or null).
+	void stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, uint64_t *offsets = nullptr);
 	// Whole count pass (every level kernel and the scan), asynchronous.
 	void launch_count(cudaStream_t s);
 	// Notes that work queued on `s` may still run when the call returns.
@@ -135,16 +138,18 @@ struct Batch {
 	void launch_count_rest(uint32_t from, cudaStream_t s);
 	// Count pass with the host waiting for it: the top pass for small batches, the
 	// whole pass otherwise; grows the frontier buffer until the pass fits.  With `to` the
-	// results (when they fit) and offsets are written too, before the one wait that the
-	// pass ends with; read_ctl's status of the last pass tells how that went.
+	// results (when they fit) are written too, before the one wait that the pass ends with;
+	// last_status tells how that went.
 	void count_sync(cudaStream_t s, uint64_t *total, const EmitTo *to = nullptr);
 	void count_full_sync(cudaStream_t s, uint64_t *total, const EmitTo *to);
 	void count_small_sync(cudaStream_t s, uint64_t *total, const EmitTo *to);
 	void enqueue_counting(cudaStream_t s);
 	void enqueue_counting_top(cudaStream_t s);
-	void enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s);
-	pst_status read_ctl(cudaStream_t s, uint64_t *total);
-	pst_status last_status() const;  // of the control block read last
+	// to_host: the emit also writes the host's copy of the control block.
+	void enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s, bool to_host = false);
+	pst_status read_ctl(cudaStream_t s, uint64_t *total);  // of the device, after whatever ran
+	pst_status finish(cudaStream_t s);  // waits for a waiting call's last kernels
+	pst_status last_status() const;     // of the pass waited for last
 	uint64_t record_size(pst_ret ret) const;
 
   private:
@@ -154,13 +159,11 @@ struct Batch {
 	void enqueue_count_top(cudaStream_t s);
 	template <typename T>
 	void enqueue_count_rest(uint32_t from, cudaStream_t s);
-	void emit_to(const EmitTo &to, cudaStream_t s);
-	void fetch_ctl(cudaStream_t s);
 	void launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStream_t s);
 	template <typename T>
-	void enqueue_emit_v(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s);
+	void enqueue_emit_v(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s, bool to_host);
 	template <typename T, bool HAS_ID, bool POINTS>
-	void enqueue_emit_t(void *out, uint64_t capacity, cudaStream_t s);
+	void enqueue_emit_t(void *out, uint64_t capacity, cudaStream_t s, bool to_host);
 };
 
 // One query into a caller buffer using only the library's static device scratch

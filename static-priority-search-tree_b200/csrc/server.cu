@@ -595,7 +595,7 @@ uint32_t server_add_tree(Server *s, TreeStorage *t, const pst_batch_opts *tuning
 				q.max1.i32 = 0;
 			}
 			uint64_t total = 0;
-			sl->eng.stage_queries(&q, 1, false, sl->stream, true);
+			sl->eng.stage_queries(&q, 1, false, sl->stream);
 			sl->eng.count_full_sync(sl->stream, &total, nullptr);
 			sl->eng.stage_queries(&q, 1, false, sl->stream);
 			sl->eng.count_small_sync(sl->stream, &total, nullptr);

@@ -71,3 +71,37 @@ def test_where_the_pass_stops_writing(pst, oracle, hits, ret):
     out.fill_(0xCD)
     assert tree.search_into(q[0], out, hits - 1, *q[1:], ret=ret) == -hits and (out == 0xCD).all()
     tree.close()
+
+
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("nq,top", [(2, 1), (17, 4), (32, 1), (33, 1), (150, 1), (700, 1)])
+@pytest.mark.parametrize("n", [3, 700, 9001, 150001])
+def test_whole_passes(pst, oracle, dt, nq, top, n):
+    """Batches above the engine's limit for the top pass: the first levels by groups of
+    queries, the rest by level kernels; waiting and asynchronous, again and again (the
+    later passes from a graph), with other queries each time."""
+    import torch
+    pts = rand_points(n, dt, ids="random", dup=n == 700, seed=n + nq)
+    tree = pst.StaticPSTGPU.from_numpy(pts, dt)
+    engine = pst.BatchEngine(tree, max_queries=nq, top_pass_queries=top, task_capacity=256)
+    for k in range(7):
+        qs = rand_queries(pts, nq, seed=nq + k)
+        batch = _batch(pst, qs, dt)
+        off, idx = oracle.Orc.brute_multi(pts, dt, batch["kind"], *[[q[i] for q in qs] for i in (1, 2, 3)])
+        total = int(off[-1])
+        out = torch.zeros(max(total, 1), dtype=torch.int32, device="cuda")
+        offs = torch.empty(nq + 1, dtype=torch.int64, device="cuda")
+        if k % 3 == 2:
+            assert engine.count(batch)[1] == total  # grows the frontier, which an asynchronous pass cannot
+            engine.run(batch, out, offs, sync=False)
+            torch.cuda.synchronize()
+        else:
+            assert engine.run(batch, out, offs) == (0, total)
+            assert engine.last_stats()["points"] == total
+        assert offs.cpu().numpy().astype(np.uint64).tolist() == off.tolist()
+        ids = out.cpu().numpy().view(np.uint32)
+        for i in range(nq):
+            a, b = int(off[i]), int(off[i + 1])
+            assert np.array_equal(np.sort(ids[a:b]), np.sort(pts["id"][idx[a:b].astype(np.int64)])), qs[i]
+    engine.close()
+    tree.close()
