@@ -80,13 +80,9 @@ TreeLayout tree_layout(pst_dtype dt, pst_idtype it, uint64_t n)
 	return L;
 }
 
-// Subtree builder capacity: nodes of at most ST_CAP points are finished by one CTA
-// (a power of two; PST_SUBTREE_CAP overrides it at build time).
-#ifndef PST_SUBTREE_CAP
-#define PST_SUBTREE_CAP 512
-#endif
-constexpr uint32_t ST_CAP = PST_SUBTREE_CAP;
-constexpr int ST_THREADS = 256;
+// Subtree builder capacity: nodes of at most ST_CAP points are finished by one CTA.
+constexpr uint32_t ST_CAP = 512;
+constexpr int ST_THREADS = 128;
 // Arg-max tiles, and the tiles a second maximum covers.
 constexpr uint32_t TM_TILE = 512, TM_SUPER = 32;
 constexpr int LV_THREADS = 256;
@@ -550,99 +546,160 @@ __global__ void __launch_bounds__(LV_THREADS) k_level(BuildCtx<T, HAS_ID> c, uin
 }
 
 // ---------------------------------------------------------------------------
-// Subtree builder: one CTA per node of level L0 finishes its whole subtree.  The
-// CTA holds the 64-bit dim2 keys of its points in dim1 order, each with the slot
-// of its point in a shared-memory copy of the subtree's points (gathered once, all
-// reads in flight together), so node writes never wait on global memory.
+// Subtree builder: one CTA per node of level L0 finishes its whole subtree.
+//
+// The CTA gathers the 64-bit dim2 keys of its free points in dim1 order into shared
+// memory.  Sub-levels whose nodes hold more than 32 points are built in place, a warp per
+// node, as the wide levels are: from the maxima of 32 positions and the positions that a
+// node's bounds cut, a taken key becoming 0.  Then a warp takes each node of at most 32
+// points, a point a lane, and builds all of its sub-levels in registers: a lane knows the
+// lanes of its node (a mask) and the node's place; the largest key of a node is a scan over
+// its lanes; the lane that holds it writes the node, the lane next to the left half's end
+// its median, and every other lane goes down to a child.  No key moves, no lane waits for
+// another warp.
+//
+// Bound by instruction issue.  With a compaction of all keys per sub-level (each a pass for
+// the maxima, one for the node writes and one to move the keys, with barriers between) the
+// kernel took 2654 us at 2^26 points, 92 at 2^21 and 463 at 5 M doubles; now 1896, 68 and
+// 258.  Of the 1896, a copy that stops early puts some 400 in the gather, 500 in the
+// sub-levels of large nodes and 300 before the first sub-level of the small ones.  CTAs of
+// 256 threads took 2184 us (more wait at the barriers), of 64 1836 (but 0.5 % more in all at
+// 2^21 points and 5 M doubles), of 32 no less; 256 points a CTA 1957 us and a wide level more.
 
-// Shared-memory carve-up of k_subtree, in bytes: points first (8-byte aligned for
-// doubles), then the u64 keys, the u16 point slots, the u16 sub-node of every key
-// and the u16 arg-max per sub-node.
-template <typename T, bool HAS_ID>
-struct SubtreeSmem {
-	static constexpr size_t PTS = 0;
-	static constexpr size_t KEYA = PTS + (size_t) ST_CAP * sizeof(Point<T, HAS_ID>);
-	static constexpr size_t KEYB = KEYA + (size_t) ST_CAP * 8;
-	static constexpr size_t SLOTA = KEYB + (size_t) ST_CAP * 8;
-	static constexpr size_t SLOTB = SLOTA + (size_t) ST_CAP * 2;
-	static constexpr size_t SEGA = SLOTB + (size_t) ST_CAP * 2;
-	static constexpr size_t SEGB = SEGA + (size_t) ST_CAP * 2;
-	static constexpr size_t TOPI = SEGB + (size_t) ST_CAP * 2;
-	static constexpr size_t CNT = TOPI + (size_t) ST_CAP * 2;
-	static constexpr size_t START = CNT + (size_t) ST_CAP * 2;
-	static constexpr size_t WS = START + (size_t) ST_CAP * 2;
-	static constexpr size_t BYTES = WS + 33 * 4;
-	static_assert(KEYA % 8 == 0 && BYTES <= 227 * 1024, "subtree builder shared memory");
-};
+constexpr uint32_t ST_ROWS = ST_CAP / 32;           // positions of a warp-wide row
+constexpr uint32_t ST_TOP = ST_ROWS;                // nodes of at most 32 points, at most
+constexpr int ST_WARPS = ST_THREADS / 32;
+static_assert(ST_CAP == 512 && ST_TOP <= 32, "rows and top nodes are counted in lanes");
 
 // Chunks of ST_THREADS positions the key gather reads: a node's range holds its
 // cN <= ST_CAP free points and at most one point taken by each ancestor (< 32).
 constexpr int ST_GATHER = (ST_CAP + ST_THREADS - 1) / ST_THREADS + 1;
 
-// Count and start of every sub-node of the current sub-level (in that sub-level's
-// compacted key order) are kept in shared memory and derived level to level
-// without a scan: going down one level removes each node's point (every node
-// above the last level holds one), the left child keeps the first floor(c/2) of
-// the rest and the right child the others, so
-//   start(2t) = start(t) - t,  start(2t+1) = start(t) - t + floor(c/2).
+// A lane of a warp that builds a node of at most 32 points: its point and dim2 key, whether
+// the point is still free, the lanes of its node that are, and the node's place.
+template <typename T, bool HAS_ID>
+struct SubtreeLane {
+	Point<T, HAS_ID> pt;
+	uint32_t hi, lo;  // the dim2 key's words
+	bool alive;
+	bool right;       // its node is a right child
+	uint32_t seg, h;
+};
 
-// Sub-node counts and warps come in powers of two: every quotient in the builder is
-// a shift (a run-time divisor costs a division sequence per use, and the builder is
-// bound by its instruction issue).
-constexpr int ST_LOG_WARPS = 3;
-static_assert(ST_THREADS == 32 << ST_LOG_WARPS, "k_subtree: 8 warps");
+// The largest value of the lanes of the lane's node, at its last lane: a scan over the
+// lanes from its first on, which lie within the node's points (32 >> U at most) and one
+// lane for each ancestor in the warp.
+template <int U>
+__device__ __forceinline__ uint32_t node_max(uint32_t v, uint32_t past_start)
+{
+	constexpr uint32_t SPAN = (32u >> U) + U;
+#pragma unroll
+	for (uint32_t o = 1; o < SPAN && o < 32; o <<= 1) {
+		const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, v, o);
+		if (past_start >= o)
+			v = max(v, x);
+	}
+	return v;
+}
+
+// Sub-levels U .. 5 of the warp's node, `left` of them below sub-level 0.
+template <typename T, bool HAS_ID, int U>
+__device__ __forceinline__ void subtree_levels(const BuildCtx<T, HAS_ID> &c, SubtreeLane<T, HAS_ID> &me, uint32_t left,
+                                               uint32_t half, uint32_t first, uint32_t *s_occ)
+{
+	const uint32_t below = lanemask_lt(), seg = me.seg;
+	// the largest key's high word, then, where a node has several of it, its low word
+	bool win;
+	if constexpr (U == 5) {
+		win = me.alive;  // one point a node
+	} else {
+		const uint32_t start = __ffs(seg) - 1, end = (31 - __clz(seg)) & 31, past = lane_id() - start;
+		// (a dead lane's past may wrap round: its value is never read)
+		const uint32_t v = me.alive ? me.hi : 0u;
+		uint32_t top;
+		if constexpr (U == 0) {
+			top = __reduce_max_sync(0xFFFFFFFFu, v);
+		} else if constexpr (U == 1) {
+			const uint32_t l = __reduce_max_sync(0xFFFFFFFFu, me.right ? 0u : v),
+			               r = __reduce_max_sync(0xFFFFFFFFu, me.right ? v : 0u);
+			top = me.right ? r : l;
+		} else {
+			top = __shfl_sync(0xFFFFFFFFu, node_max<U>(v, past), end);
+		}
+		win = me.alive && me.hi == top;
+		const uint32_t many = __ballot_sync(0xFFFFFFFFu, win) & seg;
+		if (__any_sync(0xFFFFFFFFu, win && (many & (many - 1)) != 0)) {
+			const uint32_t low = __shfl_sync(0xFFFFFFFFu, node_max<U>(win ? me.lo : 0u, past), end);
+			win = win && me.lo == low;
+		}
+	}
+	const uint32_t rest = seg & ~__ballot_sync(0xFFFFFFFFu, win);
+	const uint32_t ct = __popc(seg), r = __popc(rest & below), lh = ct / 2;
+	if (win) {
+		c.write_node(me.h, me.pt);
+		if (ct == 1 && me.h < half)
+			c.med[me.h] = me.pt.dim1;  // a node of one point: its own dim1
+		if (U == left)
+			atomicOr(&s_occ[(me.h - first) >> 5], 1u << ((me.h - first) & 31));
+		me.alive = false;
+	}
+	if constexpr (U < 5) {
+		if (U == left)
+			return;
+		// the left child's lanes end with the median's
+		const bool med = me.alive && r + 1 == lh;
+		if (med)
+			c.med[me.h] = me.pt.dim1;
+		const uint32_t mm = __ballot_sync(0xFFFFFFFFu, med) & seg;
+		const uint32_t lm = mm ? rest & (2u * mm - 1u) : 0u;
+		me.right = r >= lh;
+		me.seg = me.right ? rest & ~lm : lm;
+		me.h = 2 * me.h + (me.right ? 1u : 0u);
+		subtree_levels<T, HAS_ID, U + 1>(c, me, left, half, first, s_occ);
+	}
+}
 
 template <typename T, bool HAS_ID>
 __global__ void __launch_bounds__(ST_THREADS) k_subtree(BuildCtx<T, HAS_ID> c, uint32_t L0,
                                                        const uint32_t *__restrict__ B)
 {
-	using SM = SubtreeSmem<T, HAS_ID>;
+	using Ctx = BuildCtx<T, HAS_ID>;
+	using K = typename Ctx::K;
 	using Pt = Point<T, HAS_ID>;
-	extern __shared__ __align__(16) unsigned char st_smem[];
-	Pt *spts = reinterpret_cast<Pt *>(st_smem + SM::PTS);
-	uint64_t *kc = reinterpret_cast<uint64_t *>(st_smem + SM::KEYA);
-	uint64_t *kn = reinterpret_cast<uint64_t *>(st_smem + SM::KEYB);
-	uint16_t *sc = reinterpret_cast<uint16_t *>(st_smem + SM::SLOTA);
-	uint16_t *sn = reinterpret_cast<uint16_t *>(st_smem + SM::SLOTB);
-	uint16_t *gc = reinterpret_cast<uint16_t *>(st_smem + SM::SEGA);     // sub-node of each key
-	uint16_t *gn = reinterpret_cast<uint16_t *>(st_smem + SM::SEGB);
-	uint16_t *topi = reinterpret_cast<uint16_t *>(st_smem + SM::TOPI);    // [ST_CAP]
-	uint16_t *scnt = reinterpret_cast<uint16_t *>(st_smem + SM::CNT);     // [ST_CAP]
-	uint16_t *sstart = reinterpret_cast<uint16_t *>(st_smem + SM::START); // [ST_CAP]
-	uint32_t *ws = reinterpret_cast<uint32_t *>(st_smem + SM::WS);        // [33]
-	__shared__ uint32_t s_pre[ST_GATHER][ST_THREADS / 32];
-	__shared__ uint64_t s_pk[ST_THREADS / 32];
-	__shared__ uint32_t s_pi[ST_THREADS / 32];
+	constexpr bool KEYS4 = sizeof(K) == 4;
+	__shared__ uint64_t s_key[ST_CAP];            // 0 once taken
+	__shared__ K s_k1[KEYS4 ? ST_CAP : 1];        // dim1 keys (with rebuilt points)
+	__shared__ uint64_t s_row[ST_ROWS];           // largest key of 32 positions
+	__shared__ uint16_t s_b[2][ST_TOP + 1];       // bounds of the sub-level's nodes
+	__shared__ uint16_t s_top[ST_TOP];            // position of the point of sub-node 1, 2, 3, ..
+	__shared__ uint16_t s_list[ST_WARPS][32];
+	__shared__ uint32_t s_occ[2 * ST_CAP / 32];   // occupied nodes of the last level
+	__shared__ uint32_t s_pre[ST_GATHER][ST_WARPS];
 	__shared__ uint32_t s_n;
 
 	const uint32_t j = blockIdx.x;
 	const uint32_t cN = node_count32((uint32_t) c.n, L0, j);
-	if (cN == 0 || *c.err)
+	if (cN == 0 || __any_sync(0xFFFFFFFFu, *c.err != 0))
 		return;
-	const uint32_t lo = L0 ? B[j] : 0u;
-	const uint32_t hi = L0 ? B[j + 1] : (uint32_t) c.n;
-	if (lo >= hi || hi > c.n || cN > ST_CAP || hi - lo > (uint32_t) (ST_GATHER * ST_THREADS)) {
+	const uint32_t lo0 = L0 ? B[j] : 0u;
+	const uint32_t hi0 = L0 ? B[j + 1] : (uint32_t) c.n;
+	if (lo0 >= hi0 || hi0 > c.n || cN > ST_CAP || hi0 - lo0 > (uint32_t) (ST_GATHER * ST_THREADS)) {
 		if (threadIdx.x == 0)
 			atomicOr(c.err, 16u);
 		return;
 	}
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = ST_THREADS / 32;
+	const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
 
-	// Gather the keys of the points still free in [lo, hi), in dim1 order: every
+	// Gather the keys of the points still free in [lo0, hi0), in dim1 order: every
 	// read in flight at once, then one prefix over (chunk, warp).
-	using K = typename BuildCtx<T, HAS_ID>::K;
-	// with rebuilt points the dim1 keys come along (contiguous, like the dim2 keys),
-	// staged in kn, which the sub-levels only use later
-	constexpr bool KEYS4 = sizeof(K) == 4;
-	K *k1c = reinterpret_cast<K *>(kn);
 	{
 		uint64_t v[ST_GATHER];
 		K v1[ST_GATHER];
 		uint32_t m[ST_GATHER];
 #pragma unroll
 		for (int u = 0; u < ST_GATHER; u++) {
-			const uint32_t i = lo + (uint32_t) u * ST_THREADS + threadIdx.x;
-			const bool in = i < hi;
+			const uint32_t i = lo0 + (uint32_t) u * ST_THREADS + threadIdx.x;
+			const bool in = i < hi0;
 			v[u] = in ? c.c2s[i] : 0;
 			v1[u] = (KEYS4 && c.recon && in) ? c.k1s[i] : K(0);
 		}
@@ -652,27 +709,18 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(BuildCtx<T, HAS_ID> c, u
 			if (lane == 0)
 				s_pre[u][warp] = __popc(m[u]);
 		}
+		for (uint32_t i = threadIdx.x; i < 2 * ST_CAP / 32; i += ST_THREADS)
+			s_occ[i] = 0;
 		__syncthreads();
 		if (warp == 0) {
-			// (chunk, warp) pairs in order; lane l sums pairs [l * PER, l * PER + PER)
-			constexpr int PAIRS = ST_GATHER * (ST_THREADS / 32), PER = (PAIRS + 31) / 32;
+			// (chunk, warp) pairs in order, a lane each
+			constexpr int PAIRS = ST_GATHER * ST_WARPS;
+			static_assert(PAIRS <= 32, "a pair a lane");
 			uint32_t *flat = &s_pre[0][0];
-			uint32_t loc[PER], sum = 0;
-#pragma unroll
-			for (int k = 0; k < PER; k++) {
-				const int q = lane * PER + k;
-				loc[k] = q < PAIRS ? flat[q] : 0u;
-				sum += loc[k];
-			}
-			const uint32_t inc = warp_incl_scan(sum);
-			uint32_t run = inc - sum;
-#pragma unroll
-			for (int k = 0; k < PER; k++) {
-				const int q = lane * PER + k;
-				if (q < PAIRS)
-					flat[q] = run;
-				run += loc[k];
-			}
+			const uint32_t n = lane < PAIRS ? flat[lane] : 0u;
+			const uint32_t inc = warp_incl_scan(n);
+			if (lane < PAIRS)
+				flat[lane] = inc - n;
 			if (lane == 31)
 				s_n = inc;
 		}
@@ -682,14 +730,16 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(BuildCtx<T, HAS_ID> c, u
 			if ((m[u] >> lane) & 1u) {
 				const uint32_t pos = s_pre[u][warp] + __popc(m[u] & lanemask_lt());
 				if (pos < ST_CAP) {
-					kc[pos] = v[u];
-					sc[pos] = (uint16_t) pos;
-					gc[pos] = 0;
+					s_key[pos] = v[u];
 					if (KEYS4 && c.recon)
-						k1c[pos] = v1[u];
+						s_k1[pos] = v1[u];
 				}
 			}
 		}
+	}
+	if (threadIdx.x == 0) {
+		s_b[0][0] = 0;
+		s_b[0][1] = (uint16_t) cN;
 	}
 	__syncthreads();
 	if (s_n != cN) {
@@ -697,214 +747,139 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(BuildCtx<T, HAS_ID> c, u
 			atomicOr(c.err, 2u);
 		return;
 	}
-	// ... and their points: rebuilt from the keys when they can be (no global read
-	// at all), otherwise gathered from the input, every read of the CTA in flight at
-	// once (one random 12- or 24-byte read per point)
-	{
-		constexpr int PER = (ST_CAP + ST_THREADS - 1) / ST_THREADS;
-		Pt tmp[PER];
-#pragma unroll
-		for (int u = 0; u < PER; u++) {
-			const uint32_t i = threadIdx.x + u * ST_THREADS;
-			if (i < cN) {
-				if (KEYS4 && c.recon)
-					tmp[u] = BuildCtx<T, HAS_ID>::point_from_keys(k1c[i], kc[i]);
-				else
-					tmp[u] = c.point_of_tb(BuildCtx<T, HAS_ID>::tb_of(kc[i]));
-			}
+	// the point at position pos, whose key is (or was) `key`
+	auto point_at = [&](uint32_t pos, uint64_t key) -> Pt {
+		if constexpr (KEYS4) {
+			if (c.recon)
+				return Ctx::point_from_keys(s_k1[pos], key);
 		}
-#pragma unroll
-		for (int u = 0; u < PER; u++) {
-			const uint32_t i = threadIdx.x + u * ST_THREADS;
-			if (i < cN)
-				spts[i] = tmp[u];
-		}
-	}
-	__syncthreads();
+		return c.point_of_tb(Ctx::tb_of(key));
+	};
 	const uint32_t h0 = (1u << L0) + j;
 	const uint32_t last_s = c.D - 1 - L0;
 	const uint32_t half = 1u << (c.D - 1);  // med exists for positions < half
-	uint32_t present = cN;
-	if (threadIdx.x == 0) {
-		scnt[0] = (uint16_t) cN;
-		sstart[0] = 0;
+	// sub-levels whose largest node (cN >> s points) holds more than 32
+	uint32_t S = 0;
+	while ((cN >> S) > 32)
+		S++;
+	if (S) {
+		for (uint32_t r = warp; r < (cN + 31) / 32; r += ST_WARPS) {
+			const uint64_t k = 32 * r + lane < cN ? s_key[32 * r + lane] : 0ull;
+			const uint64_t m = warp_max_key(k);
+			if (lane == 0)
+				s_row[r] = m;
+		}
+		__syncthreads();
 	}
-	__syncthreads();
-	for (uint32_t s = 0;; s++) {
-		const uint32_t nsub = 1u << s;
-		const bool wide = (present >> s) >= 64;
-		// arg-max of every sub-node (keys are distinct)
-		if (wide && nsub < (uint32_t) nwarps) {
-			// fewer sub-nodes than warps: each sub-node's keys are split over
-			// W = nwarps / nsub warps, whose maxima meet in shared memory
-			const uint32_t lw = ST_LOG_WARPS - s;  // log2 W
-			const uint32_t W = 1u << lw, t = (uint32_t) warp >> lw, p = (uint32_t) warp & (W - 1u);
-			const uint32_t ct = scnt[t], st = sstart[t];
-			const uint32_t a = st + ((ct * p) >> lw), e = st + ((ct * (p + 1)) >> lw);
-			uint64_t bk = 0;
-			uint32_t bi = 0;
-			for (uint32_t i = a + lane; i < e; i += 32)
-				if (kc[i] > bk) {
-					bk = kc[i];
-					bi = i;
-				}
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1) {
-				const uint64_t ok = __shfl_xor_sync(0xFFFFFFFFu, bk, o);
-				const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-				if (ok > bk) {
-					bk = ok;
-					bi = oi;
-				}
+	for (uint32_t s = 0; s < S; s++) {
+		const uint16_t *b = s_b[s & 1];
+		uint16_t *bn = s_b[(s + 1) & 1];
+		for (uint32_t t = warp; t < (1u << s); t += ST_WARPS) {
+			const uint32_t lo = b[t], hi = b[t + 1];
+			const uint32_t h = (h0 << s) + t;
+			const uint32_t anc = lane < s ? s_top[((1u << s) + t) >> (lane + 1)] : 0u;
+			// the node's points: its positions without those that its ancestors took
+			const bool took = lane < s && anc >= lo && anc < hi;
+			const uint32_t ct = hi - lo - __popc(__ballot_sync(0xFFFFFFFFu, took));
+			// whole rows [rf, rl), and the positions before and after them (a node without
+			// whole rows spans fewer than 64 positions)
+			const uint32_t rf = (lo + 31) / 32, rl = hi / 32;
+			const bool rows = rf < rl;
+			const uint32_t p0 = lo + lane, p1 = rows ? 32 * rl + lane : lo + 32 + lane;
+			const uint64_t k0 = p0 < (rows ? 32 * rf : hi) ? s_key[p0] : 0ull, k1 = p1 < hi ? s_key[p1] : 0ull,
+			               kr = rows && rf + lane < rl ? s_row[rf + lane] : 0ull;
+			const uint64_t best = warp_max_key(max(max(k0, k1), kr));
+			const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, k0 == best), b1 = __ballot_sync(0xFFFFFFFFu, k1 == best),
+			               br = __ballot_sync(0xFFFFFFFFu, kr == best);
+			uint32_t tp;
+			if (b0) {
+				tp = lo + __ffs(b0) - 1;
+			} else if (b1) {
+				tp = (rows ? 32 * rl : lo + 32) + __ffs(b1) - 1;
+			} else {
+				const uint32_t r = rf + __ffs(br) - 1;
+				const uint64_t k = s_key[32 * r + lane];
+				tp = 32 * r + __ffs(__ballot_sync(0xFFFFFFFFu, k == best)) - 1;
+				const uint64_t m = warp_max_key(k == best ? 0ull : k);
+				if (lane == 0)
+					s_row[r] = m;
+			}
+			if (best == 0 && lane == 0)
+				atomicOr(c.err, 8u);
+			// the median, as on the wide levels
+			const uint32_t first = lo + ct / 2 - 1;
+			uint32_t pos = first;
+			for (;;) {
+				const uint32_t p = first + (tp <= pos) + __popc(__ballot_sync(0xFFFFFFFFu, took && anc <= pos));
+				if (p == pos)
+					break;
+				pos = p;
+			}
+			if (pos >= hi) {
+				if (lane == 0)
+					atomicOr(c.err, 4u);
+				pos = hi - 1;
 			}
 			if (lane == 0) {
-				s_pk[warp] = bk;
-				s_pi[warp] = bi;
+				bn[2 * t] = (uint16_t) lo;
+				bn[2 * t + 1] = (uint16_t) (pos + 1);
+				if (t + 1 == (1u << s))
+					bn[2 * t + 2] = (uint16_t) hi;
+				s_top[(1u << s) + t] = (uint16_t) tp;
+				c.write_node(h, point_at(tp, best));
+				s_key[tp] = 0;
 			}
-			__syncthreads();
-			if (threadIdx.x < nsub) {
-				uint64_t mk = 0;
-				uint32_t mi = 0;
-				for (uint32_t q = threadIdx.x * W; q < threadIdx.x * W + W; q++)
-					if (s_pk[q] > mk) {
-						mk = s_pk[q];
-						mi = s_pi[q];
-					}
-				topi[threadIdx.x] = (uint16_t) mi;
-			}
-		} else if (wide) {
-			for (uint32_t t = warp; t < nsub; t += nwarps) {
-				const uint32_t ct = scnt[t], st = sstart[t];
-				uint64_t bk = 0;
-				uint32_t bi = 0;
-				for (uint32_t i = st + lane; i < st + ct; i += 32)
-					if (kc[i] > bk) {
-						bk = kc[i];
-						bi = i;
-					}
-#pragma unroll
-				for (int o = 16; o > 0; o >>= 1) {
-					const uint64_t ok = __shfl_xor_sync(0xFFFFFFFFu, bk, o);
-					const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-					if (ok > bk) {
-						bk = ok;
-						bi = oi;
-					}
-				}
-				if (lane == 0)
-					topi[t] = (uint16_t) bi;
-			}
-		} else {
-			for (uint32_t t = threadIdx.x; t < nsub; t += ST_THREADS) {
-				const uint32_t ct = scnt[t], st = sstart[t];
-				uint64_t bk = 0;
-				uint32_t bi = 0;
-				for (uint32_t i = st; i < st + ct; i++)
-					if (kc[i] > bk) {
-						bk = kc[i];
-						bi = i;
-					}
-				topi[t] = (uint16_t) bi;
-			}
+			if (lane == 1)
+				c.med[h] = point_at(pos, s_key[pos]).dim1;
 		}
-		__syncthreads();
-		// write the nodes of this sub-level (warps past the last sub-node skip whole)
-		for (uint32_t tb = 0; tb < nsub; tb += ST_THREADS) {
-			if (tb + (uint32_t) warp * 32 >= nsub)
-				break;
-			const uint32_t t = tb + threadIdx.x;
-			bool occupied = false;
-			uint32_t h = 0;
-			if (t < nsub) {
-				const uint32_t ct = scnt[t], st = sstart[t];
-				h = (h0 << s) + t;
-				if (ct > 0) {
-					occupied = true;
-					const uint32_t ti = topi[t];
-					const Pt p = spts[sc[ti]];
-					c.write_node(h, p);
-					if (h < half) {
-						T m = p.dim1;  // a node of one point: its own dim1
-						if (ct >= 2) {
-							uint32_t mi = st + ct / 2 - 1;
-							if (ti <= mi)
-								mi++;
-							m = spts[sc[mi]].dim1;
-						}
-						c.med[h] = m;
-					}
-				}
-			}
-			// occupancy: the lanes of a warp cover one aligned run of <= 32 positions
-			const uint32_t bits = __ballot_sync(0xFFFFFFFFu, occupied);
-			const uint32_t first = __shfl_sync(0xFFFFFFFFu, h, 0);
-			if (lane == 0 && bits) {
-				const uint32_t wbase = (h0 << s) + tb + warp * 32;
-				if (nsub >= 32)
-					atomicOr(&c.occ[wbase >> 5], bits);
-				else
-					atomicOr(&c.occ[first >> 5], bits << (first & 31));
-			}
-		}
-		if (s == last_s)
-			break;
-		// drop each sub-node's point; every sub-node above the last level holds one.
-		// Every key knows its sub-node t, so it moves on its own: past the t points
-		// dropped before its sub-node, and its own sub-node's if that came first.  Of
-		// the keys a sub-node keeps, the first floor(ct / 2) go to its left child.
-		for (uint32_t i = threadIdx.x; i < present; i += ST_THREADS) {
-			const uint32_t t = gc[i];
-			const uint32_t ti = topi[t];
-			if (i != ti) {
-				const uint32_t ni = i - t - (i > ti ? 1u : 0u);
-				const uint32_t rank = ni - (sstart[t] - t);  // among the sub-node's keys kept
-				kn[ni] = kc[i];
-				sn[ni] = sc[i];
-				gn[ni] = (uint16_t) (2u * t + (rank >= (uint32_t) (scnt[t] >> 1) ? 1u : 0u));
-			}
-		}
-		// spans of the next sub-level, in place: parents to registers, then children
-		// (warps past the last sub-node have none)
-		constexpr int PMAX = (ST_CAP / 2 + ST_THREADS - 1) / ST_THREADS;
-		uint32_t pc[PMAX] = {}, ps[PMAX] = {};
-		const bool spans = (uint32_t) warp * 32 < nsub;
-		if (spans) {
-#pragma unroll
-			for (int u = 0; u < PMAX; u++) {
-				const uint32_t t = threadIdx.x + u * ST_THREADS;
-				if (t < nsub) {
-					pc[u] = scnt[t];
-					ps[u] = sstart[t];
-				}
-			}
-		}
-		__syncthreads();
-		if (spans) {
-#pragma unroll
-			for (int u = 0; u < PMAX; u++) {
-				const uint32_t t = threadIdx.x + u * ST_THREADS;
-				if (t < nsub) {
-					const uint32_t left = pc[u] / 2;
-					scnt[2 * t] = (uint16_t) (pc[u] ? left : 0u);
-					scnt[2 * t + 1] = (uint16_t) (pc[u] ? pc[u] - 1 - left : 0u);
-					sstart[2 * t] = (uint16_t) (ps[u] - t);
-					sstart[2 * t + 1] = (uint16_t) (ps[u] - t + left);
-				}
-			}
-		}
-		present -= nsub;
-		uint64_t *tk = kc;
-		kc = kn;
-		kn = tk;
-		uint16_t *ts = sc;
-		sc = sn;
-		sn = ts;
-		ts = gc;
-		gc = gn;
-		gn = ts;
 		__syncthreads();
 	}
-
+	for (uint32_t t = warp; t < (1u << S); t += ST_WARPS) {
+		const uint32_t lo = s_b[S & 1][t], hi = s_b[S & 1][t + 1];
+		// the free positions of the node, in order: at most 32 among its own and its
+		// ancestors'
+		const uint32_t p0 = lo + lane, p1 = p0 + 32;
+		const bool f0 = p0 < hi && s_key[p0] != 0, f1 = p1 < hi && s_key[p1] != 0;
+		const uint32_t a0 = __ballot_sync(0xFFFFFFFFu, f0), a1 = __ballot_sync(0xFFFFFFFFu, f1);
+		const uint32_t n0 = __popc(a0), cnt = n0 + __popc(a1);
+		if (cnt > 32) {
+			if (lane == 0)
+				atomicOr(c.err, 2u);
+			continue;
+		}
+		const uint32_t below = lanemask_lt();
+		if (f0)
+			s_list[warp][__popc(a0 & below)] = (uint16_t) p0;
+		if (f1)
+			s_list[warp][n0 + __popc(a1 & below)] = (uint16_t) p1;
+		__syncwarp();
+		bool alive = lane < cnt;
+		uint64_t key = 0;
+		Pt pt;
+		if (alive) {
+			const uint32_t pos = s_list[warp][lane];
+			key = s_key[pos];
+			pt = point_at(pos, key);
+		}
+		__syncwarp();  // the list is rewritten by the warp's next node
+		// the lane's node: its lanes that are left, and its place
+		SubtreeLane<T, HAS_ID> me{pt, (uint32_t) (key >> 32), (uint32_t) key, alive, false,
+		                          cnt < 32 ? (1u << cnt) - 1u : 0xFFFFFFFFu, (h0 << S) + t};
+		const uint32_t first = h0 << last_s;  // the CTA's first place on the last level
+		subtree_levels<T, HAS_ID, 0>(c, me, last_s - S, half, first, s_occ);
+	}
+	__syncthreads();
+	// occupancy: every node above the last level exists
+	for (uint32_t s = threadIdx.x; s <= last_s; s += ST_THREADS) {
+		const uint32_t base = h0 << s;
+		if (s < 5) {
+			const uint32_t bits = s == last_s ? s_occ[0] : (1u << (1u << s)) - 1u;
+			atomicOr(&c.occ[base >> 5], bits << (base & 31));
+		}
+	}
+	for (uint32_t s = 5; s <= last_s; s++)
+		for (uint32_t w = threadIdx.x; w < (1u << (s - 5)); w += ST_THREADS)
+			c.occ[((h0 << s) >> 5) + w] = s == last_s ? s_occ[w] : 0xFFFFFFFFu;
 }
 
 template <typename T>
@@ -1144,9 +1119,7 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 			std::swap(B, Bn);
 		}
 	}
-	constexpr size_t st_bytes = SubtreeSmem<T, HAS_ID>::BYTES;
-	PST_CUDA(cudaFuncSetAttribute(k_subtree<T, HAS_ID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) st_bytes));
-	k_subtree<T, HAS_ID><<<(unsigned) nodes_wide, ST_THREADS, st_bytes, s>>>(c, L0, B);
+	k_subtree<T, HAS_ID><<<(unsigned) nodes_wide, ST_THREADS, 0, s>>>(c, L0, B);
 	PST_CUDA(cudaGetLastError());
 	uint32_t errs[2] = {0, 0};
 	PST_CUDA(cudaMemcpyAsync(errs, flag, 8, cudaMemcpyDeviceToHost, s));
