@@ -132,11 +132,12 @@ void exclusive_scan(const T *in, U *out, uint64_t n, T *tmp, T *total_d, cudaStr
 // single-pass scheme of Adinets and Merrill, "Onesweep: A Faster Least Significant
 // Digit Radix Sort for GPUs" (2022), written for this library.  A first kernel
 // histograms the digits of every pass at once; in a
-// pass, each tile ranks its keys stably (warp-private digit counters; the lanes of
-// a warp holding the same digit are found with eight ballots, one per digit bit),
-// publishes its digit counts, and finds the counts of all earlier tiles by walking
-// back over their published aggregates until one carries an inclusive prefix
-// (decoupled look-back).  Tiles take their numbers from an atomic counter in the
+// pass, each tile counts its digits (warp-private counters) and publishes the counts,
+// then ranks its keys stably (the lanes of a warp holding the same digit are found
+// with eight ballots, one per digit bit) straight into their sorted places in shared
+// memory, and only then finds the counts of all earlier tiles, by walking back over
+// their published aggregates, RS_WINDOW at a time, until one carries an inclusive
+// prefix (decoupled look-back).  Tiles take their numbers from an atomic counter in the
 // order they start, so a tile only waits on tiles that are already running; every
 // wait is bounded and a wait that runs out raises an error flag instead of
 // scattering.  Keys move once per pass: read, staged in shared memory in sorted
@@ -148,6 +149,7 @@ constexpr int RS_THREADS = 256;
 constexpr int RS_ITEMS = 16;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_WARPS = RS_THREADS / 32;
+constexpr int RS_WINDOW = 4;  // status words a look-back step reads at once
 constexpr int RS_MAX_PASSES = 8;
 static_assert(RS_THREADS == 256, "one thread per digit in the digit scans");
 
@@ -213,9 +215,14 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_global_hist(const K *__restri
 }
 
 // One pass.  vals_in == nullptr means the identity payload (the key's input index;
-// 32-bit payloads only).  The tile's payloads are copied into shared memory
-// asynchronously as soon as the tile is known, so their reads overlap the ranking
-// and the look-back; each sorted key carries its input slot to find its payload.
+// 32-bit payloads only).  Bound by latency: each tile's phases depend on one another,
+// three CTAs to an SM overlap them, and the look-back waits for whichever tile before
+// this one ranks slowest.  So the counts leave before the ranking, which then hides
+// them (ranking first, one status word a step: 613 us a pass of 2^26 32-bit keys with
+// 64-bit payloads, 41 of 2^21; counts first 586 and 33; four words a step as well 554
+// and 30).  The payloads are read into registers before the ranking and staged sorted
+// beside their keys; copied to shared memory in input order and found by an index per
+// key, 2^26 took as long, but 64-bit keys 63 us a pass of 5 M in place of 58.
 template <typename K, typename V>
 __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in, const V *vals_in, K *keys_out,
                                                             V *vals_out, uint64_t n, int shift,
@@ -223,10 +230,9 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in,
                                                             uint32_t *tile_counter, uint32_t epoch, uint32_t *err)
 {
 	extern __shared__ __align__(16) unsigned char rs_smem[];
-	V *sv = reinterpret_cast<V *>(rs_smem);                         // payloads, input order
+	V *sv = reinterpret_cast<V *>(rs_smem);                         // payloads, sorted within the tile
 	K *sk = reinterpret_cast<K *>(sv + RS_TILE);                    // keys, sorted within the tile
-	uint16_t *si = reinterpret_cast<uint16_t *>(sk + RS_TILE);      // input slot of each sorted key
-	uint32_t *whist = reinterpret_cast<uint32_t *>(si + RS_TILE);   // [RS_WARPS][256]
+	uint32_t *whist = reinterpret_cast<uint32_t *>(sk + RS_TILE);   // [RS_WARPS][256]
 	uint32_t *dstart = whist + RS_WARPS * 256;                      // [256] tile-local digit start
 	uint32_t *gbase = dstart + 256;                                 // [256] global start of the digit for this tile
 	uint32_t *wsum = gbase + 256;                                   // [33]
@@ -244,28 +250,52 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in,
 	const uint64_t t0 = (uint64_t) tile * RS_TILE;
 	const uint64_t rem_n = n - t0;
 	const uint32_t tile_n = rem_n < (uint64_t) RS_TILE ? (uint32_t) rem_n : (uint32_t) RS_TILE;
-	if (vals_in) {
-		// 16-byte copies, then the (4-byte multiple) tail of a partial last tile
-		const unsigned char *src = reinterpret_cast<const unsigned char *>(vals_in + t0);
-		unsigned char *dst = reinterpret_cast<unsigned char *>(sv);
-		const uint32_t bytes = tile_n * (uint32_t) sizeof(V), body = bytes & ~15u;
-		for (uint32_t o = threadIdx.x * 16u; o < body; o += RS_THREADS * 16u)
-			cp_async16(dst + o, src + o);
-		for (uint32_t o = body + threadIdx.x * 4u; o < bytes; o += RS_THREADS * 4u)
-			cp_async4(dst + o, src + o);
-		cp_async_commit();
-	}
 	K k[RS_ITEMS];
-	uint32_t loc[RS_ITEMS];
 #pragma unroll
 	for (int i = 0; i < RS_ITEMS; i++) {
 		const uint64_t idx = t0 + (uint64_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
 		k[i] = idx < n ? keys_in[idx] : K(0);
 	}
+	// the tile's digit counts: out before the ranking, for the tiles behind this one
 #pragma unroll
 	for (int i = 0; i < RS_ITEMS; i++) {
 		const uint64_t idx = t0 + (uint64_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
-		const bool valid = idx < n;
+		if (idx < n)
+			atomicAdd(&whist[warp * 256 + rs_digit(k[i], shift)], 1u);
+	}
+	__syncthreads();
+	volatile uint64_t *st = reinterpret_cast<volatile uint64_t *>(status);
+	const uint64_t tag = (uint64_t) (epoch & 0x3FFFFFFFu) << 32;
+	uint32_t cnt = 0;
+	{
+		const uint32_t d = threadIdx.x;
+		uint32_t t[RS_WARPS];
+#pragma unroll
+		for (int w = 0; w < RS_WARPS; w++) {
+			t[w] = whist[w * 256 + d];
+			cnt += t[w];
+		}
+		st[(uint64_t) tile * 256 + d] = (tile == 0 ? RS_PREFIX : RS_AGG) | tag | cnt;
+		uint32_t tot;
+		uint32_t at = block_excl_scan<uint32_t>(cnt, &tot, wsum);
+		dstart[d] = at;
+#pragma unroll
+		for (int w = 0; w < RS_WARPS; w++) {
+			whist[w * 256 + d] = at;
+			at += t[w];
+		}
+	}
+	__syncthreads();
+	V pv[RS_ITEMS];
+#pragma unroll
+	for (int i = 0; i < RS_ITEMS; i++) {
+		const uint64_t idx = t0 + (uint64_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
+		pv[i] = vals_in ? idx < n ? vals_in[idx] : V(0) : (V) idx;
+	}
+#pragma unroll
+	for (int i = 0; i < RS_ITEMS; i++) {
+		const uint32_t local = (uint32_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
+		const bool valid = t0 + local < n;
 		const uint32_t d = rs_digit(k[i], shift);
 		const uint32_t peers = rs_peers(d, valid);
 		const int leader = valid ? __ffs(peers) - 1 : lane;
@@ -275,77 +305,61 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in,
 			whist[warp * 256 + d] = old + __popc(peers);
 		}
 		old = __shfl_sync(0xFFFFFFFFu, old, leader);
-		loc[i] = old + __popc(peers & lanemask_lt());
+		if (valid) {
+			const uint32_t lp = old + __popc(peers & lanemask_lt());
+			sk[lp] = k[i];
+			sv[lp] = pv[i];
+		}
 		__syncwarp();  // the next item's leaders read the counters written here
 	}
-	__syncthreads();
 	{
 		const uint32_t d = threadIdx.x;
-		uint32_t cnt = 0;
-#pragma unroll
-		for (int w = 0; w < RS_WARPS; w++) {
-			const uint32_t t = whist[w * 256 + d];
-			whist[w * 256 + d] = cnt;
-			cnt += t;
-		}
-		// publish this tile's count, then gather the counts of the tiles before it
-		volatile uint64_t *st = reinterpret_cast<volatile uint64_t *>(status);
-		const uint64_t tag = (uint64_t) (epoch & 0x3FFFFFFFu) << 32;
+		// the counts of the tiles before this one
 		uint64_t excl = 0;
-		if (tile == 0) {
-			st[d] = RS_PREFIX | tag | cnt;
-		} else {
-			st[(uint64_t) tile * 256 + d] = RS_AGG | tag | cnt;
+		if (tile != 0) {
 			int64_t t = (int64_t) tile - 1;
 			uint32_t spins = 0;
-			for (;;) {
-				const uint64_t x = st[(uint64_t) t * 256 + d];
-				const uint64_t f = x & RS_FLAGS;
-				if (f == 0 || (x & ~RS_FLAGS & ~0xFFFFFFFFull) != tag) {
+			for (bool done = false; !done;) {
+				uint64_t x[RS_WINDOW];
+#pragma unroll
+				for (int u = 0; u < RS_WINDOW; u++)
+					x[u] = t >= u ? st[(uint64_t) (t - u) * 256 + d] : 0ull;
+				int got = 0;
+#pragma unroll
+				for (int u = 0; u < RS_WINDOW; u++) {
+					const bool agg = ((x[u] ^ tag ^ RS_AGG) >> 32) == 0, pre = ((x[u] ^ tag ^ RS_PREFIX) >> 32) == 0;
+					if (!done && got == u && (agg || pre)) {
+						excl += (uint32_t) x[u];
+						got++;
+						done = pre;
+					}
+				}
+				t -= got;
+				if (!got) {
 					if (++spins > RS_SPIN_LIMIT) {
 						atomicOr(err, RS_ERR_LOOKBACK);
 						s_fail = 1;
 						break;
 					}
 					__nanosleep(64);
-					continue;
 				}
-				excl += x & 0xFFFFFFFFull;
-				if (f == RS_PREFIX)
-					break;
-				t--;
 			}
 			st[(uint64_t) tile * 256 + d] = RS_PREFIX | tag | (excl + cnt);
 		}
 		uint32_t tot;
 		const uint32_t hb = block_excl_scan<uint32_t>(hist[d], &tot, wsum);
-		dstart[d] = block_excl_scan<uint32_t>(cnt, &tot, wsum);
 		gbase[d] = hb + (uint32_t) excl;
 	}
 	__syncthreads();
-	if (s_fail) {
-		cp_async_wait_all();  // no copy may still target this CTA's shared memory
+	if (s_fail)
 		return;
-	}
-#pragma unroll
-	for (int i = 0; i < RS_ITEMS; i++) {
-		const uint32_t local = (uint32_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
-		if (t0 + local < n) {
-			const uint32_t d = rs_digit(k[i], shift);
-			const uint32_t lp = dstart[d] + whist[warp * 256 + d] + loc[i];
-			sk[lp] = k[i];
-			si[lp] = (uint16_t) local;
-		}
-	}
-	cp_async_wait_all();
-	__syncthreads();
 	for (uint32_t j = threadIdx.x; j < tile_n; j += RS_THREADS) {
 		const K key = sk[j];
 		const uint32_t d = rs_digit(key, shift);
 		const uint64_t g = (uint64_t) gbase[d] + (j - dstart[d]);
 		if (g < n) {
 			keys_out[g] = key;
-			vals_out[g] = vals_in ? sv[si[j]] : (V) (t0 + si[j]);
+			vals_out[g] = sv[j];
 		}
 	}
 }
@@ -353,7 +367,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in,
 template <typename K, typename V>
 constexpr size_t rs_onesweep_smem()
 {
-	return RS_TILE * (sizeof(K) + sizeof(V) + 2) + (RS_WARPS * 256 + 256 + 256 + 33) * 4;
+	return RS_TILE * (sizeof(K) + sizeof(V)) + (RS_WARPS * 256 + 256 + 256 + 33) * 4;
 }
 
 inline uint64_t rs_num_tiles(uint64_t n) { return (n + RS_TILE - 1) / RS_TILE; }
