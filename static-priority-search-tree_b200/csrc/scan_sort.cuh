@@ -158,18 +158,33 @@ constexpr uint64_t RS_AGG = 1ull << 62, RS_PREFIX = 2ull << 62, RS_FLAGS = 3ull 
 constexpr uint32_t RS_SPIN_LIMIT = 1u << 22;
 constexpr uint32_t RS_ERR_LOOKBACK = 32u;  // error bit raised when a look-back wait runs out
 
+// One byte of the key.
 template <typename K>
-__device__ __forceinline__ uint32_t rs_digit(K k, int shift) { return (uint32_t) (k >> shift) & 0xFFu; }
+__device__ __forceinline__ uint32_t rs_digit(K k, int shift)
+{
+	const uint32_t sel = 0x4440u | ((uint32_t) shift >> 3 & 3u);
+	if constexpr (sizeof(K) == 8)
+		return __byte_perm(shift >= 32 ? (uint32_t) (k >> 32) : (uint32_t) k, 0u, sel);
+	else
+		return __byte_perm(k, 0u, sel);
+}
 
-// Mask of the valid lanes of this warp that hold the same digit as this lane.
+// Mask of the valid lanes of this warp that hold the same digit as this lane (every
+// lane of the warp calls it).  A ballot per bit, in four instructions: the predicate,
+// the vote, this lane's flip and the three-input combination; written as an expression
+// it took more, and the ranking is bound by instructions (a pass of 2^26 32-bit keys
+// with 64-bit payloads 533 us, now 495; __match_any_sync 655; an atomic or of the lane's
+// bit on a mask per digit in shared memory 565).
 __device__ __forceinline__ uint32_t rs_peers(uint32_t d, bool valid)
 {
 	uint32_t peers = __ballot_sync(0xFFFFFFFFu, valid);
 #pragma unroll
 	for (int b = 0; b < 8; b++) {
-		const bool bit = (d >> b) & 1u;
-		const uint32_t m = __ballot_sync(0xFFFFFFFFu, bit);
-		peers &= bit ? m : ~m;
+		asm volatile("{ .reg .pred p; .reg .b32 t, m; and.b32 t, %1, %2; setp.ne.b32 p, t, 0;"
+		             " vote.sync.ballot.b32 m, p, 0xffffffff; selp.b32 t, 0, 0xffffffff, p;"
+		             " lop3.b32 %0, %0, m, t, 0x60; }"  // peers & (m ^ t)
+		             : "+r"(peers)
+		             : "r"(d), "r"(1u << b));
 	}
 	return peers;
 }
@@ -214,15 +229,21 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_global_hist(const K *__restri
 	}
 }
 
-// One pass.  vals_in == nullptr means the identity payload (the key's input index;
-// 32-bit payloads only).  Bound by latency: each tile's phases depend on one another,
-// three CTAs to an SM overlap them, and the look-back waits for whichever tile before
-// this one ranks slowest.  So the counts leave before the ranking, which then hides
-// them (ranking first, one status word a step: 613 us a pass of 2^26 32-bit keys with
-// 64-bit payloads, 41 of 2^21; counts first 586 and 33; four words a step as well 554
-// and 30).  The payloads are read into registers before the ranking and staged sorted
-// beside their keys; copied to shared memory in input order and found by an index per
-// key, 2^26 took as long, but 64-bit keys 63 us a pass of 5 M in place of 58.
+// One pass over n < 2^31 keys.  vals_in == nullptr means the identity payload (the key's
+// input index; 32-bit payloads only).  Bound by instructions (an issue slot in 1.7
+// taken) and by latency: each tile's phases depend on one another, three CTAs to an SM
+// overlap them, and the look-back waits for whichever tile before this one is slowest.
+// So the counts leave before the ranking, which then hides them, and the ranking is
+// unrolled without a test per key for a whole tile.  The payloads are read into
+// registers before the ranking and staged sorted beside their keys.  Microseconds a
+// pass, 2^21 and 2^26 32-bit keys with 64-bit payloads, 5 M 64-bit keys with 64-bit and
+// 32-bit ones: ranking before the counts, one status word a look-back step 41, 613, 78,
+// 71; counts first, four words 30, 554, 63, 52; payloads through registers 30, 560, 58,
+// 51 (before, copied to shared memory in input order and found by an index per key);
+// a lane reads its digit's counter itself, 32-bit slots and places 28, 533, 58, 49; the
+// ballots of rs_peers 26, 495, 54, 45; digits by byte, whole tiles apart 25, 469, 55, 45.
+// (Persistent CTAs that count the next tile before they write this one: 577 against 560.
+// Tiles of 3072 keys, four CTAs to an SM: 510; of 6144, two: 477.)
 template <typename K, typename V>
 __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in, const V *vals_in, K *keys_out,
                                                             V *vals_out, uint64_t n, int shift,
@@ -234,7 +255,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in,
 	K *sk = reinterpret_cast<K *>(sv + RS_TILE);                    // keys, sorted within the tile
 	uint32_t *whist = reinterpret_cast<uint32_t *>(sk + RS_TILE);   // [RS_WARPS][256]
 	uint32_t *dstart = whist + RS_WARPS * 256;                      // [256] tile-local digit start
-	uint32_t *gbase = dstart + 256;                                 // [256] global start of the digit for this tile
+	uint32_t *gbase = dstart + 256;                                 // [256] global start of the digit for this tile, less dstart
 	uint32_t *wsum = gbase + 256;                                   // [33]
 	__shared__ uint32_t s_tile, s_fail;
 
@@ -248,20 +269,20 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in,
 	__syncthreads();
 	const uint32_t tile = s_tile;
 	const uint64_t t0 = (uint64_t) tile * RS_TILE;
-	const uint64_t rem_n = n - t0;
-	const uint32_t tile_n = rem_n < (uint64_t) RS_TILE ? (uint32_t) rem_n : (uint32_t) RS_TILE;
+	const uint32_t tile_n = (uint32_t) (n - t0 < (uint64_t) RS_TILE ? n - t0 : (uint64_t) RS_TILE);
+	const uint32_t first = (uint32_t) warp * (RS_ITEMS * 32) + lane;  // this lane's slots: first + 32 i
+	const int left = (int) tile_n - (int) first;                      // valid: 32 i < left
+	uint32_t *wh = whist + warp * 256;
 	K k[RS_ITEMS];
+	const K *kp = keys_in + t0 + first;
 #pragma unroll
-	for (int i = 0; i < RS_ITEMS; i++) {
-		const uint64_t idx = t0 + (uint64_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
-		k[i] = idx < n ? keys_in[idx] : K(0);
-	}
+	for (int i = 0; i < RS_ITEMS; i++)
+		k[i] = 32 * i < left ? kp[32 * i] : K(0);
 	// the tile's digit counts: out before the ranking, for the tiles behind this one
 #pragma unroll
 	for (int i = 0; i < RS_ITEMS; i++) {
-		const uint64_t idx = t0 + (uint64_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
-		if (idx < n)
-			atomicAdd(&whist[warp * 256 + rs_digit(k[i], shift)], 1u);
+		if (32 * i < left)
+			atomicAdd(&wh[rs_digit(k[i], shift)], 1u);
 	}
 	__syncthreads();
 	volatile uint64_t *st = reinterpret_cast<volatile uint64_t *>(status);
@@ -287,31 +308,33 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in,
 	}
 	__syncthreads();
 	V pv[RS_ITEMS];
+	const V *vp = vals_in ? vals_in + t0 + first : nullptr;
 #pragma unroll
-	for (int i = 0; i < RS_ITEMS; i++) {
-		const uint64_t idx = t0 + (uint64_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
-		pv[i] = vals_in ? idx < n ? vals_in[idx] : V(0) : (V) idx;
-	}
+	for (int i = 0; i < RS_ITEMS; i++)
+		pv[i] = vp ? 32 * i < left ? vp[32 * i] : V(0) : (V) (t0 + first + 32 * i);
+	const uint32_t below = lanemask_lt();
+	auto rank = [&](auto full) {
 #pragma unroll
-	for (int i = 0; i < RS_ITEMS; i++) {
-		const uint32_t local = (uint32_t) warp * (RS_ITEMS * 32) + i * 32 + lane;
-		const bool valid = t0 + local < n;
-		const uint32_t d = rs_digit(k[i], shift);
-		const uint32_t peers = rs_peers(d, valid);
-		const int leader = valid ? __ffs(peers) - 1 : lane;
-		uint32_t old = 0;
-		if (valid && lane == leader) {
-			old = whist[warp * 256 + d];
-			whist[warp * 256 + d] = old + __popc(peers);
+		for (int i = 0; i < RS_ITEMS; i++) {
+			const bool valid = decltype(full)::value || 32 * i < left;
+			const uint32_t d = rs_digit(k[i], shift);
+			const uint32_t peers = rs_peers(d, valid);
+			uint32_t lp = 0;
+			if (valid) {
+				lp = wh[d] + __popc(peers & below);
+				sk[lp] = k[i];
+				sv[lp] = pv[i];
+			}
+			__syncwarp();  // every peer has read the counter: the last of them moves it on
+			if (valid && peers >> lane == 1u)
+				wh[d] = lp + 1u;
+			__syncwarp();  // the next key's lanes read the counters written here
 		}
-		old = __shfl_sync(0xFFFFFFFFu, old, leader);
-		if (valid) {
-			const uint32_t lp = old + __popc(peers & lanemask_lt());
-			sk[lp] = k[i];
-			sv[lp] = pv[i];
-		}
-		__syncwarp();  // the next item's leaders read the counters written here
-	}
+	};
+	if (tile_n == RS_TILE)
+		rank(std::true_type());
+	else
+		rank(std::false_type());
 	{
 		const uint32_t d = threadIdx.x;
 		// the counts of the tiles before this one
@@ -348,16 +371,16 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(const K *keys_in,
 		}
 		uint32_t tot;
 		const uint32_t hb = block_excl_scan<uint32_t>(hist[d], &tot, wsum);
-		gbase[d] = hb + (uint32_t) excl;
+		gbase[d] = hb + (uint32_t) excl - dstart[d];
 	}
 	__syncthreads();
 	if (s_fail)
 		return;
+#pragma unroll 4
 	for (uint32_t j = threadIdx.x; j < tile_n; j += RS_THREADS) {
 		const K key = sk[j];
-		const uint32_t d = rs_digit(key, shift);
-		const uint64_t g = (uint64_t) gbase[d] + (j - dstart[d]);
-		if (g < n) {
+		const uint32_t g = gbase[rs_digit(key, shift)] + j;
+		if (g < (uint32_t) n) {
 			keys_out[g] = key;
 			vals_out[g] = sv[j];
 		}
