@@ -217,6 +217,7 @@ __global__ void k_id_keys(const Point<T, HAS_ID> *pts, uint64_t n, uint32_t *key
 // Copies of the digit histogram a block of k_prep_keys keeps in shared memory (a
 // quarter of its warps on each), so that keys sharing a digit meet on fewer counters.
 constexpr int PK_HIST_COPIES = 4;
+constexpr int PK_THREADS = 512, PK_CTAS = 2, PK_ITEMS = 4;  // points in flight per thread
 
 // Keys in tiebreak-rank order r (input index P[r]): k1[r] = dim1 key and either the
 // final 64-bit dim2 key (4-byte values) or the raw dim2 key k2[r] (doubles).
@@ -228,8 +229,14 @@ constexpr int PK_HIST_COPIES = 4;
 // digits of the dim1 keys, hist[d * 256 + v] += keys whose digit d is v, for every
 // digit of the key (the radix sort's histogram, which the order of the keys does
 // not change); dynamic shared memory PK_HIST_COPIES * sizeof(K) * 256 words.
+// Bound by memory at 2^26 points (1.61 GB: 246 us), below some 10 M by the atomics that
+// end a CTA: up to 256 counters per digit and the ranges, all CTAs' on the same words.
+// So two CTAs of 512 threads to an SM and no more, which keep four points a thread in
+// flight, in place of up to 16 of 256 with one: 2^21 metacells 31.6 -> 13.5 us, 5 M
+// doubles 56.9 -> 35.2, 2^26 points 305 -> 282 (eight points 18, 61, 379; two 13.7, 37,
+// 322).
 template <typename T, bool HAS_ID, bool SCAN_IDS>
-__global__ void k_prep_keys(const Point<T, HAS_ID> *pts, const uint32_t *P, uint64_t n,
+__global__ void __launch_bounds__(PK_THREADS, PK_CTAS) k_prep_keys(const Point<T, HAS_ID> *pts, const uint32_t *P, uint64_t n,
                             typename KeyOf<T>::K *k1, uint64_t *c2, typename KeyOf<T>::K *k2,
                             typename KeyOf<T>::K *range, uint32_t *negzero, uint32_t *idflag,
                             uint32_t *id_range, uint32_t *hist)
@@ -247,34 +254,49 @@ __global__ void k_prep_keys(const Point<T, HAS_ID> *pts, const uint32_t *P, uint
 	bool nz = false;
 	uint32_t ilo = 0xFFFFFFFFu, ihi = 0;
 	bool dec = false, other = false;
-	for (uint64_t r = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (uint64_t) gridDim.x * blockDim.x) {
-		const Point<T, HAS_ID> p = pts[P ? P[r] : r];
-		if constexpr (SCAN_IDS && HAS_ID) {
-			const uint32_t v = p.id;
-			ilo = min(ilo, v);
-			ihi = max(ihi, v);
-			if (r + 1 < n && v > pts[r + 1].id)
-				dec = true;
-			if ((uint64_t) v != r)
-				other = true;
-		}
-		const K a = KeyOf<T>::key(p.dim1), b = KeyOf<T>::key(p.dim2);
-		if constexpr (!std::is_integral<T>::value)
-			nz |= (p.dim1 == T(0) && signbit(p.dim1)) || (p.dim2 == T(0) && signbit(p.dim2));
-		k1[r] = a;
-		if constexpr (sizeof(K) == 4)
-			c2[r] = ((uint64_t) b << 32) | (uint64_t) (r + 1);
-		else
-			k2[r] = b;
-		if (hist) {
+	const uint64_t step = (uint64_t) gridDim.x * PK_THREADS * PK_ITEMS;
+	for (uint64_t base = (uint64_t) blockIdx.x * PK_THREADS * PK_ITEMS + threadIdx.x; base < n; base += step) {
+		Point<T, HAS_ID> p[PK_ITEMS];
+		uint32_t after[PK_ITEMS];  // the next point's id
 #pragma unroll
-			for (int d = 0; d < ND; d++)
-				atomicAdd(&myh[d * 256 + (uint32_t) ((a >> (8 * d)) & 0xFFu)], 1u);
+		for (int u = 0; u < PK_ITEMS; u++) {
+			const uint64_t r = base + u * PK_THREADS;
+			if (r < n) {
+				p[u] = pts[P ? P[r] : r];
+				if constexpr (SCAN_IDS && HAS_ID)
+					after[u] = r + 1 < n ? pts[r + 1].id : 0xFFFFFFFFu;
+			}
 		}
-		lo1 = a < lo1 ? a : lo1;
-		hi1 = a > hi1 ? a : hi1;
-		lo2 = b < lo2 ? b : lo2;
-		hi2 = b > hi2 ? b : hi2;
+#pragma unroll
+		for (int u = 0; u < PK_ITEMS; u++) {
+			const uint64_t r = base + u * PK_THREADS;
+			if (r >= n)
+				break;
+			if constexpr (SCAN_IDS && HAS_ID) {
+				const uint32_t v = p[u].id;
+				ilo = min(ilo, v);
+				ihi = max(ihi, v);
+				dec |= v > after[u];
+				other |= (uint64_t) v != r;
+			}
+			const K a = KeyOf<T>::key(p[u].dim1), b = KeyOf<T>::key(p[u].dim2);
+			if constexpr (!std::is_integral<T>::value)
+				nz |= (p[u].dim1 == T(0) && signbit(p[u].dim1)) || (p[u].dim2 == T(0) && signbit(p[u].dim2));
+			k1[r] = a;
+			if constexpr (sizeof(K) == 4)
+				c2[r] = ((uint64_t) b << 32) | (uint64_t) (r + 1);
+			else
+				k2[r] = b;
+			if (hist) {
+#pragma unroll
+				for (int d = 0; d < ND; d++)
+					atomicAdd(&myh[d * 256 + rs_digit(a, 8 * d)], 1u);
+			}
+			lo1 = a < lo1 ? a : lo1;
+			hi1 = a > hi1 ? a : hi1;
+			lo2 = b < lo2 ? b : lo2;
+			hi2 = b > hi2 ? b : hi2;
+		}
 	}
 	if (__any_sync(0xFFFFFFFFu, nz) && (threadIdx.x & 31) == 0)
 		atomicOr(negzero, 1u);
@@ -1012,8 +1034,10 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 	// dim1 keys' digits for their sort
 	uint32_t *hist1 = scr.at<uint32_t>(SL.hist1);
 	PST_CUDA(cudaMemsetAsync(hist1, 0, RS_MAX_PASSES * 256 * 4, s));
+	const unsigned pk_g = (unsigned) std::min<uint64_t>((n + PK_THREADS * PK_ITEMS - 1) / (PK_THREADS * PK_ITEMS),
+	                                                    (uint64_t) device_info().sms * PK_CTAS);
 	const size_t pk_smem = (size_t) PK_HIST_COPIES * sizeof(K) * 256 * 4;
-	k_prep_keys<T, HAS_ID, HAS_ID><<<g, 256, pk_smem, s>>>(pts, nullptr, n, static_cast<K *>(k1), c2,
+	k_prep_keys<T, HAS_ID, HAS_ID><<<pk_g, PK_THREADS, pk_smem, s>>>(pts, nullptr, n, static_cast<K *>(k1), c2,
 	                                                       scr.at<K>(SL.k2), krange, flag + 4, flag, flag + 2,
 	                                                       hist1);
 	PST_CUDA(cudaGetLastError());
@@ -1043,7 +1067,7 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 			P = scr.at<uint32_t>(SL.P);
 			// the same keys in the new order: ranges and digit counts stand, so neither
 			// is made again (the sort's error bits in flag[1] are kept)
-			k_prep_keys<T, HAS_ID, false><<<g, 256, 0, s>>>(pts, P, n, static_cast<K *>(k1), c2, scr.at<K>(SL.k2),
+			k_prep_keys<T, HAS_ID, false><<<pk_g, PK_THREADS, 0, s>>>(pts, P, n, static_cast<K *>(k1), c2, scr.at<K>(SL.k2),
 			                                                krange, flag + 4, nullptr, nullptr, nullptr);
 			PST_CUDA(cudaGetLastError());
 		}
