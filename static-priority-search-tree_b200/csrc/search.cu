@@ -1730,10 +1730,13 @@ void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 	grid = (uint32_t) device_info().sms * blocks_per_sm;
 	const size_t vs = value_size(t->dtype);
 	path_cap = 2 * max_q;
-	// groups of queries for the first levels of a whole pass, a CTA each
+	// groups of queries for the first levels of a whole pass, a CTA each; for a batch of any
+	// size, also where waiting ones start with the one-CTA pass (1, 4, 16 and 32 isovalues,
+	// asynchronously: 124, 124, 130 and 134 us on 2^21 points by levels alone, 86, 91, 89
+	// and 88 this way; on 2^26 145, 155, 230 and 292, and 110, 122, 189 and 245)
 	group = (max_q + (uint32_t) device_info().sms - 1) / (uint32_t) device_info().sms;
 	group_stop = group_levels(t->levels, group);
-	if (group_stop < GROUP_MIN_LEVELS || max_q <= top_q)
+	if (group_stop < GROUP_MIN_LEVELS)
 		group_stop = 0;
 	ro_cap = max_q * (2 * 32 + (group_stop ? group_records(group_stop) : 0));
 	{

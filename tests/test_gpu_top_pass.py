@@ -74,11 +74,11 @@ def test_where_the_pass_stops_writing(pst, oracle, hits, ret):
 
 
 @pytest.mark.parametrize("dt", ["f32", "f64"])
-@pytest.mark.parametrize("nq,top", [(2, 1), (17, 4), (32, 1), (33, 1), (150, 1), (700, 1)])
+@pytest.mark.parametrize("nq,top", [(1, 1), (2, 1), (17, 4), (32, 1), (32, 32), (33, 1), (150, 1), (700, 1)])
 @pytest.mark.parametrize("n", [3, 700, 9001, 150001])
 def test_whole_passes(pst, oracle, dt, nq, top, n):
-    """Batches above the engine's limit for the top pass: the first levels by groups of
-    queries, the rest by level kernels; waiting and asynchronous, again and again (the
+    """Batches above the engine's limit for the top pass, and asynchronous ones within it:
+    the first levels by groups of queries, the rest by level kernels; waiting and asynchronous, again and again (the
     later passes from a graph), with other queries each time."""
     import torch
     pts = rand_points(n, dt, ids="random", dup=n == 700, seed=n + nq)
