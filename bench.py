@@ -54,6 +54,7 @@ SEL_LO, SEL_HI = 1e-7, 1e-2
 # needs no dim1 test, so the search can move as little as 12 B per point.
 BYTES_PER_PT = 16
 BYTES_PER_PT_MIN = 12
+GROUP_LEVELS = 11  # levels of the timed pass that k_bfs_groups takes in its one launch
 
 
 _T0 = time.perf_counter()
@@ -1051,7 +1052,7 @@ def main():
     peak, peak_kind = measured_peak()
     achieved = total * BYTES_PER_PT / (my_ms / 1000.0) / 1e9
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": None, "kernel": "batched search pass (k_bfs_level x levels + scan + k_emit)",
+            "traffic": None, "kernel": "batched search pass (k_bfs_groups + k_bfs_level x the levels below + scan + k_emit)",
             "bytes_per_unit": BYTES_PER_PT, "units_per_launch": total, "peak_source": f"{peak_kind} hbm_gbs",
             "frac_at_min_bytes": total * BYTES_PER_PT_MIN / (my_ms / 1000.0) / 1e9 / peak,
             "min_bytes_per_unit": BYTES_PER_PT_MIN}
@@ -1160,9 +1161,10 @@ def main():
             line["ips"] = ips_rows
         if iso_res is not None:
             line["isosurface"] = iso_res
-        # per step: the control block's load, query preparation, one kernel per level,
-        # offsets, emit (a batch of 4096 queries takes the one-launch offsets scan)
-        line["gpu_launches"] = (levels_main + 4) * args.steps
+        # per step: the control block's load, the first GROUP_LEVELS levels by groups of
+        # queries (28 of 4096 to each of 148 CTAs), one kernel per level below, offsets,
+        # emit (a batch of 4096 queries takes the one-launch offsets scan)
+        line["gpu_launches"] = (levels_main - GROUP_LEVELS + 4) * args.steps
         print(json.dumps(line))
     if eng is not None:
         eng.close()
