@@ -333,7 +333,10 @@ __global__ void k_rank_keys(const uint32_t *S2, uint64_t n, uint64_t *c2)
 	}
 }
 
-// The node count of node_count in 32 bits (trees hold fewer than 2^31 points).
+// Point count of the node at level d, index j within the level (trees hold fewer than
+// 2^31 points).  Construction gives a node of c points a left child of floor(c/2) and a
+// right child of c - 1 - floor(c/2) points (pst/static-pst-cpu-iter.tpp:512-541), so
+// counts depend on n and the node's path only.
 __device__ __forceinline__ uint32_t node_count32(uint32_t n, uint32_t d, uint32_t j)
 {
 	uint32_t c = n;

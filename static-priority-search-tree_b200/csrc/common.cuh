@@ -138,18 +138,6 @@ inline uint32_t tree_levels(uint64_t n)
 	return d;
 }
 
-// Point count of the node at level d, index j within the level.  Construction
-// gives a node of c points a left child of floor(c/2) and a right child of
-// c - 1 - floor(c/2) points (pst/static-pst-cpu-iter.tpp:512-541), so counts
-// depend on n and the node's path only.
-__host__ __device__ inline uint64_t node_count(uint64_t n, uint32_t d, uint64_t j)
-{
-	uint64_t c = n;
-	for (int b = (int) d - 1; b >= 0 && c != 0; b--)
-		c = ((j >> b) & 1) ? c - 1 - c / 2 : c / 2;
-	return c;
-}
-
 // ---------------------------------------------------------------------------
 // Warp helpers.
 

@@ -846,12 +846,6 @@ __device__ __forceinline__ void sh_st4(uint32_t a, const uint4 &v)
 {
 	asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-__device__ __forceinline__ uint32_t sh_ld(uint32_t a)
-{
-	uint32_t v;
-	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-	return v;
-}
 __device__ __forceinline__ void sh_st(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ uint32_t sh_add(uint32_t a, uint32_t n)
 {
