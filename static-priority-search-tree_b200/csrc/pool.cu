@@ -278,12 +278,27 @@ void pool_trim() noexcept
 void InFlight::mark(const void *owner, cudaStream_t s)
 {
 	std::lock_guard<std::mutex> lk(mu);
-	cudaEvent_t &e = ev[owner];
-	if (!e)
-		check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+	Mark &m = ev[owner];
+	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+	check_cuda(cudaStreamIsCapturing(s, &st), "cudaStreamIsCapturing");
+	if (st != cudaStreamCaptureStatusNone) {
+		m.captured = true;  // an earlier mark's event does not belong in the caller's graph
+		return;
+	}
+	if (!m.event)
+		check_cuda(cudaEventCreateWithFlags(&m.event, cudaEventDisableTiming), "cudaEventCreate");
 	else
-		check_cuda(cudaStreamWaitEvent(s, e, 0), "cudaStreamWaitEvent");
-	check_cuda(cudaEventRecord(e, s), "cudaEventRecord");
+		check_cuda(cudaStreamWaitEvent(s, m.event, 0), "cudaStreamWaitEvent");
+	check_cuda(cudaEventRecord(m.event, s), "cudaEventRecord");
+}
+
+void InFlight::wait_for(const Mark &m) noexcept
+{
+	if (m.captured)
+		cudaDeviceSynchronize();
+	else if (m.event)
+		cudaEventSynchronize(m.event);
+	cudaGetLastError();
 }
 
 void InFlight::wait(const void *owner) noexcept
@@ -292,11 +307,10 @@ void InFlight::wait(const void *owner) noexcept
 	auto it = ev.find(owner);
 	if (it == ev.end())
 		return;
-	if (it->second) {
-		cudaEventSynchronize(it->second);
-		cudaEventDestroy(it->second);
-		cudaGetLastError();
-	}
+	wait_for(it->second);
+	if (it->second.event)
+		cudaEventDestroy(it->second.event);
+	cudaGetLastError();
 	ev.erase(it);
 }
 
@@ -304,16 +318,14 @@ void InFlight::wait_all() noexcept
 {
 	std::lock_guard<std::mutex> lk(mu);
 	for (auto &x : ev)
-		if (x.second)
-			cudaEventSynchronize(x.second);
-	cudaGetLastError();
+		wait_for(x.second);
 }
 
 InFlight::~InFlight()
 {
 	for (auto &x : ev)
-		if (x.second)
-			cudaEventDestroy(x.second);
+		if (x.second.event)
+			cudaEventDestroy(x.second.event);
 	cudaGetLastError();
 }
 

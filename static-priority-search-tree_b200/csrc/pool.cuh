@@ -30,7 +30,8 @@ unsigned long long current_context_id(int dev);
 class InFlight {
   public:
 	// Marks the end of the work queued on `s` for `owner` (after its earlier mark, which
-	// may lie on another stream).
+	// may lie on another stream).  Work captured into a graph of the caller's may run at any
+	// time: from then on the owner waits for the whole device.
 	void mark(const void *owner, cudaStream_t s);
 	void wait(const void *owner) noexcept;  // and forget it
 	void wait_all() noexcept;
@@ -38,7 +39,12 @@ class InFlight {
 
   private:
 	std::mutex mu;
-	std::map<const void *, cudaEvent_t> ev;
+	struct Mark {
+		cudaEvent_t event = nullptr;
+		bool captured = false;
+	};
+	static void wait_for(const Mark &m) noexcept;
+	std::map<const void *, Mark> ev;
 };
 
 }  // namespace pst
