@@ -205,6 +205,33 @@ __device__ void block_range_fold(K lo, K hi, K *range)
 // ---------------------------------------------------------------------------
 // Preparation kernels.
 
+// What the key pass finds, in the construction's flag words.
+template <typename K>
+struct BuildFlags {
+	uint32_t id_order;     // bits of k_prep_keys' idflag
+	uint32_t err;          // error bits
+	uint32_t id_range[2];  // [min, max]
+	uint32_t negzero;      // -0.0 seen
+	uint32_t unused[11];
+	K range[4];  // [k1 min, k1 max, k2 min, k2 max]
+};
+static_assert(sizeof(BuildFlags<uint64_t>) <= 256 && offsetof(BuildFlags<uint64_t>, range) == 64, "flag words");
+
+// The flag words as k_prep_keys wants them, and the bounds of the root.  (A copy of each
+// from the host, and one back for each group of flags: 349 us for a build of 2^21
+// metacells, with the search index made behind another wait; now 314.)
+template <typename K>
+__global__ void k_build_init(uint32_t *flag, uint32_t *bounds, uint32_t n)
+{
+	BuildFlags<K> *f = reinterpret_cast<BuildFlags<K> *>(flag);
+	if (threadIdx.x < 16)
+		flag[threadIdx.x] = threadIdx.x == 2 ? 0xFFFFFFFFu : 0u;
+	if (threadIdx.x < 4)
+		f->range[threadIdx.x] = threadIdx.x & 1 ? K(0) : ~K(0);
+	if (threadIdx.x < 2)
+		bounds[threadIdx.x] = threadIdx.x ? n : 0u;
+}
+
 template <typename T, bool HAS_ID>
 __global__ void k_id_keys(const Point<T, HAS_ID> *pts, uint64_t n, uint32_t *keys)
 {
@@ -1012,17 +1039,8 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 	void *k1 = scr.at<void>(SL.k1), *kalt = scr.at<void>(SL.kalt);
 	uint64_t *c2 = scr.at<uint64_t>(SL.c2);
 	void *valt = scr.at<void>(SL.valt);
-	uint32_t *flag = scr.at<uint32_t>(SL.flags);  // [0] id order bits, [1] error bits, [2..3] id range, [4] -0.0 seen
+	uint32_t *flag = scr.at<uint32_t>(SL.flags);  // the words of BuildFlags
 	K *krange = reinterpret_cast<K *>(scr.at<unsigned char>(SL.flags) + 64);  // [k1 min, k1 max, k2 min, k2 max]
-	{
-		unsigned char init[256];
-		memset(init, 0, sizeof(init));
-		const uint32_t id_init[2] = {0xFFFFFFFFu, 0u};
-		memcpy(init + 8, id_init, 8);
-		const K kinit[4] = {~K(0), K(0), ~K(0), K(0)};
-		memcpy(init + 64, kinit, sizeof(kinit));
-		PST_CUDA(cudaMemcpyAsync(flag, init, sizeof(init), cudaMemcpyHostToDevice, s));
-	}
 	// one SortScratch for every sort of this build: its epoch tags the look-back
 	// status of each pass, which is cleared only here
 	SortScratch sc;
@@ -1030,13 +1048,17 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 	sc.hist = scr.at<uint32_t>(SL.rs_misc);
 	sc.counters = sc.hist + RS_MAX_PASSES * 256;
 	sc.err = flag + 1;
-	PST_CUDA(cudaMemsetAsync(sc.status, 0, 256 * rs_num_tiles(n) * 8, s));
+	sc.cleared = true;
+	uint32_t *B = scr.at<uint32_t>(SL.Ba), *Bn = scr.at<uint32_t>(SL.Bb);
+	// the sorts' status, counters and the digit counts, which lie side by side
+	PST_CUDA(cudaMemsetAsync(sc.status, 0, SL.flags - SL.rs_status, s));
+	k_build_init<K><<<1, 64, 0, s>>>(flag, B, (uint32_t) n);
+	PST_CUDA(cudaGetLastError());
 
 	const unsigned g = grid_for(n, 256);
 	// ---- keys, made in input order; the same pass checks the ids and counts the
 	// dim1 keys' digits for their sort
 	uint32_t *hist1 = scr.at<uint32_t>(SL.hist1);
-	PST_CUDA(cudaMemsetAsync(hist1, 0, RS_MAX_PASSES * 256 * 4, s));
 	const unsigned pk_g = (unsigned) std::min<uint64_t>((n + PK_THREADS * PK_ITEMS - 1) / (PK_THREADS * PK_ITEMS),
 	                                                    (uint64_t) device_info().sms * PK_CTAS);
 	const size_t pk_smem = (size_t) PK_HIST_COPIES * sizeof(K) * 256 * 4;
@@ -1044,27 +1066,26 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 	                                                       scr.at<K>(SL.k2), krange, flag + 4, flag, flag + 2,
 	                                                       hist1);
 	PST_CUDA(cudaGetLastError());
-	K range[4];
-	uint32_t negzero = 0, idscan[4] = {0, 0, 0, 0};
-	PST_CUDA(cudaMemcpyAsync(range, krange, sizeof(range), cudaMemcpyDeviceToHost, s));
-	PST_CUDA(cudaMemcpyAsync(&negzero, flag + 4, 4, cudaMemcpyDeviceToHost, s));
-	PST_CUDA(cudaMemcpyAsync(idscan, flag, 16, cudaMemcpyDeviceToHost, s));
+	BuildFlags<K> seen;
+	PST_CUDA(cudaMemcpyAsync(&seen, flag, sizeof(seen), cudaMemcpyDeviceToHost, s));
 	PST_CUDA(cudaStreamSynchronize(s));
+	const K *range = seen.range;
+	const bool negzero = seen.negzero != 0;
 	// ---- tiebreak order (id, input index): the input order unless the ids decrease
 	// somewhere, then the keys are made again in the order of one sort of the ids
 	const uint32_t *P = nullptr;
 	bool ids_are_indices = true;
 	if constexpr (HAS_ID) {
-		ids_are_indices = !(idscan[0] & 2u);
-		if (idscan[0] & 1u) {
+		ids_are_indices = !(seen.id_order & 2u);
+		if (seen.id_order & 1u) {
 			uint32_t *idk = static_cast<uint32_t *>(k1);  // k1 holds at least n u32
 			k_id_keys<T, HAS_ID><<<g, 256, 0, s>>>(pts, n, idk);
 			sc.keys_alt = kalt;
 			sc.vals_alt = valt;  // n u32 fit in the u64 buffers
 			sc.vals_tmp = c2;
 			uint32_t *kres, *vres;
-			radix_sort<uint32_t, uint32_t>(idk, nullptr, n, rs_passes<uint32_t>(idscan[2], idscan[3]), sc, &kres,
-			                               &vres, s);
+			radix_sort<uint32_t, uint32_t>(idk, nullptr, n, rs_passes<uint32_t>(seen.id_range[0], seen.id_range[1]), sc,
+			                               &kres, &vres, s);
 			// ids decrease somewhere, so they are not all equal and the sort ran
 			PST_CUDA(cudaMemcpyAsync(scr.at<uint32_t>(SL.P), vres, n * 4, cudaMemcpyDeviceToDevice, s));
 			P = scr.at<uint32_t>(SL.P);
@@ -1120,11 +1141,6 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 	c.err = flag + 1;
 	c.n = n;
 	c.D = D;
-	uint32_t *B = scr.at<uint32_t>(SL.Ba), *Bn = scr.at<uint32_t>(SL.Bb);
-	{
-		const uint32_t b0[2] = {0u, (uint32_t) n};
-		PST_CUDA(cudaMemcpyAsync(B, b0, 8, cudaMemcpyHostToDevice, s));
-	}
 	if (L0) {
 		k_tile_max<<<(unsigned) ((ntiles + TM_SUPER - 1) / TM_SUPER), LV_THREADS, 0, s>>>(c2s, n, c.tmax, c.smax);
 		PST_CUDA(cudaGetLastError());
@@ -1148,6 +1164,7 @@ void build_impl(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 	}
 	k_subtree<T, HAS_ID><<<(unsigned) nodes_wide, ST_THREADS, 0, s>>>(c, L0, B);
 	PST_CUDA(cudaGetLastError());
+	finish_tree_aux(t, s);  // its reads stay inside the tree whatever the check below finds
 	uint32_t errs[2] = {0, 0};
 	PST_CUDA(cudaMemcpyAsync(errs, flag, 8, cudaMemcpyDeviceToHost, s));
 	PST_CUDA(cudaStreamSynchronize(s));
@@ -1210,8 +1227,6 @@ void build_tree(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s)
 			t.idtype == PST_ID_U32 ? build_impl<int32_t, true>(t, pts_d, n, s) : build_impl<int32_t, false>(t, pts_d, n, s);
 			break;
 		}
-		finish_tree_aux(t, s);
-		PST_CUDA(cudaStreamSynchronize(s));
 	} catch (...) {
 		cudaStreamSynchronize(s);
 		free_tree(t);

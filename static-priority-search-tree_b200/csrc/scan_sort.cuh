@@ -404,10 +404,11 @@ struct SortScratch {
 	void *vals_alt = nullptr;  // n payloads
 	void *vals_tmp = nullptr;  // n payloads (second buffer for an identity input payload)
 	uint64_t *status = nullptr;  // rs_num_tiles(n) * 256
-	uint32_t *hist = nullptr;    // RS_MAX_PASSES * 256, zeroed by radix_sort
-	uint32_t *counters = nullptr;  // RS_MAX_PASSES tile counters, zeroed by radix_sort
+	uint32_t *hist = nullptr;    // RS_MAX_PASSES * 256, zeroed by radix_sort unless cleared
+	uint32_t *counters = nullptr;  // RS_MAX_PASSES tile counters, the same
 	uint32_t *err = nullptr;
 	uint32_t epoch = 1;
+	bool cleared = false;  // hist and counters are zero already
 };
 
 constexpr size_t rs_misc_words() { return RS_MAX_PASSES * 256 + RS_MAX_PASSES; }
@@ -443,7 +444,9 @@ void radix_sort(K *keys, V *vals, uint64_t n, int passes, SortScratch &sc, K **k
 	const uint64_t tiles = rs_num_tiles(n);
 	PST_CUDA(cudaFuncSetAttribute(k_rs_onesweep<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                              (int) rs_onesweep_smem<K, V>()));
-	PST_CUDA(cudaMemsetAsync(sc.hist, 0, rs_misc_words() * 4, s));
+	if (!sc.cleared)
+		PST_CUDA(cudaMemsetAsync(sc.hist, 0, rs_misc_words() * 4, s));
+	sc.cleared = false;
 	const unsigned hg = (unsigned) std::min<uint64_t>((n + RS_THREADS - 1) / RS_THREADS,
 	                                                  (uint64_t) device_info().sms * 4);
 	if (!pre_hist)
