@@ -218,7 +218,14 @@ pst_status pst_batch_destroy(pst_batch *batch);
  * the result exceeds out_capacity records, nothing is written to out_d,
  * offsets are still valid and PST_ERR_CAPACITY is returned.  sync = 0 makes the
  * call asynchronous on `stream` (then *total is only valid after a stream sync
- * and capacity overflow is reported by pst_batch_status). */
+ * and capacity overflow is reported by pst_batch_status).
+ * A call with sync = 0 on a stream that is being captured adds the pass to the
+ * caller's graph.  Its queries must then be a device array (PST_ERR_UNSUPPORTED
+ * otherwise, before anything is captured), which each replay reads anew; every replay
+ * writes out_d, offsets_d and, unless it is null, *total of this call, whatever the
+ * engine is called with in between.  Replays use the engine's workspace: they and the
+ * engine's other calls must follow one another (on one stream, or by events), and the
+ * graph must not be replayed once the engine or the tree is destroyed. */
 pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq, int queries_on_device,
                          pst_ret ret, void *out_d, uint64_t out_capacity, uint64_t *offsets_d,
                          uint64_t *total, int sync, pst_stream_t stream);

@@ -489,7 +489,10 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 			fail(PST_ERR_INVALID, "bad return type");
 		if (ret == PST_RET_IDS && b.tree->idtype != PST_ID_U32)
 			fail(PST_ERR_UNSUPPORTED, "an id-less tree can only return points");
-		b.stage_queries(queries, nq, queries_on_device != 0, s, offsets_d);
+		const bool in_graph =
+		    !sync && b.run_captured(queries, nq, queries_on_device != 0, ret, out_d, out_capacity, offsets_d, s);
+		if (!in_graph)
+			b.stage_queries(queries, nq, queries_on_device != 0, s, offsets_d);
 		uint64_t tot = 0;
 		if (sync) {
 			const EmitTo to{ret, out_d, out_capacity};
@@ -498,11 +501,14 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 				*total = tot;
 			result = tot > out_capacity ? PST_ERR_CAPACITY : b.last_status();
 		} else {
-			b.launch_count(s);
-			b.enqueue_emit(ret, out_d, out_capacity, s);
+			if (!in_graph) {
+				b.launch_count(s);
+				b.enqueue_emit(ret, out_d, out_capacity, s);
+			}
 			if (total)
 				check_cuda(cudaMemcpyAsync(total, &b.ctl->total, 8, cudaMemcpyDeviceToHost, s), "copy total");
-			b.mark_async(s);
+			if (!in_graph)
+				b.mark_async(s);
 		}
 	});
 	if (st != PST_OK)

@@ -282,6 +282,7 @@ void InFlight::mark(const void *owner, cudaStream_t s)
 	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
 	check_cuda(cudaStreamIsCapturing(s, &st), "cudaStreamIsCapturing");
 	if (st != cudaStreamCaptureStatusNone) {
+		check_cuda(cudaGetDevice(&m.device), "cudaGetDevice");
 		m.captured = true;  // an earlier mark's event does not belong in the caller's graph
 		return;
 	}
@@ -294,10 +295,17 @@ void InFlight::mark(const void *owner, cudaStream_t s)
 
 void InFlight::wait_for(const Mark &m) noexcept
 {
-	if (m.captured)
+	if (m.captured) {
+		int cur = 0;
+		cudaGetDevice(&cur);
+		if (cur != m.device)
+			cudaSetDevice(m.device);
 		cudaDeviceSynchronize();
-	else if (m.event)
+		if (cur != m.device)
+			cudaSetDevice(cur);
+	} else if (m.event) {
 		cudaEventSynchronize(m.event);
+	}
 	cudaGetLastError();
 }
 

@@ -29,9 +29,9 @@ unsigned long long current_context_id(int dev);
 // engine waits for its own pass, a tree for all of them, before its memory is freed.
 class InFlight {
   public:
-	// Marks the end of the work queued on `s` for `owner` (after its earlier mark, which
-	// may lie on another stream).  Work captured into a graph of the caller's may run at any
-	// time: from then on the owner waits for the whole device.
+	// Marks the end of the work queued on `s`, of the current device, for `owner` (after its
+	// earlier mark, which may lie on another stream).  Work captured into a graph of the
+	// caller's may run at any time: from then on the owner waits for the whole device.
 	void mark(const void *owner, cudaStream_t s);
 	void wait(const void *owner) noexcept;  // and forget it
 	void wait_all() noexcept;
@@ -42,6 +42,7 @@ class InFlight {
 	struct Mark {
 		cudaEvent_t event = nullptr;
 		bool captured = false;
+		int device = 0;
 	};
 	static void wait_for(const Mark &m) noexcept;
 	std::map<const void *, Mark> ev;

@@ -603,6 +603,20 @@ __global__ void k_load_ctl(const BatchCtl *src, BatchCtl *dst)
 		d[i] = s[i];
 }
 
+// The control block of a pass that a caller captures into a graph of theirs, from the
+// kernel's own parameters: the engine's pinned copy belongs to the calls that come later.
+__global__ void k_set_ctl(BatchCtl *ctl, const PassStart start)
+{
+	for (uint32_t i = threadIdx.x; i < sizeof(BatchCtl) / 4; i += blockDim.x)
+		reinterpret_cast<uint32_t *>(ctl)[i] = 0;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		ctl->nq = start.nq;
+		ctl->raw = start.raw;
+		ctl->user_offsets = start.offsets;
+	}
+}
+
 // Start of a full pass (after the control block's load): the batch's queries
 // unpacked and checked, their level-0 paths, and the per-query counts and output
 // cursors zeroed (all max_q of them: the scan reads every count).
@@ -1687,6 +1701,9 @@ void Batch::release()
 		passes->wait(this);  // an asynchronous pass may still use the buffers
 	pool_release(work, device);
 	pool_release(rec, device);
+	for (void *p : captured_recs)
+		pool_release(p, device);
+	captured_recs.clear();
 	work = nullptr;
 	pinned_release(ctl_host, device);  // the staged queries lie behind the control block
 	ctl_host = nullptr;
@@ -1781,11 +1798,16 @@ void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 
 void Batch::grow_tasks(uint64_t cap, cudaStream_t s)
 {
-	// Only the passes that used the old frontier are waited for (those on `s`, and an
-	// asynchronous one), not work on the device's other streams.
-	PST_CUDA(cudaStreamSynchronize(s));
-	passes->wait(this);
-	pool_release(rec, device);
+	if (captured) {
+		// a graph of the caller's holds the old frontier's address
+		captured_recs.push_back(rec);
+	} else {
+		// Only the passes that used the old frontier are waited for (those on `s`, and an
+		// asynchronous one), not work on the device's other streams.
+		PST_CUDA(cudaStreamSynchronize(s));
+		passes->wait(this);
+		pool_release(rec, device);
+	}
 	rec = nullptr;
 	task_cap = 0;
 	rec = static_cast<uint4 *>(pool_alloc(cap * sizeof(uint4), "frontier"));
@@ -1798,12 +1820,15 @@ void Batch::grow_tasks(uint64_t cap, cudaStream_t s)
 	WorkDev w{rec, task_cap, path0, path1, seed0, seed1, path_cap, ro, ro_cap, counts, cursor, offsets, ctl}
 
 template <typename T>
-void Batch::enqueue_count(cudaStream_t s)
+void Batch::enqueue_count(cudaStream_t s, const PassStart *own)
 {
 	TreeDev<T> tv = tree->view<T>();
 	QDev<T> qd{kind, static_cast<const T *>(min1), static_cast<const T *>(max1), static_cast<const T *>(min2)};
 	PST_WORKDEV;
-	k_load_ctl<<<1, 256, 0, s>>>(ctl_host_d, ctl);
+	if (own)
+		k_set_ctl<<<1, 256, 0, s>>>(ctl, *own);
+	else
+		k_load_ctl<<<1, 256, 0, s>>>(ctl_host_d, ctl);
 	const QOut<T> qo{kind, static_cast<T *>(min1), static_cast<T *>(max1), static_cast<T *>(min2)};
 	if (group_stop) {
 		const uint32_t rocap = 2 * group_stop * group, rcap = group * group_records(group_stop);
@@ -1818,7 +1843,7 @@ void Batch::enqueue_count(cudaStream_t s)
 	}
 	for (uint32_t d = group_stop; d < tv.levels; d++)
 		launch_level<T>(tv, qd, w, d, grid, threads, s);
-	scan_offsets(counts, offsets, max_q, scan_tmp, ctl, back_d, s);
+	scan_offsets(counts, offsets, max_q, scan_tmp, ctl, own ? nullptr : back_d, s);
 	PST_CUDA(cudaGetLastError());
 }
 
@@ -1870,12 +1895,12 @@ void Batch::enqueue_emit_v(pst_ret ret, void *out, uint64_t capacity, cudaStream
 	}
 }
 
-void Batch::enqueue_counting(cudaStream_t s)
+void Batch::enqueue_counting(cudaStream_t s, const PassStart *own)
 {
 	switch (tree->dtype) {
-	case PST_F32: enqueue_count<float>(s); break;
-	case PST_F64: enqueue_count<double>(s); break;
-	case PST_I32: enqueue_count<int32_t>(s); break;
+	case PST_F32: enqueue_count<float>(s, own); break;
+	case PST_F64: enqueue_count<double>(s, own); break;
+	case PST_I32: enqueue_count<int32_t>(s, own); break;
 	}
 }
 
@@ -1897,8 +1922,9 @@ void Batch::enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t
 	}
 }
 
-void Batch::launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStream_t s)
+void Batch::launch_count(cudaStream_t s)
 {
+	Graph &g = full_graph;
 	// an engine's first passes on a stream are launched as they are: capturing one and
 	// destroying it again takes 310 us, many engines live for a query or two, and a replay
 	// saves 4 us (a top pass) to 60 us of host time (a whole pass)
@@ -1908,7 +1934,7 @@ void Batch::launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStr
 		g.drop();
 		g.direct++;
 		g.stream = s;
-		(this->*enqueue)(s);
+		enqueue_counting(s);
 		return;
 	}
 	if (!g.exec) {
@@ -1917,7 +1943,7 @@ void Batch::launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStr
 		cudaGraph_t gr;
 		PST_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
 		try {
-			(this->*enqueue)(cs);
+			enqueue_counting(cs);
 		} catch (...) {
 			cudaStreamEndCapture(cs, &gr);
 			cudaStreamDestroy(cs);
@@ -1931,7 +1957,27 @@ void Batch::launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStr
 	PST_CUDA(cudaGraphLaunch(g.exec, s));
 }
 
-void Batch::launch_count(cudaStream_t s) { launch_graph(full_graph, &Batch::enqueue_counting, s); }
+bool Batch::run_captured(const pst_query *q, uint32_t nq, bool on_device, pst_ret ret, void *out, uint64_t capacity,
+                         uint64_t *to_offsets, cudaStream_t s)
+{
+	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+	PST_CUDA(cudaStreamIsCapturing(s, &st));
+	if (st == cudaStreamCaptureStatusNone)
+		return false;
+	check_queries(q, nq);
+	if (!on_device && nq)
+		fail(PST_ERR_UNSUPPORTED, "the queries of a pass that is captured into a graph must be a device array");
+	// Nothing of the pass is the engine's to change later: its queries' and offsets' places
+	// are kernel parameters, the kernels are the caller's graph's own, and the frontier stays
+	// (grow_tasks).  The block that the host waits with is left alone: a pass before this one
+	// may still use it.
+	captured = true;
+	const PassStart own{nq, q, to_offsets};
+	enqueue_counting(s, &own);
+	enqueue_emit(ret, out, capacity, s);
+	passes->mark(this, s);
+	return true;
+}
 
 void Batch::launch_count_top(cudaStream_t s)
 {
@@ -1949,13 +1995,18 @@ void Batch::launch_count_rest(uint32_t from, cudaStream_t s)
 	}
 }
 
-void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, uint64_t *to_offsets)
+void Batch::check_queries(const pst_query *q, uint32_t nq) const
 {
 	if (nq > max_q)
 		fail(PST_ERR_INVALID, "batch of " + std::to_string(nq) + " queries exceeds max_queries " +
 		                          std::to_string(max_q));
 	if (nq && !q)
 		fail(PST_ERR_INVALID, "null query array");
+}
+
+void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, uint64_t *to_offsets)
+{
+	check_queries(q, nq);
 	// the pinned control block and query staging may still feed an earlier pass
 	if (!idle)
 		PST_CUDA(cudaStreamSynchronize(s));

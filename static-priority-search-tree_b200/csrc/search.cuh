@@ -1,6 +1,8 @@
 // Batched / single-query search engine (host side).
 #pragma once
 
+#include <vector>
+
 #include "tree.cuh"
 
 namespace pst {
@@ -64,6 +66,13 @@ struct TopIn {
 	pst_query q[TOP_IN_QUERIES];
 };
 
+// What a whole pass starts from, apart from the control block's zeros.
+struct PassStart {
+	uint32_t nq;
+	const pst_query *raw;
+	uint64_t *offsets;
+};
+
 // Where a waiting call wants its results.
 struct EmitTo {
 	pst_ret ret;
@@ -117,6 +126,8 @@ struct Batch {
 		void drop();
 	};
 	Graph full_graph;
+	bool captured = false;              // a graph of the caller's holds a pass of this engine
+	std::vector<void *> captured_recs;  // outgrown frontiers such a graph may use
 
 	~Batch();
 	void init(TreeStorage *t, const pst_batch_opts &o);
@@ -126,6 +137,11 @@ struct Batch {
 	void stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, uint64_t *offsets = nullptr);
 	// Whole count pass (every level kernel and the scan), asynchronous.
 	void launch_count(cudaStream_t s);
+	// Where `s` is capturing: adds the asynchronous pass to the caller's graph and returns
+	// true.  Replays answer the same queries into the same buffers whatever the engine is
+	// called with in between.
+	bool run_captured(const pst_query *q, uint32_t nq, bool on_device, pst_ret ret, void *out, uint64_t capacity,
+	                  uint64_t *offsets, cudaStream_t s);
 	// Notes that work queued on `s` may still run when the call returns.
 	void mark_async(cudaStream_t s)
 	{
@@ -143,7 +159,8 @@ struct Batch {
 	void count_sync(cudaStream_t s, uint64_t *total, const EmitTo *to = nullptr);
 	void count_full_sync(cudaStream_t s, uint64_t *total, const EmitTo *to);
 	void count_small_sync(cudaStream_t s, uint64_t *total, const EmitTo *to);
-	void enqueue_counting(cudaStream_t s);
+	// own: the pass's start by value instead of the engine's control block.
+	void enqueue_counting(cudaStream_t s, const PassStart *own = nullptr);
 	void enqueue_counting_top(cudaStream_t s);
 	// to_host: the emit also writes the host's copy of the control block.
 	void enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s, bool to_host = false);
@@ -154,12 +171,12 @@ struct Batch {
 
   private:
 	template <typename T>
-	void enqueue_count(cudaStream_t s);
+	void enqueue_count(cudaStream_t s, const PassStart *own);
 	template <typename T>
 	void enqueue_count_top(cudaStream_t s);
 	template <typename T>
 	void enqueue_count_rest(uint32_t from, cudaStream_t s);
-	void launch_graph(Graph &g, void (Batch::*enqueue)(cudaStream_t), cudaStream_t s);
+	void check_queries(const pst_query *q, uint32_t nq) const;
 	template <typename T>
 	void enqueue_emit_v(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s, bool to_host);
 	template <typename T, bool HAS_ID, bool POINTS>

@@ -151,6 +151,14 @@ def _stream(stream=None):
     return C.c_void_p(s.cuda_stream)
 
 
+def _capturing(stream=None) -> bool:
+    torch = _torch()
+    if stream is None:
+        return torch.cuda.is_current_stream_capturing()
+    with torch.cuda.stream(stream):
+        return torch.cuda.is_current_stream_capturing()
+
+
 def point_dtype(dt: str, has_id: bool) -> np.dtype:
     """numpy layout of the reference's PointStruct (helpers/point-struct.h)."""
     fields = [("dim1", NP[dt]), ("dim2", NP[dt])]
@@ -467,8 +475,10 @@ class BatchEngine:
         rec = 4 if ret == "ids" else self.tree.rec_point.itemsize
         cap = out_d.numel() * out_d.element_size() // rec
         tot = C.c_uint64()
+        # a captured pass would write the total at every replay, long after this call
+        to = None if not sync and _capturing(stream) else C.byref(tot)
         st = lib().pst_batch_run(self._h, qp, nq, int(queries_on_device), RET[ret], C.c_void_p(out_d.data_ptr()),
-                                 cap, C.c_void_p(offsets_d.data_ptr()), C.byref(tot), int(sync), _stream(stream))
+                                 cap, C.c_void_p(offsets_d.data_ptr()), to, int(sync), _stream(stream))
         if st not in (0, 4):
             _check(st)
         return st, tot.value
