@@ -497,6 +497,8 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 		if (sync) {
 			const EmitTo to{ret, out_d, out_capacity};
 			b.count_sync(s, &tot, &to);
+			if (b.copy_offsets(nq, s))
+				check_cuda(cudaStreamSynchronize(s), "sync");
 			if (total)
 				*total = tot;
 			result = tot > out_capacity ? PST_ERR_CAPACITY : b.last_status();
@@ -504,6 +506,7 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 			if (!in_graph) {
 				b.launch_count(s);
 				b.enqueue_emit(ret, out_d, out_capacity, s);
+				b.copy_offsets(nq, s);
 			}
 			if (total)
 				check_cuda(cudaMemcpyAsync(total, &b.ctl->total, 8, cudaMemcpyDeviceToHost, s), "copy total");

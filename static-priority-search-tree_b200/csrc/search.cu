@@ -1760,6 +1760,7 @@ void Batch::init(TreeStorage *t, const pst_batch_opts &o)
 		};
 		auto layout = [&] {
 			off = 0;
+			take(&q_copy, (size_t) max_q * sizeof(pst_query));
 			take(&kind, (size_t) max_q * 4);
 			take(&min1, (size_t) max_q * vs);
 			take(&max1, (size_t) max_q * vs);
@@ -1972,9 +1973,10 @@ bool Batch::run_captured(const pst_query *q, uint32_t nq, bool on_device, pst_re
 	// (grow_tasks).  The block that the host waits with is left alone: a pass before this one
 	// may still use it.
 	captured = true;
-	const PassStart own{nq, q, to_offsets};
+	const PassStart own = place(q, nq, on_device, to_offsets, s);
 	enqueue_counting(s, &own);
 	enqueue_emit(ret, out, capacity, s);
+	copy_offsets(nq, s);
 	passes->mark(this, s);
 	return true;
 }
@@ -2004,6 +2006,51 @@ void Batch::check_queries(const pst_query *q, uint32_t nq) const
 		fail(PST_ERR_INVALID, "null query array");
 }
 
+// Whether kernels of the engine's device can use the caller's array of 8-byte words where
+// it is: an array of another device may be out of their reach, and an address that is not
+// a multiple of 8 would end the context.
+static bool usable_in_place(const void *p, int device)
+{
+	if (reinterpret_cast<uintptr_t>(p) & 7u)
+		return false;
+	cudaPointerAttributes a{};
+	if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+		cudaGetLastError();
+		return false;
+	}
+	return a.type == cudaMemoryTypeDevice ? a.device == device : a.type != cudaMemoryTypeUnregistered && a.devicePointer == p;
+}
+
+// Where the pass finds its queries and leaves the caller's offsets: the caller's arrays
+// themselves where kernels can use them (a copy of each costs 2 to 3 us), the staged
+// queries through their mapping, or else copies.
+PassStart Batch::place(const pst_query *q, uint32_t nq, bool on_device, uint64_t *to_offsets, cudaStream_t s)
+{
+	PassStart at{nq, q, to_offsets};
+	copy_offsets_to = nullptr;
+	if (!on_device) {
+		if (nq)
+			memcpy(q_stage, q, (size_t) nq * sizeof(pst_query));
+		at.raw = q_stage_d;
+	} else if (nq && !usable_in_place(q, device)) {
+		PST_CUDA(cudaMemcpyAsync(q_copy, q, (size_t) nq * sizeof(pst_query), cudaMemcpyDeviceToDevice, s));
+		at.raw = q_copy;
+	}
+	if (to_offsets && !usable_in_place(to_offsets, device)) {
+		copy_offsets_to = to_offsets;
+		at.offsets = nullptr;
+	}
+	return at;
+}
+
+bool Batch::copy_offsets(uint32_t nq, cudaStream_t s)
+{
+	if (!copy_offsets_to)
+		return false;
+	PST_CUDA(cudaMemcpyAsync(copy_offsets_to, offsets, ((size_t) nq + 1) * 8, cudaMemcpyDeviceToDevice, s));
+	return true;
+}
+
 void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, uint64_t *to_offsets)
 {
 	check_queries(q, nq);
@@ -2011,18 +2058,16 @@ void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaS
 	if (!idle)
 		PST_CUDA(cudaStreamSynchronize(s));
 	idle = false;
-	// the kernels read the queries where they are, the staged ones through their mapping
-	if (!on_device && nq)
-		memcpy(q_stage, q, (size_t) nq * sizeof(pst_query));
+	const PassStart at = place(q, nq, on_device, to_offsets, s);
 	ctl_host->nq = nq;
-	ctl_host->raw = on_device ? q : q_stage_d;
-	ctl_host->user_offsets = to_offsets;
+	ctl_host->raw = at.raw;
+	ctl_host->user_offsets = at.offsets;
 	ctl_host->host_fault = &back_d->fault;
 	ctl_host->emit_follows = 0;
 	back->fault = 0;
 	top_in.args = TopArgs{};
 	top_in.args.nq = nq;
-	top_in.args.offsets = to_offsets;
+	top_in.args.offsets = at.offsets;
 	if (!on_device && nq <= TOP_IN_QUERIES)
 		std::copy(q, q + nq, top_in.q);
 	else

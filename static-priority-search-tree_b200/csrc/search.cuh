@@ -93,6 +93,8 @@ struct Batch {
 	uint32_t blocks_per_sm = 0;
 	uint32_t grid = 0;
 	// queries
+	pst_query *q_copy = nullptr;   // of a device array that kernels cannot read where it is
+	uint64_t *copy_offsets_to = nullptr;  // the caller's offsets where kernels cannot write them
 	pst_query *q_stage = nullptr;  // pinned staging for host query arrays
 	uint32_t *kind = nullptr;
 	void *min1 = nullptr, *max1 = nullptr, *min2 = nullptr;
@@ -142,6 +144,9 @@ struct Batch {
 	// called with in between.
 	bool run_captured(const pst_query *q, uint32_t nq, bool on_device, pst_ret ret, void *out, uint64_t capacity,
 	                  uint64_t *offsets, cudaStream_t s);
+	// Queues the copy of the pass's offsets to an array that its kernels could not write;
+	// false where they have.
+	bool copy_offsets(uint32_t nq, cudaStream_t s);
 	// Notes that work queued on `s` may still run when the call returns.
 	void mark_async(cudaStream_t s)
 	{
@@ -177,6 +182,7 @@ struct Batch {
 	template <typename T>
 	void enqueue_count_rest(uint32_t from, cudaStream_t s);
 	void check_queries(const pst_query *q, uint32_t nq) const;
+	PassStart place(const pst_query *q, uint32_t nq, bool on_device, uint64_t *to_offsets, cudaStream_t s);
 	template <typename T>
 	void enqueue_emit_v(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s, bool to_host);
 	template <typename T, bool HAS_ID, bool POINTS>
