@@ -1923,6 +1923,13 @@ void Batch::enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t
 	}
 }
 
+void Batch::capture_next(cudaStream_t s)
+{
+	full_graph.drop();
+	full_graph.stream = s;
+	full_graph.direct = DIRECT_PASSES;
+}
+
 void Batch::launch_count(cudaStream_t s)
 {
 	Graph &g = full_graph;

@@ -137,6 +137,8 @@ struct Batch {
 	void grow_tasks(uint64_t cap, cudaStream_t s);
 	// offsets: where the pass also writes the result offsets (nq + 1 on the device, or null).
 	void stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaStream_t s, uint64_t *offsets = nullptr);
+	// Has the next whole pass on `s` captured at once: for an engine that will serve many.
+	void capture_next(cudaStream_t s);
 	// Whole count pass (every level kernel and the scan), asynchronous.
 	void launch_count(cudaStream_t s);
 	// Where `s` is capturing: adds the asynchronous pass to the caller's graph and returns

@@ -578,8 +578,8 @@ uint32_t server_add_tree(Server *s, TreeStorage *t, const pst_batch_opts *tuning
 		bo.task_capacity = std::max<uint64_t>(1ull << 16, t->n / 8);
 		sl->eng.init(t, bo);
 		check_cuda(cudaStreamCreateWithFlags(&sl->stream, cudaStreamNonBlocking), "cudaStreamCreate");
-		// warm-up passes: capture the slot's graphs (the whole count pass, and the top pass
-		// of small batches) now rather than under the first requests
+		// warm-up passes: the slot's graph (of the whole count pass) is captured now rather
+		// than under the requests, which it would keep waiting for 310 us on every slot
 		{
 			// an inverted 3-sided range walks one path and reports nothing
 			pst_query q{};
@@ -595,6 +595,7 @@ uint32_t server_add_tree(Server *s, TreeStorage *t, const pst_batch_opts *tuning
 				q.max1.i32 = 0;
 			}
 			uint64_t total = 0;
+			sl->eng.capture_next(sl->stream);
 			sl->eng.stage_queries(&q, 1, false, sl->stream);
 			sl->eng.count_full_sync(sl->stream, &total, nullptr);
 			sl->eng.stage_queries(&q, 1, false, sl->stream);
