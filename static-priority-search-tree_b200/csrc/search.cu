@@ -1435,12 +1435,11 @@ void launch_cta_pass(const TreeDev<T> &tv, const QDev<T> &qd, const WorkDev &w, 
 	    tv, qd, w, max_q, (qcap + 1) & ~1u, pcap, rcap, qo, in, back);
 }
 
-// The host's copy of a finished pass's control block (by the whole CTA; `back` may be null).
-__device__ __forceinline__ void ctl_to_host(const BatchCtl *ctl, BatchCtl *back)
+// The host's copy of a pass's control block (by the whole CTA; `back` may be null).
+__device__ __forceinline__ void ctl_to_host(const BatchCtl *ctl, BatchCtl *back, bool emitting = false)
 {
 	if (back)
-		for (uint32_t i = threadIdx.x; i < sizeof(BatchCtl) / 4; i += blockDim.x)
-			reinterpret_cast<uint32_t *>(back)[i] = reinterpret_cast<const uint32_t *>(ctl)[i];
+		copy_ctl(ctl, back, threadIdx.x, blockDim.x, emitting);
 }
 
 // THREADS: the CTA size and U the records each warp has in flight (both tuning
@@ -1454,7 +1453,7 @@ __global__ void __launch_bounds__(THREADS) k_emit(TreeDev<T> t, WorkDev w, void 
 	__shared__ uint64_t s_total;
 	__shared__ EmitWarp<Point<T, HAS_ID>, POINTS> s_warp[THREADS / 32];
 	if (blockIdx.x == 0)
-		ctl_to_host(w.ctl, back);
+		ctl_to_host(w.ctl, back, true);
 	if (threadIdx.x == 0) {
 		uint64_t b = 0;
 		for (uint32_t e = 0; e < t.levels; e++)

@@ -1,6 +1,7 @@
 // Batched / single-query search engine (host side).
 #pragma once
 
+#include <cstddef>
 #include <vector>
 
 #include "tree.cuh"
@@ -40,14 +41,25 @@ struct BatchCtl {
 	// each instead of summing every count before them
 	uint64_t lvl_base[40];
 	uint32_t emitted;       // the top pass wrote the results itself
-	uint32_t fault;         // (host copy) the emit's consistency check failed
-	uint32_t unused[2];
+	uint32_t unused[3];
 	uint32_t top_cnt[40];   // records per level that k_bfs_groups put with the boundary nodes
 	const pst_query *raw;   // the queries: mapped pinned memory or the caller's device array
 	uint64_t *user_offsets; // the caller's nq + 1 offsets, or null
 	uint32_t *host_fault;   // `fault` of the host's copy, or null
-	uint64_t emit_follows;  // the emit hands the host its copy, while it runs, not the scan
+	uint32_t emit_follows;  // the emit hands the host its copy, while it runs, not the scan
+	uint32_t fault;         // (host copy; the last word) the emit's consistency check failed
 };
+
+// Copies words first, first + step, .. of a pass's control block to the host's copy.  An emit
+// does so while its other CTAs may be storing `fault` there (its own words hold none): it
+// leaves that one word alone.
+__host__ __device__ inline void copy_ctl(const BatchCtl *ctl, BatchCtl *to, uint32_t first, uint32_t step, bool emitting)
+{
+	const uint32_t end = sizeof(BatchCtl) / 4 - (emitting ? 1 : 0);
+	for (uint32_t i = first; i < end; i += step)
+		reinterpret_cast<uint32_t *>(to)[i] = reinterpret_cast<const uint32_t *>(ctl)[i];
+}
+static_assert(offsetof(BatchCtl, fault) + 4 == sizeof(BatchCtl), "the fault is the last word");
 
 // What the top pass of a small batch works on (kernel parameters).
 struct TopArgs {
