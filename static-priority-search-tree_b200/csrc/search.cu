@@ -1195,6 +1195,7 @@ __global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T
 		sc->need_tasks = over ? nrec : 0;
 		sc->total = total;
 		sc->emitted = emit;
+		sc->waits = 1;
 		sc->user_offsets = in.args.offsets;  // for a scan that follows
 		sc->host_fault = back ? &back->fault : nullptr;
 		sc->emit_follows = in.args.out != nullptr;
@@ -1203,7 +1204,7 @@ __global__ void __launch_bounds__(TOP_THREADS, 1) k_bfs_cta(TreeDev<T> t, QDev<T
 	if (done) {
 		for (uint32_t q = threadIdx.x; q <= max_q; q += TOP_THREADS)
 			offsets[q] = q < nq ? s_offs[q] : total;
-		if (in.args.offsets)
+		if (in.args.offsets && !(flags & BATCH_FLAGS_FAILED))
 			for (uint32_t q = threadIdx.x; q <= nq; q += TOP_THREADS)
 				in.args.offsets[q] = q < nq ? s_offs[q] : total;
 	}
@@ -1461,7 +1462,7 @@ __global__ void __launch_bounds__(THREADS) k_emit(TreeDev<T> t, WorkDev w, void 
 		s_total = b;
 	}
 	__syncthreads();
-	if (w.ctl->total > capacity || (w.ctl->flags & BATCH_FLAG_TASK_OVERFLOW)) {
+	if (w.ctl->total > capacity || (w.ctl->flags & (w.ctl->waits ? BATCH_FLAGS_FAILED : BATCH_FLAG_TASK_OVERFLOW))) {
 		if (blockIdx.x == 0 && threadIdx.x == 0 && w.ctl->total > capacity)
 			atomicOr(&w.ctl->flags, BATCH_FLAG_OUT_OVERFLOW);
 		return;
@@ -1515,7 +1516,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_offsets(const uint64_t *counts
 	asm volatile("griddepcontrol.wait;" ::: "memory");
 	__shared__ uint64_t ws[33];
 	const uint32_t nq = ctl->nq;
-	uint64_t *user = ctl->user_offsets;
+	uint64_t *user = ctl->waits && (ctl->flags & BATCH_FLAGS_FAILED) ? nullptr : ctl->user_offsets;
 	uint64_t carry = 0;
 	for (uint32_t c0 = 0; c0 < n; c0 += SCAN_TILE) {
 		const uint32_t base = c0 + threadIdx.x * SCAN_ITEMS;
@@ -1552,7 +1553,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_offsets(const uint64_t *counts
 // The end of a pass of more queries, after its scan.
 __global__ void __launch_bounds__(SCAN_THREADS) k_pass_end(const uint64_t *offsets, const BatchCtl *ctl, BatchCtl *back)
 {
-	if (ctl->user_offsets)
+	if (ctl->user_offsets && !(ctl->waits && (ctl->flags & BATCH_FLAGS_FAILED)))
 		for (uint64_t q = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; q <= ctl->nq; q += (uint64_t) gridDim.x * blockDim.x)
 			ctl->user_offsets[q] = offsets[q];
 	if (blockIdx.x == 0 && !ctl->emit_follows)
@@ -2070,6 +2071,7 @@ void Batch::stage_queries(const pst_query *q, uint32_t nq, bool on_device, cudaS
 	ctl_host->user_offsets = at.offsets;
 	ctl_host->host_fault = &back_d->fault;
 	ctl_host->emit_follows = 0;
+	ctl_host->waits = 0;
 	back->fault = 0;
 	top_in.args = TopArgs{};
 	top_in.args.nq = nq;
@@ -2139,12 +2141,13 @@ static bool settle(Batch &b, int attempt, cudaStream_t s, uint64_t *total)
 }
 
 // The whole pass, with automatic growth of the frontier buffer.  An emit queued behind a
-// count pass writes nothing when the pass did not fit the frontier or its results the
-// buffer.
+// count pass writes nothing when the pass failed, did not fit the frontier or its results
+// the buffer.
 void Batch::count_full_sync(cudaStream_t s, uint64_t *total, const EmitTo *to)
 {
 	const bool emits = to && to->out && to->capacity;
 	ctl_host->emit_follows = emits;
+	ctl_host->waits = 1;
 	for (int attempt = 0;; attempt++) {
 		launch_count(s);
 		if (emits)

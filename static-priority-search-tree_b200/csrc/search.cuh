@@ -22,6 +22,7 @@ enum : uint32_t {
 	BATCH_FLAG_OUT_OVERFLOW = 2u,   // output buffer too small (nothing written)
 	BATCH_FLAG_BAD_QUERY = 4u,      // a query kind out of range
 	BATCH_FLAG_INTERNAL = 8u,       // a device-side consistency check failed
+	BATCH_FLAGS_FAILED = BATCH_FLAG_TASK_OVERFLOW | BATCH_FLAG_BAD_QUERY | BATCH_FLAG_INTERNAL,
 };
 
 // Device control block of one pass; the host uploads a zeroed copy (with nq set)
@@ -41,7 +42,8 @@ struct BatchCtl {
 	// each instead of summing every count before them
 	uint64_t lvl_base[40];
 	uint32_t emitted;       // the top pass wrote the results itself
-	uint32_t unused[3];
+	uint32_t waits;         // the host waits for the pass: one that fails leaves the caller's buffers alone
+	uint32_t unused[2];
 	uint32_t top_cnt[40];   // records per level that k_bfs_groups put with the boundary nodes
 	const pst_query *raw;   // the queries: mapped pinned memory or the caller's device array
 	uint64_t *user_offsets; // the caller's nq + 1 offsets, or null
