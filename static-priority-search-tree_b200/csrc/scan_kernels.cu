@@ -614,6 +614,24 @@ void metacell_cols_launch(const T *vol, const uint32_t P[3], const uint32_t mc[3
 	                                                         M[0], M[1], mz_begin, mz_end, mz_begin * mc[2], mzp, out);
 }
 
+// Whether a column holds too few vertices of a metacell to pay for its way through shared
+// memory and the two barriers of a layer, on a device that `threads`, one per metacell
+// column of 8 layers, leave no room to hide the loads of a thread per metacell.  By
+// metacells and by columns, 509 x 381 x 263 vertices: f32 in 4 x 1 x 1 119 and 262 us, in
+// 4 x 4 x 1 109 and 133, in 4 x 1 x 2 108 and 142, in 4 x 2 x 2 119 and 105; f64 in 2 x 2 x 2
+// 157 and 192, in 4 x 2 x 3 121 and 145, in 8 x 2 x 2 296 and 270, in 3 x 3 x 3 131 and 142
+// (but 195 and 173 for 1031 x 300 x 200).  201 x 181 x 163, f32 in 2 x 4 x 1: 38 and 27.
+template <typename T>
+bool metacell_is_flat(const uint32_t mc[3], uint64_t threads)
+{
+	const uint64_t full = (uint64_t) device_info().sms * 2048;
+	if (mc[2] == 1)
+		return mc[1] <= 5 && threads * 5 >= full * 2;
+	if (sizeof(T) == 8)
+		return mc[0] <= 5 && (uint64_t) mc[1] * mc[2] <= 6 && threads * 5 >= full * 3;
+	return mc[0] <= 8 && (uint64_t) mc[1] * mc[2] <= 2 && threads >= full;
+}
+
 template <typename T, bool HAS_ID>
 void metacell_launch(const void *vol, const uint32_t P[3], const uint32_t mc[3], const uint32_t M[3],
                      uint32_t mz_begin, uint32_t mz_end, void *out, cudaStream_t s)
@@ -630,9 +648,10 @@ void metacell_launch(const void *vol, const uint32_t P[3], const uint32_t mc[3],
 		if constexpr (sizeof(T) == 4) {
 			// fewer layers a CTA while the device has room for more threads: a layer's planes
 			// are one chain of loads (128^3 vertices: 65 us with 8 layers a CTA, 16 with one;
-			// 512^3: 129 us with 8, 123 with 2 or 4)
+			// 512^3: 129 us with 8, 123 with 2 or 4), but no fewer than 8 planes, as CTAs share one
+			// (512 x 512 x 256 in 4 x 1 x 1: 123 us with 4 layers a CTA, 113 with 8)
 			const uint32_t gx = (M[0] + threads - 1) / threads;
-			uint32_t mzp = 4;
+			uint32_t mzp = std::max(4u, 8 / mc[2]);
 			while (mzp > 1 && (uint64_t) gx * threads * M[1] * ((layers + mzp - 1) / mzp) <
 			                      (uint64_t) device_info().sms * 2048)
 				mzp /= 2;
@@ -642,10 +661,11 @@ void metacell_launch(const void *vol, const uint32_t P[3], const uint32_t mc[3],
 			                                                 mz_end, mz_begin * mc[2], mzp, o);
 		}
 	} else if (mc[0] == 1 || mc[0] >= (uint32_t) MC_COL_THREADS ||
-	           (uint64_t) P[0] * std::min(P[1], 2 * mc[1]) >= (1ull << 30)) {
+	           (uint64_t) P[0] * std::min(P[1], 2 * mc[1]) >= (1ull << 30) ||
+	           metacell_is_flat<T>(mc, (uint64_t) (M[0] + threads - 1) / threads * threads * M[1] * ((layers + 7) / 8))) {
 		// one vertex wide (consecutive threads are consecutive vertices already: 970 us for
-		// 512^3 f32 voxels, 1090 by columns), wider than a CTA of columns, or rows too long
-		// for its 32-bit offsets: a thread per metacell
+		// 512^3 f32 voxels, 1090 by columns), wider than a CTA of columns, rows too long
+		// for its 32-bit offsets, or few vertices to a column: a thread per metacell
 		const dim3 grid((M[0] + threads - 1) / threads, M[1], (layers + 7) / 8);
 		k_metacells<T, HAS_ID><<<grid, threads, 0, s>>>(v, P[0], P[1], P[2], mc[0], mc[1], mc[2], M[0], M[1], mz_begin,
 		                                                mz_end, mz_begin * mc[2], 8, o);
