@@ -1,5 +1,6 @@
 // The block pool of pool.cuh.
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -45,37 +46,25 @@ struct Block {
 	size_t bytes;
 };
 
-// One device's blocks, with the context they belong to: cudaDeviceReset ends that
-// context, and its blocks are forgotten at the next call.
+// One context's blocks.
 struct Pool {
 	const bool pinned;
-	std::mutex mu;
-	unsigned long long ctx = 0;
 	size_t keep = 0, kept = 0;
 	std::vector<Block> idle;                    // oldest first
 	std::unordered_map<void *, size_t> live;
 
-	explicit Pool(bool host) : pinned(host) {}
+	explicit Pool(bool host) : pinned(host)
+	{
+		size_t fr = 0, total = 0;
+		check_cuda(cudaMemGetInfo(&fr, &total), "cudaMemGetInfo");
+		keep = pinned ? KEEP_PINNED : total / KEEP_SHARE;
+	}
 	cudaError_t get(void **ptr, size_t bytes) const { return pinned ? cudaMallocHost(ptr, bytes) : cudaMalloc(ptr, bytes); }
 	void give_back(const std::vector<Block> &blocks) const noexcept
 	{
 		for (const Block &b : blocks)
 			if ((pinned ? cudaFreeHost(b.ptr) : cudaFree(b.ptr)) != cudaSuccess)
 				cudaGetLastError();
-	}
-
-	// (with mu held)
-	void enter(unsigned long long now)
-	{
-		if (ctx == now)
-			return;
-		idle.clear();
-		live.clear();
-		kept = 0;
-		size_t fr = 0, total = 0;
-		check_cuda(cudaMemGetInfo(&fr, &total), "cudaMemGetInfo");
-		keep = pinned ? KEEP_PINNED : total / KEEP_SHARE;
-		ctx = now;
 	}
 
 	// The smallest idle block that holds `bytes` and is at most an eighth larger.
@@ -108,13 +97,28 @@ struct Pool {
 	}
 };
 
-// The pools of every device.
+// The pools of one device, by the id of their context.  A block belongs to the context it
+// was made in, and programs may switch between several; cudaDeviceReset ends one, whose
+// pool is then never entered again (ids are not used twice).
 struct Pools {
-	Pool mem{false}, pinned{true};
-};
-Pools g_pools[64];
+	const bool pinned;
+	std::mutex mu;
+	std::map<unsigned long long, Pool> of;
 
-Pools &pools_of(int dev)
+	explicit Pools(bool host) : pinned(host) {}
+	// (with mu held)
+	Pool &enter(unsigned long long ctx)
+	{
+		const auto it = of.find(ctx);
+		return it != of.end() ? it->second : of.emplace(ctx, pinned).first->second;
+	}
+};
+struct DevicePools {
+	Pools mem{false}, pinned{true};
+};
+DevicePools g_pools[64];
+
+DevicePools &pools_of(int dev)
 {
 	if (dev < 0 || dev >= 64)
 		fail(PST_ERR_CUDA, "device index out of range");
@@ -169,66 +173,80 @@ unsigned long long current_context_id(int dev)
 
 namespace {
 
-void *alloc_in(Pool &p, int dev, size_t bytes, const char *what)
+void *alloc_in(Pools &pools, int dev, size_t bytes, const char *what)
 {
 	const unsigned long long ctx = current_context_id(dev);
 	const size_t want = block_bytes(bytes);
-	{
-		std::lock_guard<std::mutex> lk(p.mu);
-		p.enter(ctx);
-		if (void *ptr = p.take(want))
-			return ptr;
-	}
+	Pool *p = nullptr;
 	void *ptr = nullptr;
-	cudaError_t e = p.get(&ptr, want);
+	std::vector<Block> out;
+	{
+		std::lock_guard<std::mutex> lk(pools.mu);
+		p = &pools.enter(ctx);  // (a map's elements stay where they are)
+		ptr = p->take(want);
+		out = p->shrink(p->keep);  // (what was released under another context)
+	}
+	p->give_back(out);
+	if (ptr)
+		return ptr;
+	cudaError_t e = p->get(&ptr, want);
 	if (e == cudaErrorMemoryAllocation) {
 		cudaGetLastError();
 		pool_trim();
-		e = p.get(&ptr, want);
+		e = p->get(&ptr, want);
 	}
 	if (e == cudaErrorMemoryAllocation) {
 		cudaGetLastError();
 		fail(PST_ERR_NOMEM, std::string(what) + " allocation of " + std::to_string(bytes) + " B failed");
 	}
 	check_cuda(e, "cudaMalloc");
-	std::lock_guard<std::mutex> lk(p.mu);
-	p.live[ptr] = want;
+	std::lock_guard<std::mutex> lk(pools.mu);
+	p->live[ptr] = want;
 	return ptr;
 }
 
-void release_in(Pool &p, int dev, void *ptr)
+void release_in(Pools &pools, int dev, void *ptr)
 {
 	std::vector<Block> out;
+	Pool *p = nullptr;
 	{
 		const unsigned long long ctx = current_context_id(dev);
-		std::lock_guard<std::mutex> lk(p.mu);
-		p.enter(ctx);
-		const auto it = p.live.find(ptr);
-		if (it == p.live.end())
-			return;  // a block of a context that is gone went with it
+		std::lock_guard<std::mutex> lk(pools.mu);
+		Pool &here = pools.enter(ctx);
+		p = &here;
+		if (here.live.find(ptr) == here.live.end())
+			for (auto &x : pools.of)
+				if (x.second.live.find(ptr) != x.second.live.end())
+					p = &x.second;
+		const auto it = p->live.find(ptr);
+		if (it == p->live.end())
+			return;
 		const Block b{ptr, it->second};
-		p.live.erase(it);
-		if (b.bytes > p.keep) {
+		p->live.erase(it);
+		if (p == &here && b.bytes > p->keep) {
 			out.push_back(b);
 		} else {
-			p.idle.push_back(b);
-			p.kept += b.bytes;
-			out = p.shrink(p.keep);
+			p->idle.push_back(b);
+			p->kept += b.bytes;
+			// another context's blocks are given back from there (it may be gone, too)
+			if (p == &here)
+				out = p->shrink(p->keep);
 		}
 	}
-	p.give_back(out);
+	p->give_back(out);
 }
 
-void trim(Pool &p, int dev)
+void trim(Pools &pools, int dev)
 {
 	std::vector<Block> out;
+	Pool *p = nullptr;
 	{
 		const unsigned long long ctx = current_context_id(dev);
-		std::lock_guard<std::mutex> lk(p.mu);
-		p.enter(ctx);
-		out = p.shrink(0);
+		std::lock_guard<std::mutex> lk(pools.mu);
+		p = &pools.enter(ctx);
+		out = p->shrink(0);
 	}
-	p.give_back(out);
+	p->give_back(out);
 }
 
 void release_on(bool pinned, void *ptr, int device) noexcept
