@@ -457,7 +457,9 @@ __global__ void __launch_bounds__(LV_THREADS) k_level(BuildCtx<T, HAS_ID> c, uin
 	// the ancestors' positions, wanted for the median
 	const uint32_t anc = lane < d ? c.top_pos[h >> (lane + 1)] : 0u;
 	const uint32_t cnt = node_count32((uint32_t) c.n, d, j);
-	if (err)  // after an error the bounds may hold unwritten entries
+	// after an error the bounds may hold unwritten entries (a CTA's warps find out together,
+	// below: one that returned alone would leave its words of s_key unwritten)
+	if (GROUP == 32 && err)
 		return;
 	if (cnt < 2 || lo >= hi || hi > c.n) {
 		if (t == 0)
@@ -513,8 +515,7 @@ __global__ void __launch_bounds__(LV_THREADS) k_level(BuildCtx<T, HAS_ID> c, uin
 			s_key[threadIdx.x >> 5] = best;
 			s_at[threadIdx.x >> 5] = at;
 		}
-		__syncthreads();
-		if (threadIdx.x >= 32)
+		if (__syncthreads_or(err) || threadIdx.x >= 32)
 			return;
 		key = lane < LV_THREADS / 32 ? s_key[lane] : 0ull;
 		best = warp_max_key(key);
@@ -561,6 +562,11 @@ __global__ void __launch_bounds__(LV_THREADS) k_level(BuildCtx<T, HAS_ID> c, uin
 			if (lane == 0)
 				c.smax[at & AT_INDEX] = m;
 		}
+	}
+	if (tp < lo || tp >= hi) {
+		if (lane == 0)
+			atomicOr(c.err, 8u);
+		return;
 	}
 	// the median: the floor(cnt / 2)-th position of [lo, hi) that no ancestor's point, nor
 	// this node's, holds: the smallest pos = first + (positions taken up to pos)
@@ -731,7 +737,8 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(BuildCtx<T, HAS_ID> c, u
 
 	const uint32_t j = blockIdx.x;
 	const uint32_t cN = node_count32((uint32_t) c.n, L0, j);
-	if (cN == 0 || __any_sync(0xFFFFFFFFu, *c.err != 0))
+	const bool err = *c.err != 0;
+	if (cN == 0)
 		return;
 	const uint32_t lo0 = L0 ? B[j] : 0u;
 	const uint32_t hi0 = L0 ? B[j + 1] : (uint32_t) c.n;
@@ -763,7 +770,9 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(BuildCtx<T, HAS_ID> c, u
 		}
 		for (uint32_t i = threadIdx.x; i < 2 * ST_CAP / 32; i += ST_THREADS)
 			s_occ[i] = 0;
-		__syncthreads();
+		// (together: a warp that returned alone would leave its counts and keys unwritten)
+		if (__syncthreads_or(err))
+			return;
 		if (warp == 0) {
 			// (chunk, warp) pairs in order, a lane each
 			constexpr int PAIRS = ST_GATHER * ST_WARPS;
