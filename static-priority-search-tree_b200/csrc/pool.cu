@@ -311,19 +311,24 @@ void InFlight::mark(const void *owner, cudaStream_t s)
 	check_cuda(cudaEventRecord(m.event, s), "cudaEventRecord");
 }
 
+void wait_for_device(int device) noexcept
+{
+	int cur = 0;
+	cudaGetDevice(&cur);
+	if (cur != device)
+		cudaSetDevice(device);
+	cudaDeviceSynchronize();
+	if (cur != device)
+		cudaSetDevice(cur);
+	cudaGetLastError();
+}
+
 void InFlight::wait_for(const Mark &m) noexcept
 {
-	if (m.captured) {
-		int cur = 0;
-		cudaGetDevice(&cur);
-		if (cur != m.device)
-			cudaSetDevice(m.device);
-		cudaDeviceSynchronize();
-		if (cur != m.device)
-			cudaSetDevice(cur);
-	} else if (m.event) {
+	if (m.captured)
+		wait_for_device(m.device);
+	else if (m.event)
 		cudaEventSynchronize(m.event);
-	}
 	cudaGetLastError();
 }
 

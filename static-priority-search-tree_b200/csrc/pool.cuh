@@ -24,6 +24,9 @@ void pool_trim() noexcept;
 // the thread has none.
 unsigned long long current_context_id(int dev);
 
+// Waits for all the work of a device, whichever is current.
+void wait_for_device(int device) noexcept;
+
 // The asynchronous passes over one tree that may still be running, one event per
 // engine.  The tree and its engines share it, so either may be destroyed first: an
 // engine waits for its own pass, a tree for all of them, before its memory is freed.

@@ -1697,6 +1697,8 @@ void Batch::Graph::drop()
 void Batch::release()
 {
 	full_graph.drop();
+	if (open)
+		wait_for_device(device);  // a call that failed with some of its kernels queued, or a server's
 	if (passes)
 		passes->wait(this);  // an asynchronous pass may still use the buffers
 	pool_release(work, device);
@@ -1916,6 +1918,7 @@ void Batch::enqueue_counting_top(cudaStream_t s)
 
 void Batch::enqueue_emit(pst_ret ret, void *out, uint64_t capacity, cudaStream_t s, bool to_host)
 {
+	open = true;
 	switch (tree->dtype) {
 	case PST_F32: enqueue_emit_v<float>(ret, out, capacity, s, to_host); break;
 	case PST_F64: enqueue_emit_v<double>(ret, out, capacity, s, to_host); break;
@@ -1933,6 +1936,7 @@ void Batch::capture_next(cudaStream_t s)
 void Batch::launch_count(cudaStream_t s)
 {
 	Graph &g = full_graph;
+	open = true;
 	// an engine's first passes on a stream are launched as they are: capturing one and
 	// destroying it again takes 310 us, many engines live for a query or two, and a replay
 	// saves 4 us (a top pass) to 60 us of host time (a whole pass)
@@ -1980,11 +1984,11 @@ bool Batch::run_captured(const pst_query *q, uint32_t nq, bool on_device, pst_re
 	// (grow_tasks).  The block that the host waits with is left alone: a pass before this one
 	// may still use it.
 	captured = true;
+	passes->mark(this, s);
 	const PassStart own = place(q, nq, on_device, to_offsets, s);
 	enqueue_counting(s, &own);
 	enqueue_emit(ret, out, capacity, s);
 	copy_offsets(nq, s);
-	passes->mark(this, s);
 	return true;
 }
 
@@ -1992,11 +1996,13 @@ void Batch::launch_count_top(cudaStream_t s)
 {
 	if (ctl_host->nq > top_q)
 		fail(PST_ERR_INTERNAL, "top pass on a batch of more than " + std::to_string(top_q) + " queries");
+	open = true;
 	enqueue_counting_top(s);
 }
 
 void Batch::launch_count_rest(uint32_t from, cudaStream_t s)
 {
+	open = true;
 	switch (tree->dtype) {
 	case PST_F32: enqueue_count_rest<float>(from, s); break;
 	case PST_F64: enqueue_count_rest<double>(from, s); break;
@@ -2109,6 +2115,7 @@ pst_status Batch::finish(cudaStream_t s)
 	if (last.fault)
 		last.flags |= BATCH_FLAG_INTERNAL;
 	idle = true;
+	open = false;
 	return last_status();
 }
 

@@ -133,6 +133,7 @@ struct Batch {
 	const pst_query *q_stage_d = nullptr;
 	TopIn top_in{};
 	bool idle = false;             // no pass that uses the block can be in flight
+	bool open = false;             // kernels may be queued that nobody has waited for or marked
 	BatchCtl last{};
 	// the captured whole count pass, for the stream it was captured for
 	struct Graph {
@@ -168,6 +169,7 @@ struct Batch {
 	{
 		idle = false;
 		passes->mark(this, s);
+		open = false;
 	}
 	// Top pass of a small batch (nq <= top_q), asynchronous: when it stops
 	// above the bottom (ctl->cta_levels < tree levels), launch_count_rest finishes it.
