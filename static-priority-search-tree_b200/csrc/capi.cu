@@ -133,7 +133,7 @@ static cudaMemPool_t result_pool()
 
 static void malloc_result(void **out, uint64_t bytes, cudaStream_t s)
 {
-	cudaError_t e = cudaMallocFromPoolAsync(out, bytes, result_pool(), s);
+	const cudaError_t e = allocate_or_trim([&] { return cudaMallocFromPoolAsync(out, bytes, result_pool(), s); });
 	if (e != cudaSuccess) {
 		*out = nullptr;
 		if (e == cudaErrorMemoryAllocation) {

@@ -135,7 +135,7 @@ void metacells_from_file(const char *path, pst_dtype dt, pst_idtype it, const ui
 		}
 	} df{dev};
 	for (int i = 0; i < 2; i++) {
-		cudaError_t e = cudaMalloc(&dev[i], slab_cap);
+		const cudaError_t e = allocate_or_trim([&] { return cudaMalloc(&dev[i], slab_cap); });
 		if (e == cudaErrorMemoryAllocation) {
 			cudaGetLastError();
 			fail(PST_ERR_NOMEM, "slab allocation of " + std::to_string(slab_cap) + " B failed");

@@ -189,12 +189,7 @@ void *alloc_in(Pools &pools, int dev, size_t bytes, const char *what)
 	p->give_back(out);
 	if (ptr)
 		return ptr;
-	cudaError_t e = p->get(&ptr, want);
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		pool_trim();
-		e = p->get(&ptr, want);
-	}
+	const cudaError_t e = allocate_or_trim([&] { return p->get(&ptr, want); });
 	if (e == cudaErrorMemoryAllocation) {
 		cudaGetLastError();
 		fail(PST_ERR_NOMEM, std::string(what) + " allocation of " + std::to_string(bytes) + " B failed");

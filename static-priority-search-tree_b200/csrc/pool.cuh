@@ -20,6 +20,19 @@ void pinned_release(void *p, int device) noexcept;
 // Gives the blocks kept on the current device back.
 void pool_trim() noexcept;
 
+// The result of `allocate`, called again without the kept blocks where it first runs out of
+// memory: what the library keeps counts as free for its own allocations.
+template <typename F>
+cudaError_t allocate_or_trim(F &&allocate)
+{
+	const cudaError_t e = allocate();
+	if (e != cudaErrorMemoryAllocation)
+		return e;
+	cudaGetLastError();
+	pool_trim();
+	return allocate();
+}
+
 // Unique id of the calling thread's current context on device `dev`, made current when
 // the thread has none.
 unsigned long long current_context_id(int dev);

@@ -59,7 +59,7 @@ struct Arena {
 	void init(uint64_t bytes, bool host_mirror)
 	{
 		size = (bytes + 255) / 256 * 256;
-		check_cuda(cudaMalloc(&base, size), "cudaMalloc(result arena)");
+		check_cuda(allocate_or_trim([&] { return cudaMalloc(&base, size); }), "cudaMalloc(result arena)");
 		if (host_mirror)
 			check_cuda(cudaMallocHost((void **) &host, size), "cudaMallocHost(result staging)");
 		free_[0] = size;
