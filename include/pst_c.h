@@ -82,6 +82,15 @@ size_t pst_point_size(pst_dtype dtype, pst_idtype idtype);
  * free those results with cudaFree (testers/pst-tester-functions.tu:711-713). */
 pst_status pst_free(void *ptr_d);
 
+/* Gives back the memory of the current device (and context) that the library keeps for
+ * reuse.  It keeps the device memory of destroyed trees, engines and scratch up to 1/32
+ * of the device (5.6 GiB of 179), up to 1 GiB of freed results, and up to 8 MiB of
+ * pinned host memory; its own allocations take it back by themselves when the device
+ * runs full, another allocator in the process needs this call.  Reuse is what makes
+ * repeated builds fast: the next ones map their memory anew.  No reference counterpart
+ * (its memory is cudaMalloc'd and freed per object). */
+pst_status pst_trim_memory(void);
+
 /* ------------------------------------------------------------------------- */
 /* Tree                                                                       */
 

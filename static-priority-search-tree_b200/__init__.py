@@ -30,4 +30,5 @@ from .pst import (  # noqa: F401
     point_dtype,
     points_to_device,
     readInVertices,
+    trim_memory,
 )

@@ -224,6 +224,15 @@ pst_status pst_free(void *ptr_d)
 	});
 }
 
+pst_status pst_trim_memory(void)
+{
+	return guarded([&] {
+		require_device();
+		pool_trim();
+		check_cuda(cudaMemPoolTrimTo(result_pool(), 0), "cudaMemPoolTrimTo");
+	});
+}
+
 pst_status pst_mem_needed(pst_dtype dtype, pst_idtype idtype, uint64_t n, uint64_t *bytes)
 {
 	return guarded([&] {

@@ -15,7 +15,8 @@ namespace pst {
 namespace {
 
 // Freed memory kept per device: 1/KEEP_SHARE of its memory (5.6 of 179 GiB), enough for
-// the build of a 2^26-point tree beside the tree that it replaces (3.6 GiB).  cudaMalloc
+// the build of a 2^26-point tree beside the tree that it replaces (3.6 GiB); of a larger
+// one, as of 2^28 points, the scratch is mapped and unmapped at each build.  cudaMalloc
 // and cudaFree map and unmap pages, and cudaFree waits for the whole device: 19 and 20 of
 // them took 2.1 of the 4.4 ms of an isosurface pass over a 384^3 volume, and 1.2 of the
 // 1.9 ms of a build of 2^21 points.  A stream-ordered CUDA pool did as well while the

@@ -97,6 +97,7 @@ def lib():
         "pst_two_sided_left": (i32, [vp, u64, u64, i32, P(vp), P(u64), vp]),
         "pst_two_sided_right": (i32, [vp, u64, u64, i32, P(vp), P(u64), vp]),
         "pst_search_into": (i32, [vp, P(Query), i32, vp, u64, P(u64), vp]),
+        "pst_trim_memory": (i32, []),
         "pst_batch_create": (i32, [P(vp), vp, P(BatchOpts)]),
         "pst_batch_destroy": (i32, [vp]),
         "pst_batch_run": (i32, [vp, vp, u32, i32, i32, vp, u64, vp, P(u64), i32, vp]),
@@ -214,6 +215,12 @@ def free_device(ptr: int):
     """Releases a result returned by a drop-in search (pst_free)."""
     if ptr:
         _check(lib().pst_free(C.c_void_p(ptr)))
+
+
+def trim_memory():
+    """Gives back the device memory that the library keeps for reuse (pst_trim_memory)."""
+    _torch()
+    _check(lib().pst_trim_memory())
 
 
 def make_queries(kinds, min1, max1, min2, dt: str) -> np.ndarray:
