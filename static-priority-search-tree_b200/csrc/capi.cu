@@ -186,6 +186,8 @@ static uint64_t run_single(pst_tree *tr, const pst_query *q, pst_ret ret, void *
 		// counted and written in one go, where the results fit
 		const EmitTo to{ret, *out_d, capacity};
 		b.count_sync(s, &total, *out_d ? &to : nullptr);
+		if (total && total <= capacity && !*out_d)
+			fail(PST_ERR_INVALID, "null output buffer");
 		if (total && total <= capacity && b.last_status() != PST_OK)
 			fail(b.last_status(), "search emit failed");
 		return total;
@@ -510,6 +512,8 @@ pst_status pst_batch_run(pst_batch *batch, const pst_query *queries, uint32_t nq
 				check_cuda(cudaStreamSynchronize(s), "sync");
 			if (total)
 				*total = tot;
+			if (tot && tot <= out_capacity && !out_d)
+				fail(PST_ERR_INVALID, "null output buffer");
 			result = tot > out_capacity ? PST_ERR_CAPACITY : b.last_status();
 		} else {
 			if (!in_graph) {
