@@ -1400,6 +1400,54 @@ void finish_tree_aux(TreeStorage &t, cudaStream_t s)
 	}
 }
 
+namespace {
+
+// Zeros for the places of a field that hold no node: place 0, and those of the last level
+// without one.
+template <typename T>
+__global__ void k_clear_absent(T *dim1, T *dim2, T *med, uint32_t *id, const uint32_t *occ, uint64_t slots)
+{
+	const uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
+	const uint64_t h = i == 0 ? 0 : slots / 2 + i - 1;
+	if (h >= slots || ((occ[h >> 5] >> (h & 31)) & 1u))
+		return;
+	dim1[h] = dim2[h] = T(0);
+	if (h == 0)
+		med[0] = T(0);
+	if (id)
+		id[h] = 0;
+}
+
+template <typename T>
+void clear_absent_t(const TreeStorage &t, cudaStream_t s)
+{
+	const uint64_t slots = 1ull << t.levels;
+	k_clear_absent<T><<<(unsigned) ((slots / 2 + 1 + 255) / 256), 256, 0, s>>>(as<T>(t.dim1), as<T>(t.dim2), as<T>(t.med),
+	                                                                        t.id, t.occ, slots);
+	PST_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+void clear_absent(const TreeStorage &t, cudaStream_t s)
+{
+	if (!t.n)
+		return;
+	// the gaps behind the fields of a small tree
+	const TreeLayout L = tree_layout(t.dtype, t.idtype, t.n);
+	const size_t vs = value_size(t.dtype), S = size_t(1) << t.levels;
+	const size_t ends[] = {L.off_dim1 + S * vs, L.off_dim2 + S * vs, L.off_med + S / 2 * vs,
+	                       L.off_id + (t.id ? S * 4 : 0), L.off_occ + std::max<size_t>(S / 32, 1) * 4};
+	for (size_t e : ends)
+		if (e % ALIGN)
+			PST_CUDA(cudaMemsetAsync(static_cast<char *>(t.mem) + e, 0, ALIGN - e % ALIGN, s));
+	switch (t.dtype) {
+	case PST_F32: clear_absent_t<float>(t, s); break;
+	case PST_F64: clear_absent_t<double>(t, s); break;
+	case PST_I32: clear_absent_t<int32_t>(t, s); break;
+	}
+}
+
 void free_tree(TreeStorage &t)
 {
 	t.passes->wait_all();  // asynchronous passes may still read the tree

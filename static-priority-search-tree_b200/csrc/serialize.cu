@@ -1,6 +1,7 @@
 // Tree images: save a built tree and load it back without rebuilding (for a
 // serving loop that restarts with the same resident trees).  The image is a 64-byte
-// header followed by the tree's single device allocation byte for byte, so a load
+// header followed by the tree's single device allocation byte for byte (zeros where there
+// is no node, so equal trees give equal images), so a load
 // is one allocation and one copy; files stream through pinned double buffers, the
 // disk transfer of one chunk overlapping the host-device copy of the previous one.
 #include <cstdio>
@@ -122,6 +123,7 @@ void save_tree(const TreeStorage &t, void *host, uint64_t capacity, cudaStream_t
 	const Header h = make_header(t);
 	memcpy(host, &h, HEADER_BYTES);
 	if (t.bytes) {
+		clear_absent(t, s);
 		PST_CUDA(cudaMemcpyAsync(static_cast<unsigned char *>(host) + HEADER_BYTES, t.mem, t.bytes,
 		                         cudaMemcpyDeviceToHost, s));
 		PST_CUDA(cudaStreamSynchronize(s));
@@ -164,6 +166,7 @@ void save_tree_file(const TreeStorage &t, const char *path)
 		cudaStream_t s;
 		check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
 		std::unique_ptr<CUstream_st, void (*)(cudaStream_t)> sguard(s, [](cudaStream_t x) { cudaStreamDestroy(x); });
+		clear_absent(t, s);
 		const uint64_t chunk = std::min<uint64_t>(FILE_CHUNK, t.bytes);
 		PinnedPair pp(chunk);
 		// copy chunk i+1 to the host while chunk i is written to disk

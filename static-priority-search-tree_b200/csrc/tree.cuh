@@ -64,6 +64,9 @@ void mc_tables(uint8_t *ntri, uint8_t *edges);
 uint64_t mc_run(const float *vol, const uint32_t P[3], const uint32_t mc[3], const uint32_t *ids, uint64_t n, float iso,
                 float *tri, uint64_t capacity, bool emit, cudaStream_t s);
 
+// Zeros every place of the tree's memory that holds no node (searches never look there; an
+// image holds what the memory's last user left there otherwise).
+void clear_absent(const TreeStorage &t, cudaStream_t s);
 void build_tree(TreeStorage &t, const void *pts_d, uint64_t n, cudaStream_t s);
 void free_tree(TreeStorage &t);
 // Host copy in the reference's field layout (slot = heap index - 1).
