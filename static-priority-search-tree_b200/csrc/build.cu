@@ -616,9 +616,9 @@ __global__ void __launch_bounds__(LV_THREADS) k_level(BuildCtx<T, HAS_ID> c, uin
 // its median, and every other lane goes down to a child.  No key moves, no lane waits for
 // another warp.
 //
-// Bound by instruction issue.  With a compaction of all keys per sub-level (each a pass for
-// the maxima, one for the node writes and one to move the keys, with barriers between) the
-// kernel took 2654 us at 2^26 points, 92 at 2^21 and 463 at 5 M doubles; now 1896, 68 and
+// Bound by instruction issue (81 % of the cycles at 2^24 points).  With a compaction of all
+// keys per sub-level (each a pass for the maxima, one for the node writes and one to move the
+// keys, with barriers between) the kernel took 2654 us at 2^26 points, 92 at 2^21 and 463 at 5 M doubles; now 1896, 68 and
 // 258.  Of the 1896, a copy that stops early puts some 400 in the gather, 500 in the
 // sub-levels of large nodes and 300 before the first sub-level of the small ones.  CTAs of
 // 256 threads took 2184 us (more wait at the barriers), of 64 1836 (but 0.5 % more in all at
@@ -1273,7 +1273,7 @@ __device__ __forceinline__ T min_of_none()
 // blocks' values.  A CTA owns 2^(depth - 1) consecutive blocks of level e and all their
 // ancestors down to one: the minima of their own children are independent reads, whatever
 // the level, and the blocks' values are then folded up in shared memory.  SM_DEPTH levels a
-// launch in place of one each: 2^26 points 256 us in 21 launches, 148 in 3; 2^21 40, 21.  (Level by
+// launch in place of one each: 2^26 points 256 us in 21 launches, 134 in 3; 2^21 40, 19.  (Level by
 // level inside the CTA, with a barrier between them: 189 us.)
 constexpr int SM_DEPTH = 7, SM_THREADS = 256, SM_WARPS = SM_THREADS / 32;
 

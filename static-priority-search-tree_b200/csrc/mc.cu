@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(MC_THREADS) k_mc_cells(const float *__restrict
 // cell's pattern is cut out by a shift; the vertices of the next group are on their way
 // meanwhile.  In the emit 64 cells list their triangles, and a lane makes a triangle: a
 // lane per cell would walk 0 to 5 triangles of its own, the warp as long as its fullest
-// cell, each vertex through indexed registers (local memory).  Bound by instruction issue:
+// cell, each vertex through indexed registers (local memory).  Bound by instructions and by
+// what they wait for in shared memory (57 % of the cycles issue):
 // 76 k active metacells of a 512^3 volume (3.9 M triangles, 142 MB) took 2 x 48 us to
 // count, 22 to scan and 241 to emit with a lane per cell, and take 2 x 29 and 102 (the
 // vertices as floats in shared memory, a lane per triangle corner: 2 x 46 and 128).  More

@@ -230,9 +230,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_global_hist(const K *__restri
 }
 
 // One pass over n < 2^31 keys.  vals_in == nullptr means the identity payload (the key's
-// input index; 32-bit payloads only).  Bound by instructions (an issue slot in 1.7
-// taken) and by latency: each tile's phases depend on one another, three CTAs to an SM
-// overlap them, and the look-back waits for whichever tile before this one is slowest.
+// input index; 32-bit payloads only).  Bound by latency, then by instructions: each tile's
+// phases depend on one another, the three CTAs to an SM that the registers leave (36 % of
+// the warps) overlap them, and the look-back waits for whichever tile before this one is
+// slowest; 47 % of the cycles issue, L1 and shared memory run at 68 %, DRAM at 37 %.
 // So the counts leave before the ranking, which then hides them, and the ranking is
 // unrolled without a test per key for a whole tile.  The payloads are read into
 // registers before the ranking and staged sorted beside their keys.  Microseconds a

@@ -1939,7 +1939,7 @@ void Batch::launch_count(cudaStream_t s)
 	open = true;
 	// an engine's first passes on a stream are launched as they are: capturing one and
 	// destroying it again takes 310 us, many engines live for a query or two, and a replay
-	// saves 4 us (a top pass) to 60 us of host time (a whole pass)
+	// saves 60 us of host time
 	if (!use_graph || g.stream != s || g.direct < DIRECT_PASSES) {
 		if (g.stream != s)
 			g.direct = 0;
