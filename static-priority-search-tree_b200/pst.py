@@ -152,12 +152,10 @@ def _stream(stream=None):
     return C.c_void_p(s.cuda_stream)
 
 
-def _capturing(stream=None) -> bool:
-    torch = _torch()
-    if stream is None:
-        return torch.cuda.is_current_stream_capturing()
-    with torch.cuda.stream(stream):
-        return torch.cuda.is_current_stream_capturing()
+def _capturing(stream: C.c_void_p) -> bool:
+    """Whether the stream is being captured (the runtime that the library is linked to)."""
+    status = C.c_int()
+    return lib().cudaStreamIsCapturing(stream, C.byref(status)) == 0 and status.value != 0
 
 
 def point_dtype(dt: str, has_id: bool) -> np.dtype:
@@ -483,9 +481,10 @@ class BatchEngine:
         cap = out_d.numel() * out_d.element_size() // rec
         tot = C.c_uint64()
         # a captured pass would write the total at every replay, long after this call
-        to = None if not sync and _capturing(stream) else C.byref(tot)
+        s = _stream(stream)
+        to = None if not sync and _capturing(s) else C.byref(tot)
         st = lib().pst_batch_run(self._h, qp, nq, int(queries_on_device), RET[ret], C.c_void_p(out_d.data_ptr()),
-                                 cap, C.c_void_p(offsets_d.data_ptr()), to, int(sync), _stream(stream))
+                                 cap, C.c_void_p(offsets_d.data_ptr()), to, int(sync), s)
         if st not in (0, 4):
             _check(st)
         return st, tot.value

@@ -37,10 +37,10 @@ class Case:
         return (torch.zeros(max(self.total, 1), dtype=torch.int32, device="cuda"),
                 torch.zeros(len(self.lo) + 1, dtype=torch.int64, device="cuda"))
 
-    def capture(self, out=None, offs=None):
+    def capture(self, out=None, offs=None, mode="thread_local"):
         import torch
         graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, stream=self.stream, capture_error_mode="thread_local"):
+        with torch.cuda.graph(graph, stream=self.stream, capture_error_mode=mode):
             st, _ = self.engine.run(self.q, self.out if out is None else out, self.offs if offs is None else offs,
                                     queries_on_device=True, sync=False, stream=self.stream)
         assert st == 0
@@ -107,6 +107,35 @@ def test_capture_after_asynchronous_passes(pst, earlier):
         assert c.replayed(first) and c.replayed(second, out2, offs2)
     assert c.engine.run(c.batch, c.out, c.offs, stream=c.stream) == (0, c.total)
     c.close(first, second)
+
+
+@pytest.mark.parametrize("mode", ["global", "relaxed"])
+def test_capture_modes(pst, mode):
+    """Nothing in the call is refused in any mode, also as an engine's first call."""
+    c = Case(pst, np.linspace(0.9, 1, 30), 30)
+    graph = c.capture(mode=mode)
+    assert c.replayed(graph) and c.replayed(graph)
+    c.close(graph)
+
+
+class _Handle:
+    """A stream of another framework: all that the binding asks for is its handle."""
+
+    def __init__(self, stream):
+        self.cuda_stream = stream.cuda_stream
+
+
+def test_total_of_a_captured_pass_is_left_alone(pst):
+    import torch
+    c = Case(pst, np.linspace(0.9, 1, 30), 30)
+    st, total = c.engine.run(c.q, c.out, c.offs, queries_on_device=True, sync=False, stream=_Handle(c.stream))
+    c.stream.synchronize()
+    assert (st, total) == (0, c.total)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=c.stream, capture_error_mode="thread_local"):
+        assert c.engine.run(c.q, c.out, c.offs, queries_on_device=True, sync=False, stream=_Handle(c.stream)) == (0, 0)
+    assert c.replayed(graph)
+    c.close(graph)
 
 
 def test_frontier_grown_between_replays(pst):
