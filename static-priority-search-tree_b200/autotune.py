@@ -33,6 +33,7 @@ from .pst import BatchEngine, StaticPSTGPU
 
 DEFAULT_CACHE = Path(os.environ.get("PST_AUTOTUNE_CACHE", Path.home() / ".cache" / "pst_b200" / "autotune.json"))
 MAX_TOP_PASS = 1024
+CAPTURED_AT = 5  # run on a stream at which an engine captures its pass (DIRECT_PASSES + 1 of csrc/search.cuh)
 
 
 def cache_key(tree: StaticPSTGPU, nq: int) -> str:
@@ -75,7 +76,9 @@ def _time(eng, qd, out, offs, ret, repeats, torch):
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
     s = torch.cuda.current_stream()
     eng.run(qd, out, offs, ret=ret, queries_on_device=True, sync=True)  # sizes the frontier
-    for _ in range(2):
+    # an engine captures its pass at the fifth run on a stream, which has to lie before the
+    # timed ones (it takes as long as several passes)
+    for _ in range(CAPTURED_AT):
         eng.run(qd, out, offs, ret=ret, queries_on_device=True, sync=False)
     torch.cuda.synchronize()
     ev[0].record(s)
