@@ -109,10 +109,11 @@ def test_capture_after_asynchronous_passes(pst, earlier):
     c.close(first, second)
 
 
+@pytest.mark.parametrize("nq", [30, 17000])  # (more than one CTA's scan of the offsets)
 @pytest.mark.parametrize("mode", ["global", "relaxed"])
-def test_capture_modes(pst, mode):
+def test_capture_modes(pst, mode, nq):
     """Nothing in the call is refused in any mode, also as an engine's first call."""
-    c = Case(pst, np.linspace(0.9, 1, 30), 30)
+    c = Case(pst, np.linspace(0.999, 1, nq), nq)
     graph = c.capture(mode=mode)
     assert c.replayed(graph) and c.replayed(graph)
     c.close(graph)

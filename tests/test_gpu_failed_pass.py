@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("ret", ["ids", "points"])
-@pytest.mark.parametrize("nq", [2, 20, 33, 100])
+@pytest.mark.parametrize("nq", [2, 20, 33, 100, 17000])
 def test_bad_kind(pst, nq, ret):
     import torch
     pts = rand_points(20000, "f32", seed=4)
